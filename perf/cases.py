@@ -399,7 +399,7 @@ def _gbuffer(case, seed):
     z = _linear_depth(case, g, r)
     h, w = z.shape
     inv_p = torch.tensor(list(b.ubo.cameraInverseProjection), dtype=torch.float64, device="cuda").reshape(4, 4)
-    inv_v = torch.linalg.inv(torch.tensor(list(b.ubo.cameraView), dtype=torch.float64, device="cuda").reshape(4, 4))
+    inv_v = torch.linalg.inv(torch.tensor(list(b.ubo.cameraView), dtype=torch.float64).reshape(4, 4)).cuda()
     clip = torch.ones(h, w, 4, dtype=torch.float64, device="cuda")
     clip[..., 0] = (torch.arange(w, device="cuda") + 0.5) / w * 2.0 - 1.0
     clip[..., 1] = ((torch.arange(h, device="cuda") + 0.5) / h * 2.0 - 1.0)[:, None]
