@@ -1,7 +1,11 @@
 // cf_batch.cpp — many views culled together (the batched form of the path).
 //
 // A batch holds N views, each with its own UBO, light set, AABBs and output
-// buffers (caller-owned device memory).  One culling pass of the batch is
+// buffers (caller-owned device memory).  One culling pass of the batch is, for
+// the views on the hit-mask path (cf_mask.cu; every view unless its grid was
+// tuned to another configuration), one launch per stage
+//   box, list, scan, sum, emit
+// and for the views on the staged path
 //   batch_xform   every view's lights to view space            (1 launch)
 //   batch_bin     every view's depth-slice candidate lists      (1 launch)
 //   cull_batch    a persistent kernel taking (view, cluster group) items
@@ -40,8 +44,8 @@ namespace {
 const cfk::CullConfig kBatchCandidates[] = {
     {1, 4, 256, 4, 1}, {2, 4, 256, 4, 1}, {4, 4, 256, 4, 1}, {1, 8, 256, 4, 1}, {2, 8, 256, 4, 1}, {4, 8, 256, 4, 1},
     {2, 4, 512, 2, 1}, {4, 4, 512, 2, 1}, {2, 8, 512, 2, 1}, {4, 8, 512, 2, 1}, {2, 8, 1024, 2, 1}, {4, 8, 1024, 2, 1},
+    cfk::kMaskConfig,
 };
-const cfk::CullConfig kBatchDefault = {2, 8, 1024, 2, 1};
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -70,7 +74,14 @@ struct CfBatch {
         int ctas;
     };
     std::vector<Launch> launches;
+    // the staged views' jobs, then the hit-mask views' by decreasing light
+    // count (the longest blocks start first); position of view i's in pos[i]
     std::vector<cfk::ViewJob> jobs;
+    std::vector<uint32_t> pos;
+    uint32_t staged = 0;  // views on the staged path
+    cfk::MaskBatch mask{};
+    uint32_t* d_mask_prefix = nullptr;
+    size_t mask_prefix_cap = 0;
     uint32_t xform_blocks = 0, bin_blocks = 0, copy_blocks_total = 0, n_items = 0;
     size_t ws_bytes = 0;
     // device
@@ -130,10 +141,20 @@ void drop_graph(CfBatch* b)
     b->graph_stream = nullptr;
 }
 
-cfk::CullConfig config_for(const CfBatch* b, uint32_t key)
+// The configuration of a view of this grid: the bucket's tuning (a hit-mask
+// tuning only where the grid fits it), else the hit-mask path where it fits.
+cfk::CullConfig config_for(const CfBatch* b, uint32_t key, uint32_t slices)
 {
     auto it = b->tuned.find(key);
-    return it == b->tuned.end() ? kBatchDefault : it->second;
+    const cfk::CullConfig c = it == b->tuned.end() ? cfk::kMaskConfig : it->second;
+    return cfk::is_mask_config(c) && !cfk::mask_fits(key * slices, key, slices) ? cfk::kStagedConfig : c;
+}
+
+// The staged configuration of a grid's views that are not on the hit-mask path.
+cfk::CullConfig staged_config(const CfBatch* b, uint32_t key)
+{
+    auto it = b->tuned.find(key);
+    return it == b->tuned.end() || cfk::is_mask_config(it->second) ? cfk::kStagedConfig : it->second;
 }
 
 bool same_config(const cfk::CullConfig& a, const cfk::CullConfig& c)
@@ -163,26 +184,43 @@ int rebuild(CfBatch* b)
     drop_graph(b);
     const uint32_t n = (uint32_t)b->views.size();
     b->jobs.assign(n, cfk::ViewJob{});
+    b->pos.assign(n, 0);
     std::vector<size_t> ws_off(n);
+    std::vector<cfk::CullConfig> cfgs(n);
     std::vector<cfk::WorkspaceLayout> lay(n);
-    std::vector<uint32_t> prefix(4 * (size_t)n), aabb_prefix(n);
+    std::vector<cfk::MaskLayout> mask_lay(n);
+    std::vector<uint32_t> aabb_prefix(n), mask_views;
     std::vector<cfk::AabbJob> aabb_jobs(n);
-    uint32_t ab = 0;
+    uint32_t ab = 0, most_lights = 0;
+    uint32_t ns = 0;  // staged views
+    for (uint32_t i = 0; i < n; ++i) {
+        const CfBatchView& bv = b->views[i];
+        uint32_t C = 0;
+        const int s = validate_view(bv, i, &C);
+        if (s) return s;
+        cfgs[i] = config_for(b, bv.ubo.sliceCountX * bv.ubo.sliceCountY, bv.ubo.sliceCountZ);
+        if (cfk::is_mask_config(cfgs[i])) {
+            mask_views.push_back(i);
+            most_lights = std::max(most_lights, bv.light_count);
+        } else {
+            b->pos[i] = ns++;
+        }
+    }
+    std::stable_sort(mask_views.begin(), mask_views.end(),
+                     [&](uint32_t x, uint32_t y) { return b->views[x].light_count > b->views[y].light_count; });
+    for (size_t r = 0; r < mask_views.size(); ++r) b->pos[mask_views[r]] = ns + (uint32_t)r;
+    const uint32_t nm = (uint32_t)mask_views.size(), seg = cfk::mask_seg_lights(most_lights);
+    b->staged = ns;
+    std::vector<uint32_t> prefix(4 * (size_t)ns), mask_prefix(cfk::kMaskStages * ((size_t)nm + 1));
     size_t ws = 0;
     uint32_t xb = 0, bb = 0, cb = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const CfBatchView& bv = b->views[i];
-        uint32_t C = 0;
-        int s = validate_view(bv, i, &C);
-        if (s) return s;
-        const uint32_t xy = bv.ubo.sliceCountX * bv.ubo.sliceCountY, Z = bv.ubo.sliceCountZ;
-        const cfk::CullConfig cfg = config_for(b, xy);
-        const uint32_t gw = (uint32_t)(cfg.warps * cfg.clusters_per_warp);
-        const uint32_t groups = cfk::group_count(C, xy, Z, gw, true);
-        lay[i] = cfk::workspace_layout(C, bv.light_count, bv.max_lights_per_cluster, Z, true, groups);
-        ws_off[i] = ws;
-        ws += align256(lay[i].bytes);
-        cfk::ViewJob& j = b->jobs[i];
+        const uint32_t xy = bv.ubo.sliceCountX * bv.ubo.sliceCountY, Z = bv.ubo.sliceCountZ, C = xy * Z;
+        const bool mask = cfk::is_mask_config(cfgs[i]);
+        const uint32_t gw = cfk::group_width(cfgs[i]);
+        const uint32_t groups = cfk::group_count(C, xy, Z, gw, cfk::kModeBinned);
+        cfk::ViewJob& j = b->jobs[b->pos[i]];
         j.v.aabbs = reinterpret_cast<const float4*>(bv.d_aabbs);
         j.v.cells = bv.d_cells;
         j.v.indices = bv.d_indices;
@@ -198,21 +236,29 @@ int rebuild(CfBatch* b)
         j.lights = bv.d_lights;
         j.light_count = bv.light_count;
         for (int q = 0; q < 16; ++q) j.view[q] = bv.ubo.cameraView[q];
-        prefix[i] = xb;
-        prefix[2 * (size_t)n + i] = cb;
+        ws_off[i] = ws;
+        if (mask) {
+            mask_lay[i] = cfk::mask_layout(C, xy, Z, bv.light_count, bv.max_lights_per_cluster, seg);
+            ws += align256(mask_lay[i].bytes);
+        } else {
+            lay[i] = cfk::workspace_layout(C, bv.light_count, bv.max_lights_per_cluster, Z, cfk::kModeBinned, groups);
+            ws += align256(lay[i].bytes);
+            prefix[b->pos[i]] = xb;
+            prefix[2 * (size_t)ns + b->pos[i]] = cb;
+            xb += cfk::granules(j.v.lpad);
+            cb += cfk::copy_blocks(groups);
+        }
         aabb_jobs[i] = cfk::AabbJob{bv.ubo, bv.d_aabbs, 0};
         aabb_prefix[i] = ab;
         ab += (C + 255) / 256;
-        xb += cfk::granules(j.v.lpad);
-        cb += cfk::copy_blocks(groups);
     }
     // binning blocks: the views with the most lights first (a block reads all
     // of its view's lights, so those blocks run longest)
-    uint32_t* const order = prefix.data() + 3 * (size_t)n;
-    for (uint32_t i = 0; i < n; ++i) order[i] = i;
-    std::stable_sort(order, order + n, [&](uint32_t a, uint32_t c) { return b->jobs[a].light_count > b->jobs[c].light_count; });
-    for (uint32_t r = 0; r < n; ++r) {
-        prefix[n + r] = bb;
+    uint32_t* const order = prefix.data() + 3 * (size_t)ns;
+    for (uint32_t i = 0; i < ns; ++i) order[i] = i;
+    std::stable_sort(order, order + ns, [&](uint32_t a, uint32_t c) { return b->jobs[a].light_count > b->jobs[c].light_count; });
+    for (uint32_t r = 0; r < ns; ++r) {
+        prefix[ns + r] = bb;
         bb += cfk::bin_blocks(b->jobs[order[r]].v.slices);
     }
     b->xform_blocks = xb;
@@ -224,8 +270,12 @@ int rebuild(CfBatch* b)
     int s = grow(reinterpret_cast<void**>(&b->d_ws), &b->ws_cap, std::max<size_t>(ws, 256), "batch workspace");
     if (s) return s;
     for (uint32_t i = 0; i < n; ++i) {
-        cfk::ViewJob& j = b->jobs[i];
+        cfk::ViewJob& j = b->jobs[b->pos[i]];
         unsigned char* w = b->d_ws + ws_off[i];
+        if (b->pos[i] >= ns) {
+            cfk::mask_bind(j.v, mask_lay[i], w, seg, true);
+            continue;
+        }
         const cfk::WorkspaceLayout& L = lay[i];
         j.v.vlights = reinterpret_cast<const float4*>(w + L.vlights);
         j.v.nonfinite = reinterpret_cast<const uint32_t*>(w + L.nonfinite);
@@ -239,22 +289,50 @@ int rebuild(CfBatch* b)
         j.v.slice_nonfinite = reinterpret_cast<uint32_t*>(w + L.slice_nonfinite);
         j.v.group_boxes = reinterpret_cast<float4*>(w + L.group_boxes);
     }
+    b->mask = cfk::MaskBatch{};
+    b->mask.n_views = nm;
+    b->mask.seg_lights = seg;
+    for (int q = 0; q < cfk::kMaskStages; ++q) {
+        uint32_t* p = mask_prefix.data() + q * ((size_t)nm + 1);
+        uint64_t blocks = 0;
+        for (uint32_t r = 0; r < nm; ++r) {
+            p[r] = (uint32_t)blocks;
+            blocks += cfk::mask_batch_blocks(b->jobs[ns + r].v, (cfk::MaskStage)q);
+        }
+        if (blocks > 0x7fffffffull) return fail(CF_ERROR_INVALID_ARGUMENT, "the batch needs more blocks than a launch holds");
+        p[nm] = b->mask.blocks[q] = (uint32_t)blocks;
+    }
     // buckets and items: views by decreasing light count, groups in order
     std::map<uint32_t, std::vector<uint32_t>> by_key;
-    for (uint32_t i = 0; i < n; ++i) by_key[b->jobs[i].v.slice_clusters].push_back(i);
+    for (uint32_t i = 0; i < n; ++i) by_key[b->jobs[b->pos[i]].v.slice_clusters].push_back(b->pos[i]);
     if (by_key.size() > cfk::kMaxBatchQueues)
         return fail(CF_ERROR_INVALID_ARGUMENT, "%zu distinct grids exceed %u per batch", by_key.size(),
                     cfk::kMaxBatchQueues);
     // largest grids first: their items are the longest, so within a launch
     // shared with smaller grids they start in the first wave
     std::vector<uint2> items;
+    uint32_t mask_items = 0;
     b->buckets.clear();
     b->launches.clear();
     for (auto it = by_key.rbegin(); it != by_key.rend(); ++it) {
         std::vector<uint32_t>& vs = it->second;
+        // a bucket has one configuration, but for slices too many for the hit-mask path
+        uint32_t mask_ctas = 0, mask_groups = 0;
+        auto on_mask = [&](uint32_t q) { return q >= ns; };
+        for (uint32_t q : vs)
+            if (on_mask(q)) {
+                mask_ctas += cfk::mask_batch_blocks(b->jobs[q].v, cfk::kMaskScan);
+                mask_groups += b->jobs[q].v.groups;
+            }
+        vs.erase(std::remove_if(vs.begin(), vs.end(), on_mask), vs.end());
+        mask_items += mask_groups;
+        if (vs.empty()) {
+            b->buckets.push_back(CfBatch::Bucket{it->first, cfk::kMaskConfig, (uint32_t)items.size(), 0, (int)mask_ctas});
+            continue;
+        }
         std::stable_sort(vs.begin(), vs.end(),
                          [&](uint32_t x, uint32_t y) { return b->jobs[x].light_count > b->jobs[y].light_count; });
-        CfBatch::Bucket bk{it->first, config_for(b, it->first), (uint32_t)items.size(), 0, 0};
+        CfBatch::Bucket bk{it->first, staged_config(b, it->first), (uint32_t)items.size(), 0, 0};
         for (uint32_t vi : vs)
             for (uint32_t gi = 0; gi < b->jobs[vi].v.groups; ++gi) items.push_back(make_uint2(vi, gi));
         bk.item_count = (uint32_t)items.size() - bk.item_begin;
@@ -271,16 +349,20 @@ int rebuild(CfBatch* b)
             b->launches.push_back(CfBatch::Launch{bk.cfg, bk.item_begin, bk.item_count, bk.ctas});
         }
     }
-    b->n_items = (uint32_t)items.size();
+    b->n_items = (uint32_t)items.size() + mask_items;
     s = grow(reinterpret_cast<void**>(&b->d_jobs), &b->jobs_cap, std::max<size_t>(n, 1) * sizeof(cfk::ViewJob), "batch jobs");
-    if (!s) s = grow(reinterpret_cast<void**>(&b->d_prefix), &b->prefix_cap, std::max<size_t>(4 * (size_t)n, 1) * 4, "batch prefix");
+    if (!s) s = grow(reinterpret_cast<void**>(&b->d_prefix), &b->prefix_cap, std::max<size_t>(4 * (size_t)ns, 1) * 4, "batch prefix");
+    if (!s) s = grow(reinterpret_cast<void**>(&b->d_mask_prefix), &b->mask_prefix_cap, mask_prefix.size() * 4, "batch prefix");
     if (!s) s = grow(reinterpret_cast<void**>(&b->d_items), &b->items_cap, std::max<size_t>(items.size(), 1) * sizeof(uint2), "batch items");
     if (!s) s = grow(reinterpret_cast<void**>(&b->d_aabb_jobs), &b->aabb_jobs_cap, std::max<size_t>(n, 1) * sizeof(cfk::AabbJob), "batch AABB jobs");
     if (!s) s = grow(reinterpret_cast<void**>(&b->d_aabb_prefix), &b->aabb_prefix_cap, std::max<size_t>(n, 1) * 4, "batch AABB prefix");
     if (s) return s;
     cudaError_t e = cudaSuccess;
     if (n) e = cudaMemcpy(b->d_jobs, b->jobs.data(), n * sizeof(cfk::ViewJob), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && n) e = cudaMemcpy(b->d_prefix, prefix.data(), prefix.size() * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && ns) e = cudaMemcpy(b->d_prefix, prefix.data(), prefix.size() * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && nm) e = cudaMemcpy(b->d_mask_prefix, mask_prefix.data(), mask_prefix.size() * 4, cudaMemcpyHostToDevice);
+    b->mask.jobs = b->d_jobs + ns;
+    b->mask.prefix = b->d_mask_prefix;
     if (e == cudaSuccess && !items.empty())
         e = cudaMemcpy(b->d_items, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && n) e = cudaMemcpy(b->d_aabb_jobs, aabb_jobs.data(), n * sizeof(cfk::AabbJob), cudaMemcpyHostToDevice);
@@ -290,7 +372,9 @@ int rebuild(CfBatch* b)
 
 int enqueue_batch(CfBatch* b, cudaStream_t st)
 {
-    const uint32_t n = (uint32_t)b->views.size();
+    cudaError_t em = cfk::launch_mask_batch(b->mask, st);
+    if (em != cudaSuccess) return cuda_fail(em, "batch launch");
+    const uint32_t n = b->staged;
     if (n == 0) return CF_SUCCESS;
     const uint32_t* px = b->d_prefix;
     const uint32_t* pb = b->d_prefix + n;
@@ -380,6 +464,7 @@ int cf_batch_destroy(CfBatch* b)
     if (b->last_use) cudaEventDestroy(b->last_use);
     cudaFree(b->d_jobs);
     cudaFree(b->d_prefix);
+    cudaFree(b->d_mask_prefix);
     cudaFree(b->d_items);
     cudaFree(b->d_queues);
     cudaFree(b->d_ws);
@@ -404,7 +489,7 @@ int cf_batch_update_view_matrices(CfBatch* b, const CfClusterForwardUBO* ubos, u
     const int w = wait_idle(b);  // a pass queued on another stream may still read the table
     if (w) return w;
     for (uint32_t i = 0; i < n; ++i) {
-        for (int q = 0; q < 16; ++q) b->jobs[i].view[q] = ubos[i].cameraView[q];
+        for (int q = 0; q < 16; ++q) b->jobs[b->pos[i]].view[q] = ubos[i].cameraView[q];
         b->views[i].ubo = ubos[i];
     }
     // synchronous for a pageable source; the graph reads the table at replay
@@ -473,7 +558,7 @@ int cf_batch_autotune(CfBatch* b, int repeats, void* stream)
     int status = CF_SUCCESS;
     for (uint32_t key : keys) {
         float best = 1e30f;
-        cfk::CullConfig best_cfg = config_for(b, key);
+        cfk::CullConfig best_cfg = cfk::kMaskConfig;
         for (const cfk::CullConfig& c : kBatchCandidates) {
             b->tuned[key] = c;
             if ((status = rebuild(b))) break;

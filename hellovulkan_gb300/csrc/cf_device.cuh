@@ -70,6 +70,18 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t x, uint32_t lan
     return x;
 }
 
+// Index of the view whose range [prefix[v], prefix[v+1]) holds block b.
+__device__ __forceinline__ uint32_t find_view(const uint32_t* __restrict__ prefix, uint32_t n_views, uint32_t b)
+{
+    uint32_t lo = 0, hi = n_views;  // prefix[lo] <= b < prefix[hi]
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(&prefix[mid]) <= b) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
 // Exact for every finite light coordinate against boxes with min <= max on
 // each axis (or NaN bounds), which every generated AABB satisfies:
 //   v < min:  max3(min - v, v - max, 0) = min - v
@@ -162,6 +174,31 @@ __device__ __forceinline__ void hit_pair(f2 lx, f2 ly, f2 lz, float ar2, float b
     f2_unpack(sq, sa, sb);
     ha = sa < ar2;
     hb = sb < br2;
+}
+
+// hit_fast for two lights against one box: the differences and squares packed,
+// the sums scalar.  The compiler merges a packed product and a packed sum into
+// one packed FMA, rounding once where the shader rounds twice (a light one ulp
+// from a box's reach then changes sides), also under -fmad=false and however
+// the two are written; a scalar __fadd_rn it leaves alone.
+__device__ __forceinline__ void hit_pair_twice_rounded(f2 lx, f2 ly, f2 lz, float ar2, float br2, f2 mnx, f2 mny, f2 mnz,
+                                                       f2 mxx, f2 mxy, f2 mxz, bool& ha, bool& hb)
+{
+    float a0, a1, b0, b1, xa, xb, ya, yb, za, zb;
+    f2_unpack(f2_sub(mnx, lx), a0, a1);
+    f2_unpack(f2_sub(lx, mxx), b0, b1);
+    const f2 dx = f2_pack(max3f(a0, b0, 0.0f), max3f(a1, b1, 0.0f));
+    f2_unpack(f2_sub(mny, ly), a0, a1);
+    f2_unpack(f2_sub(ly, mxy), b0, b1);
+    const f2 dy = f2_pack(max3f(a0, b0, 0.0f), max3f(a1, b1, 0.0f));
+    f2_unpack(f2_sub(mnz, lz), a0, a1);
+    f2_unpack(f2_sub(lz, mxz), b0, b1);
+    const f2 dz = f2_pack(max3f(a0, b0, 0.0f), max3f(a1, b1, 0.0f));
+    f2_unpack(f2_mul(dx, dx), xa, xb);
+    f2_unpack(f2_mul(dy, dy), ya, yb);
+    f2_unpack(f2_mul(dz, dz), za, zb);
+    ha = __fadd_rn(__fadd_rn(xa, ya), za) < ar2;
+    hb = __fadd_rn(__fadd_rn(xb, yb), zb) < br2;
 }
 
 }  // namespace cfk

@@ -31,10 +31,10 @@
 // explicit round-to-nearest intrinsic, so nothing is contracted into an FMA.
 #include "cf_kernels.cuh"
 #include "cf_device.cuh"
+#include "cf_launch.cuh"
 
 #include <algorithm>
 #include <atomic>
-#include <utility>
 
 #include "cf_pinned_math.h"
 
@@ -236,18 +236,6 @@ __global__ void __launch_bounds__(kFlagGranule) light_xform_kernel(const CfLight
     grid_dependency_wait();
     launch_dependents();
     light_xform_body(lights, count, lpad, view.m, out, nonfinite, blockIdx.x);
-}
-
-// Index of the view whose range [prefix[v], prefix[v+1]) holds block b.
-__device__ __forceinline__ uint32_t find_view(const uint32_t* __restrict__ prefix, uint32_t n_views, uint32_t b)
-{
-    uint32_t lo = 0, hi = n_views;  // prefix[lo] <= b < prefix[hi]
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(&prefix[mid]) <= b) lo = mid;
-        else hi = mid;
-    }
-    return lo;
 }
 
 // Batched light transform: block b is granule b - prefix[v] of view v.  Block
@@ -1365,28 +1353,6 @@ __global__ void __launch_bounds__(kCopyWarps * 32) batch_copy_kernel(const ViewJ
     copy_body(jobs[vi].v, blockIdx.x - __ldg(&prefix[vi]));
 }
 
-// Launches `kernel`; with `overlap`, with programmatic stream serialisation
-// (see grid_dependency_wait): it may be scheduled while the stream's previous
-// kernel is still running.  A single view's step uses it.  Batched passes do
-// not: their kernels are long, and with several streams in flight (the
-// server) CTAs launched early would hold SM slots while they wait.
-template <typename... Params, typename... Args>
-cudaError_t launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
-                         cudaStream_t stream, Args&&... args)
-{
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = overlap ? attr : nullptr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 template <int K, int WARPS, int TILE, int STAGES, bool kBinned>
 cudaError_t launch_cull_t(const ViewCull& v, uint32_t* dev_error, cudaStream_t stream)
 {
@@ -1448,6 +1414,7 @@ cudaError_t launch_cull_t(const ViewCull& v, uint32_t* dev_error, cudaStream_t s
 
 bool cull_config_supported(const CullConfig& c)
 {
+    if (is_mask_config(c)) return true;
     if (c.binned == kModeOneLaunch)
         return c.clusters_per_warp >= 1 && (uint32_t)c.clusters_per_warp <= kOneLaunchMaxClustersPerCta &&
                c.stages == 1 && one_launch_shape_supported(c.warps, c.tile);
@@ -1458,18 +1425,35 @@ bool cull_config_supported(const CullConfig& c)
     return false;
 }
 
-// Slice binning pays off once a view has enough tests to amortise its extra
-// launch and passes: on a GB300 the 2560x1600 32x18x48 view with 16384
-// lights (453 M tests) culls five times faster binned than brute force.
-// Below that, a view whose lights fit one launch's registers (at most
+// Where the lines lie (GB300, back-to-back passes, brute force against the
+// hit-mask path, which takes 16 to 20 us whatever the size of a small view:
+// its five dependent launches are what it costs):
+//   lights   3456 clusters, 2604 lights (9 M tests)   23.9 against 19.5 us
+//            1024 clusters, 2929 lights (3 M)         21.7          19.4
+//            3105 clusters, 2254 lights (7 M)         20.9          20.0
+//            the brute-force kernel's time grows with the lights each warp
+//            streams, so above kMaskMinLights the hit-mask path always wins
+//   tests    27648 clusters, 434 lights (12 M)        19.0          18.1
+//            10752 clusters, 1116 lights (12 M)       20.0          18.4
+//            10752 clusters,  837 lights (9 M)        16.9          18.8
+// Below both lines, a view whose lights fit one launch's registers (at most
 // kOneLaunchMaxLights) and whose clusters spread over the resident CTAs at
 // most kOneLaunchMaxClustersPerCta each is culled in one launch; the rest
-// brute force.
-constexpr uint64_t kBinnedMinTests = 16ull << 20;
+// brute force.  Grids beyond the hit-mask path's limits (mask_fits) take the
+// staged binned path once it pays: 453 M tests cull five times faster with it
+// than brute force, 16 M about the same.
+constexpr uint32_t kMaskMinLights = 2560;
+constexpr uint64_t kMaskMinTests = 10ull << 20;
+constexpr uint64_t kStagedMinTests = 16ull << 20;
 
 CullConfig default_cull_config(uint32_t clusters, uint32_t lights, uint32_t slices)
 {
-    if (slices >= 2 && (uint64_t)clusters * lights >= kBinnedMinTests) return CullConfig{2, 8, 1024, 2, 1};
+    const uint64_t tests = (uint64_t)clusters * lights;
+    if (slices >= 2 && mask_fits(clusters, clusters / slices, slices)) {
+        if (lights >= kMaskMinLights || tests >= kMaskMinTests) return kMaskConfig;
+    } else if (slices >= 2 && tests >= kStagedMinTests) {
+        return kStagedConfig;
+    }
     CullConfig one{};
     if (one_launch_config(clusters, lights, &one)) return one;
     if (clusters <= 8192) return CullConfig{1, 8, 512, 4, 0};

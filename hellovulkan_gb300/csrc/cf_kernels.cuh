@@ -75,6 +75,26 @@ struct ViewCull {
     uint32_t* group_sums;     // capped hit count of each group (plain path)
     uint32_t* group_offsets;  // exclusive scan of group_sums (plain path)
     uint32_t* queue;          // single-view binned launch: item counter, zeroed by the binning launch
+    // hit-mask path (cf_mask.cu): slice_lights / slice_idx hold, per slice, one
+    // part per segment of seg_lights lights, from entry segment * seg_lights
+    float4* slice_boxes;             // per slice: the union of its boxes (lo, hi)
+    uint32_t* seg_count;             // [slice * segs + segment]: lights listed
+    uint32_t* slice_total;           // per slice: lights listed
+    uint32_t* slice_first;           // the scan's plan (see Plan)
+    uint32_t* group_total;           // per group: hits
+    uint16_t* group_count;           // per group and cluster: hits
+    uint32_t* block_total;           // per 32 groups: hits
+    uint32_t* unit_run;              // per unit: its batches in the pool, or a mark
+    uint8_t* unit_count;             // per unit and cluster: hits (at most kMaskMaxRun)
+    uint16_t* unit_before;           // ... and the hits in the group's earlier units, cut at the cap
+    uint32_t* pool;                  // the units' masks and light indices, in batches
+    unsigned long long* pool_head;   // batches asked for
+    uint32_t pool_batches;
+    uint32_t max_units;              // units the workspace holds
+    uint32_t run;                    // candidates per unit, at first (see Plan)
+    uint32_t seg_lights;
+    uint32_t segs;
+    uint32_t list_slices;            // slices a list CTA takes
     uint32_t lpad;
     uint32_t clusters;
     uint32_t cap;
@@ -134,6 +154,38 @@ inline uint32_t group_width(const CullConfig& c)
     return c.binned == kModeOneLaunch ? (uint32_t)c.clusters_per_warp : (uint32_t)(c.warps * c.clusters_per_warp);
 }
 
+// The hit-mask path (cf_mask.cu) as a configuration of the binned mode: 32
+// clusters per group, 32 lights per mask, no staging (1 stage).
+constexpr CullConfig kMaskConfig{4, 8, 32, 1, kModeBinned};
+constexpr CullConfig kStagedConfig{2, 8, 1024, 2, kModeBinned};  // the staged binned path's own default
+// Most groups the automatic choice gives the hit-mask path: a group reads the
+// totals of earlier groups as sums of 32, so their number grows with the view.
+constexpr uint32_t kMaskMaxGroups = 32768;
+constexpr uint32_t kMaskMaxSlices = 1024;  // slices whose first units a scanning CTA keeps in shared memory
+constexpr uint32_t kMaskMaxRun = 128;      // most candidates per scanning unit
+constexpr uint32_t kMaskGroup = 32;      // clusters per group
+constexpr uint32_t kMaxSegLights = 1024; // most lights per list segment
+inline bool is_mask_config(const CullConfig& c)
+{
+    return c.clusters_per_warp == kMaskConfig.clusters_per_warp && c.warps == kMaskConfig.warps &&
+           c.tile == kMaskConfig.tile && c.stages == kMaskConfig.stages && c.binned == kMaskConfig.binned;
+}
+inline uint32_t mask_segments(uint32_t lpad, uint32_t seg_lights) { return (lpad + seg_lights - 1) / seg_lights; }
+
+// Scratch of one view on the hit-mask path.
+struct MaskLayout {
+    size_t slice_first, group_total, group_count, block_total, group_boxes, slice_boxes, seg_count, pool_head, slice_total, unit_run,
+        unit_count, unit_before, pool, slice_lights, slice_idx, bytes;
+    uint32_t pool_batches;
+    uint32_t max_units;
+};
+MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slices, uint32_t lights, uint32_t cap,
+                       uint32_t seg_lights);
+// Points v's hit-mask buffers into a workspace (v.lpad set).
+void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg_lights, bool batch);
+// Lights per list segment for a view of its own.
+uint32_t mask_seg_lights(uint32_t lights);
+
 // Workspace carve-up for one view (cf_cull_lights).  A one-launch view needs
 // only the status block and one 8-byte word per CTA (`partials`).
 struct WorkspaceLayout {
@@ -145,6 +197,11 @@ constexpr size_t kEpochWord = 128;  // byte offset of the one-launch kernel's ep
 // Scratch of one view; `groups` = group_count(...) of the configuration used.
 WorkspaceLayout workspace_layout(uint32_t clusters, uint32_t lights, uint32_t cap, uint32_t slices, int mode,
                                  uint32_t groups);
+
+inline bool mask_fits(uint32_t clusters, uint32_t slice_clusters, uint32_t slices)
+{
+    return slices <= kMaskMaxSlices && group_count(clusters, slice_clusters, slices, kMaskGroup, kModeBinned) <= kMaskMaxGroups;
+}
 
 // One-launch culling of a small view (cf_fused.cu): light transform,
 // LightCulling.comp's test for every (cluster, light) pair, the capped
@@ -199,6 +256,10 @@ cudaError_t launch_light_xform(const CfLightData* lights, uint32_t count, const 
 cudaError_t launch_bin(const ViewCull& v, cudaStream_t stream);
 cudaError_t launch_cull(const ViewCull& v, const CullConfig& cfg, uint32_t* dev_error, cudaStream_t stream);
 cudaError_t launch_finalize(const ViewCull& v, cudaStream_t stream);
+// Hit-mask path of one view: union boxes and candidate lists; the tests; the output.
+cudaError_t launch_mask_lists(const ViewJob& j, cudaStream_t stream);
+cudaError_t launch_mask_scan(const ViewJob& j, cudaStream_t stream);
+cudaError_t launch_mask_emit(const ViewJob& j, cudaStream_t stream);
 // total, cells and min(total, capacity) indices of one view into device-addressable host memory
 cudaError_t launch_readback(const CfLightCell* cells, uint32_t clusters, const uint32_t* indices,
                             const uint32_t* d_total, uint64_t capacity, CfLightCell* h_cells, uint32_t* h_indices,
@@ -255,6 +316,17 @@ cudaError_t launch_batch_bin(const ViewJob* jobs, const uint32_t* prefix, const 
                              uint32_t blocks, cudaStream_t stream);
 cudaError_t launch_batch_cull(const BatchCull& b, const CullConfig& cfg, int ctas, uint32_t* dev_error,
                               cudaStream_t stream);
+// The hit-mask path of many views: per stage, view v owns blocks
+// [prefix[v], prefix[v + 1]) of the launch (n_views + 1 entries per stage).
+enum MaskStage { kMaskBox, kMaskList, kMaskScan, kMaskSum, kMaskEmit, kMaskStages };
+struct MaskBatch {
+    const ViewJob* jobs;
+    const uint32_t* prefix;
+    uint32_t n_views, seg_lights;
+    uint32_t blocks[kMaskStages];
+};
+uint32_t mask_batch_blocks(const ViewCull& v, MaskStage stage);
+cudaError_t launch_mask_batch(const MaskBatch& b, cudaStream_t stream);
 cudaError_t batch_cull_resident_ctas(const CullConfig& cfg, int* ctas);
 cudaError_t launch_batch_scan(const ViewJob* jobs, uint32_t n_views, cudaStream_t stream);
 cudaError_t launch_batch_copy(const ViewJob* jobs, const uint32_t* prefix, uint32_t n_views, uint32_t blocks,

@@ -1,0 +1,915 @@
+// cf_mask.cu — binned culling with hit masks (LightCulling.comp:26-87): five
+// launches from lights and AABBs to cells and the packed index list, for one
+// view or for every view of a batch.
+//
+//   box_kernel     one CTA per depth slice: the union box of the slice and of
+//                  each group of 32 consecutive clusters, and the reset of
+//                  the words that the later launches count in
+//   list_kernel    one CTA per segment of lights and block of slices:
+//                  transforms its lights (posView = cameraView * position,
+//                  r^2) and writes, per slice, those whose sphere reaches the
+//                  slice's box, in light order, into the segment's own part of
+//                  the slice's list.  No segment needs another's count.
+//   scan_kernel    warps take units, each a run of a slice's candidates against
+//                  one group: the warp keeps the lights that reach the group's
+//                  union box and tests each of them against 32 clusters, one
+//                  per lane; a lane's results for 32 lights are one mask word
+//                  in shared memory.  The masks and the lights' indices go to
+//                  the view's pool.  No warp waits for another, and a dense
+//                  group's work spreads over many.
+//   sum_kernel     one CTA per group: adds up the units' counts
+//   emit_kernel    warps write the groups' cells, and the units' hits from
+//                  their masks straight to their places in the packed list
+//
+// Why this split.  A view's hits are concentrated: on the 2560x1600 view with
+// 16384 lights one group of 864 has a twentieth of all (light, group) pairs, and
+// half the slices none.  CTAs that own a group and take its candidates in
+// tiles (cull_pipe_kernel) are bound by the longest ones; here the longest unit
+// is 128 candidates, units of one group go to different SMs, and slices that
+// nothing reaches cost nothing.  What is left is latency: the five launches of
+// a single view overlap by programmatic dependent launch, and each is a chain
+// of two to five L2 round trips (0.5 us each) with 0.9 us to the next launch.
+// Batches are bound by issue (2.2 to 2.8 of 4 instructions per cycle in the
+// list and scan launches).  Measured, back-to-back passes, against the staged
+// path: that view 33.8 -> 22.8 us; 65536 lights 77.4 -> 36.5 us; 64 views of the
+// benchmark's mix 367 -> 188 us; 256 animated views of 4096 lights
+// 1474 -> 537 us.
+//
+// The tests are the ones of cf_device.cuh; pruning by union box is exact: per
+// axis the distance to a box that contains another is never larger, and the
+// rounded squares and sums are monotonic.  A NaN bound makes a union infinite.
+#include "cf_kernels.cuh"
+#include "cf_device.cuh"
+#include "cf_launch.cuh"
+
+#include <algorithm>
+
+#include "cf_pinned_math.h"
+
+namespace cfk {
+namespace {
+
+constexpr uint32_t kGroup = kMaskGroup;  // clusters per group: one per lane
+
+// ---------------------------------------------------------------------------
+// Slice and group boxes.
+// ---------------------------------------------------------------------------
+// threads per slice: a view's own launch reduces up to 1024 clusters in one
+// step; a batch has slices enough to fill the GPU with smaller CTAs
+constexpr uint32_t kBoxThreads = 1024, kBoxThreadsBatch = 256;
+
+__device__ __forceinline__ float4 min4(float4 a, float4 b)
+{
+    return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.f);
+}
+__device__ __forceinline__ float4 max4(float4 a, float4 b)
+{
+    return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), 0.f);
+}
+
+// The union of the lanes' boxes, in every lane.
+__device__ __forceinline__ void warp_union(float4& lo, float4& hi)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo.x = fminf(lo.x, __shfl_xor_sync(kFull, lo.x, o));
+        lo.y = fminf(lo.y, __shfl_xor_sync(kFull, lo.y, o));
+        lo.z = fminf(lo.z, __shfl_xor_sync(kFull, lo.z, o));
+        hi.x = fmaxf(hi.x, __shfl_xor_sync(kFull, hi.x, o));
+        hi.y = fmaxf(hi.y, __shfl_xor_sync(kFull, hi.y, o));
+        hi.z = fmaxf(hi.z, __shfl_xor_sync(kFull, hi.z, o));
+    }
+}
+
+template <uint32_t kThreads>
+__device__ __forceinline__ void box_body(const ViewCull& v, uint32_t k)
+{
+    constexpr uint32_t kWarps = kThreads / 32;
+    __shared__ float4 s_lo[kWarps], s_hi[kWarps];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t xy = v.slice_clusters, gps = (xy + kGroup - 1) / kGroup;
+    const float inf = __uint_as_float(0x7f800000u);
+    const uint32_t blocks = (v.groups + kGroup - 1) / kGroup;
+    for (uint32_t u = k + v.slices * threadIdx.x; u < blocks; u += v.slices * kThreads) v.block_total[u] = 0u;
+    if (threadIdx.x == 0) {
+        v.slice_total[k] = 0u;
+        if (k == 0) *v.pool_head = 0ull;
+    }
+    float4 lo = make_float4(inf, inf, inf, 0.f), hi = make_float4(-inf, -inf, -inf, 0.f);
+    for (uint32_t g = warp; g < gps; g += kWarps) {
+        const uint32_t c = g * kGroup + lane;
+        float4 a = make_float4(inf, inf, inf, 0.f), b = make_float4(-inf, -inf, -inf, 0.f);
+        if (c < xy) {
+            a = __ldg(&v.aabbs[2 * ((size_t)k * xy + c)]);
+            b = __ldg(&v.aabbs[2 * ((size_t)k * xy + c) + 1]);
+        }
+        const bool nan = (a.x != a.x) | (a.y != a.y) | (a.z != a.z) | (b.x != b.x) | (b.y != b.y) | (b.z != b.z);
+        warp_union(a, b);
+        if (__any_sync(kFull, nan)) {
+            a = make_float4(-inf, -inf, -inf, 0.f);
+            b = make_float4(inf, inf, inf, 0.f);
+        }
+        lo = min4(lo, a);
+        hi = max4(hi, b);
+        if (lane == 0) {
+            v.group_boxes[2 * ((size_t)k * gps + g)] = a;
+            v.group_boxes[2 * ((size_t)k * gps + g) + 1] = b;
+        }
+    }
+    if (lane == 0) {
+        s_lo[warp] = lo;
+        s_hi[warp] = hi;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        lo = s_lo[lane % kWarps];
+        hi = s_hi[lane % kWarps];
+        warp_union(lo, hi);
+        if (lane == 0) {
+            v.slice_boxes[2 * k] = lo;
+            v.slice_boxes[2 * k + 1] = hi;
+        }
+    }
+}
+
+template <uint32_t kThreads>
+__global__ void __launch_bounds__(kThreads) box_kernel(const ViewJob* __restrict__ jobs,
+                                                            const uint32_t* __restrict__ prefix, uint32_t n_views,
+                                                            const __grid_constant__ ViewJob single)
+{
+    grid_dependency_wait();
+    // after the wait: the list launch starts once every earlier launch has
+    // finished, so it may read the lights before its own wait
+    launch_dependents();
+    if (jobs) {
+        const uint32_t vi = find_view(prefix, n_views, blockIdx.x);
+        box_body<kThreads>(jobs[vi].v, blockIdx.x - __ldg(&prefix[vi]));
+    } else {
+        box_body<kThreads>(single.v, blockIdx.x);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Candidate lists.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kListSlices = 16;         // most slices per CTA
+
+__device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
+{
+    __shared__ uint32_t s_mask[kListSlices][32];
+    __shared__ uint32_t s_off[kListSlices][32];
+    __shared__ float4 s_box[2 * kListSlices];
+    const ViewCull& v = j.v;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const uint32_t seg = blk % v.segs, z0 = (blk / v.segs) * v.list_slices;
+    const uint32_t nz = min(v.list_slices, v.slices - z0);
+    const uint32_t i = seg * v.seg_lights + tid;
+    float4 L = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0xff800000u));  // past the lights: reaches nothing
+    if (i < j.light_count) {
+        // Read before the wait below: the box launch lets this one start only
+        // once every earlier launch has finished.  From L2, not from an L1
+        // that may hold the lights of an earlier frame.
+        const float4 p = __ldcg(reinterpret_cast<const float4*>(&j.lights[i].position[0]));
+        const float r = __ldcg(&j.lights[i].radius);
+        L.x = cf_mat4_row(j.view, 0, p.x, p.y, p.z, p.w);
+        L.y = cf_mat4_row(j.view, 1, p.x, p.y, p.z, p.w);
+        L.z = cf_mat4_row(j.view, 2, p.x, p.y, p.z, p.w);
+        L.w = cf_fmul(r, r);
+    }
+    grid_dependency_wait();  // the boxes
+    launch_dependents();
+    if (tid < 2 * nz) s_box[tid] = v.slice_boxes[2 * z0 + tid];
+    __syncthreads();
+    const bool lights = seg * v.seg_lights + warp * 32 < j.light_count;  // whether the warp has any
+    for (uint32_t q = 0; q < nz; ++q) {
+        if (!lights) {
+            if (lane == 0) s_mask[q][warp] = 0u;
+            continue;
+        }
+        const float4 lo = s_box[2 * q], hi = s_box[2 * q + 1];
+        const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
+        const uint32_t m = __ballot_sync(kFull, hit_fast(L, mn, mx));
+        if (lane == 0) s_mask[q][warp] = m;
+    }
+    __syncthreads();
+    for (uint32_t q = warp; q < nz; q += nw) {
+        const uint32_t c = lane < nw ? __popc(s_mask[q][lane]) : 0u;
+        const uint32_t incl = warp_inclusive_scan(c, lane);
+        s_off[q][lane] = incl - c;
+        if (lane == 31) {
+            v.seg_count[(size_t)(z0 + q) * v.segs + seg] = incl;
+            if (incl) atomicAdd(&v.slice_total[z0 + q], incl);
+        }
+    }
+    __syncthreads();
+    for (uint32_t q = 0; lights && q < nz; ++q) {
+        const uint32_t m = s_mask[q][warp];
+        if ((m >> lane) & 1u) {
+            const size_t at = (size_t)(z0 + q) * v.lpad + seg * v.seg_lights + s_off[q][warp] +
+                              __popc(m & ((1u << lane) - 1u));
+            v.slice_lights[at] = L;
+            v.slice_idx[at] = i;
+        }
+    }
+    if (v.work && tid == 0) atomicAdd(&v.work[0], (unsigned long long)nz * blockDim.x);
+}
+
+__global__ void __launch_bounds__(kMaxSegLights, 2) list_kernel(const ViewJob* __restrict__ jobs,
+                                                             const uint32_t* __restrict__ prefix, uint32_t n_views,
+                                                             const __grid_constant__ ViewJob single)
+{
+    if (jobs) {
+        const uint32_t vi = find_view(prefix, n_views, blockIdx.x);
+        list_body(jobs[vi], blockIdx.x - __ldg(&prefix[vi]));
+    } else {
+        list_body(single, blockIdx.x);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Scanning.
+// ---------------------------------------------------------------------------
+
+// Per-thread asynchronous copies: a thread waits only for its own.
+__device__ __forceinline__ void async16(void* dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void async4(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+constexpr uint32_t kBank = kMaskMaxRun / 32;  // most chunks of 32 candidates per unit
+
+// Shared memory of one warp: the unit's candidates (each lane copies and reads
+// only its own), its pending survivors (a ring of 64, one array per component
+// so that four lights' x are one 16-byte read), the light indices of its
+// survivors and their mask words.
+struct ScanWarp {
+    float4 in[kBank][32];
+    float x[64], y[64], z[64], r2[64];
+    uint32_t in_idx[kBank][32];
+    uint32_t idx[32 * kBank];
+    uint32_t word[kBank][32];
+};
+
+// One lane's cluster box, each bound in both halves of a packed pair.
+struct LaneBox {
+    f2 mnx, mny, mnz, mxx, mxy, mxz;
+};
+
+// Mask of the n pending survivors from ring position `at` that reach this
+// lane's box.  Four lights per step, two per packed operation; the ring is
+// padded with never-hit lights to a multiple of four.
+__device__ __forceinline__ uint32_t test_pending(const ScanWarp& s, uint32_t at, uint32_t n, const LaneBox& b)
+{
+    uint32_t word = 0;
+#pragma unroll 2
+    for (uint32_t j = 0; j < n; j += 4) {
+        const uint32_t p = (at + j) & 63u;  // `at` is a multiple of 32
+        const float4 x = *reinterpret_cast<const float4*>(&s.x[p]);
+        const float4 y = *reinterpret_cast<const float4*>(&s.y[p]);
+        const float4 z = *reinterpret_cast<const float4*>(&s.z[p]);
+        const float4 r2 = *reinterpret_cast<const float4*>(&s.r2[p]);
+        bool h0, h1, h2, h3;
+        hit_pair_twice_rounded(f2_pack(x.x, x.y), f2_pack(y.x, y.y), f2_pack(z.x, z.y), r2.x, r2.y, b.mnx, b.mny, b.mnz,
+                               b.mxx, b.mxy, b.mxz, h0, h1);
+        hit_pair_twice_rounded(f2_pack(x.z, x.w), f2_pack(y.z, y.w), f2_pack(z.z, z.w), r2.z, r2.w, b.mnx, b.mny, b.mnz,
+                               b.mxx, b.mxy, b.mxz, h2, h3);
+        word |= ((h0 ? 1u : 0u) | (h1 ? 2u : 0u) | (h2 ? 4u : 0u) | (h3 ? 8u : 0u)) << j;
+    }
+    return word;
+}
+
+// The same with the shader's branchy test, for survivors that include a
+// non-finite coordinate.
+__device__ __noinline__ uint32_t test_pending_exact(const ScanWarp& s, uint32_t at, uint32_t n, const float4 lo,
+                                                    const float4 hi)
+{
+    const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
+    uint32_t word = 0;
+    for (uint32_t j = 0; j < n; ++j) {
+        const uint32_t p = (at + j) & 63u;
+        if (hit_exact(make_float4(s.x[p], s.y[p], s.z[p], s.r2[p]), mn, mx)) word |= 1u << j;
+    }
+    return word;
+}
+
+// Writes the hits of 32 lights (`word`: the lane's cluster's mask, idx: the
+// lights' indices) in light order at the lane's next place `pos`, up to `lim`,
+// four at a time; returns the place after them.
+__device__ __forceinline__ uint32_t emit_word(uint32_t word, const uint32_t* idx, uint32_t* __restrict__ out,
+                                              uint32_t pos, uint32_t lim)
+{
+    const uint32_t n = min((uint32_t)__popc(word), lim - min(pos, lim));
+    for (uint32_t t = 0; t < n; t += 4) {
+        uint32_t x[4];
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+            x[e] = idx[(__ffs(word) - 1) & 31];
+            word &= word - 1;
+        }
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e)
+            if (t + e < n) out[pos + t + e] = x[e];
+    }
+    return pos + n;
+}
+
+// One group as a warp sees it: lane i holds cluster i.
+struct GroupLane {
+    float4 lo, hi, ulo, uhi;  // the lane's box (+inf past the slice), the group's union box
+    LaneBox box;
+    bool present;
+};
+
+__device__ __forceinline__ GroupLane load_group(const ViewCull& v, uint32_t g, uint32_t k, uint32_t lane)
+{
+    const uint32_t xy = v.slice_clusters, gps = (xy + kGroup - 1) / kGroup;
+    const uint32_t c = k * xy + (g - k * gps) * kGroup + lane;
+    const float inf = __uint_as_float(0x7f800000u);
+    GroupLane q;
+    q.present = c < (k + 1) * xy;
+    q.lo = q.hi = make_float4(inf, inf, inf, 0.f);
+    if (q.present) {
+        q.lo = __ldg(&v.aabbs[2 * (size_t)c]);
+        q.hi = __ldg(&v.aabbs[2 * (size_t)c + 1]);
+    }
+    q.ulo = __ldg(&v.group_boxes[2 * (size_t)g]);
+    q.uhi = __ldg(&v.group_boxes[2 * (size_t)g + 1]);
+    q.box = LaneBox{f2_pack(q.lo.x, q.lo.x), f2_pack(q.lo.y, q.lo.y), f2_pack(q.lo.z, q.lo.z),
+                    f2_pack(q.hi.x, q.hi.x), f2_pack(q.hi.y, q.hi.y), f2_pack(q.hi.z, q.hi.z)};
+    return q;
+}
+
+// Starts the copies of candidates [t0, t0 + n) of slice k's list, n <= kMaskMaxRun,
+// into s.  The list is one part per segment: lane i of a window of 32 segments
+// holds segment i's first position in the list as a whole, and each lane finds
+// its candidates' segments by a binary search over the lanes.
+__device__ __forceinline__ void fetch_candidates(const ViewCull& v, ScanWarp& s, uint32_t k, uint32_t t0, uint32_t n,
+                                                 uint32_t lane)
+{
+    const uint32_t* __restrict__ counts = v.seg_count + (size_t)k * v.segs;
+    const float4* __restrict__ lists = v.slice_lights + (size_t)k * v.lpad;
+    const uint32_t* __restrict__ lists_i = v.slice_idx + (size_t)k * v.lpad;
+    uint32_t base = 0;  // candidates before the window
+    for (uint32_t w0 = 0; w0 < v.segs && base < t0 + n; w0 += 32) {
+        const uint32_t c = w0 + lane < v.segs ? __ldg(&counts[w0 + lane]) : 0u;
+        const uint32_t incl = warp_inclusive_scan(c, lane);
+        const uint32_t first = base + incl - c, end = base + __shfl_sync(kFull, incl, 31);
+        if (end > t0) {
+#pragma unroll
+            for (uint32_t b = 0; b < kBank; ++b) {
+                if (b * 32 >= n) break;
+                const uint32_t t = t0 + b * 32 + lane;
+                uint32_t i = 0;  // the last segment of the window that starts at or before t
+#pragma unroll
+                for (uint32_t step = 16; step; step >>= 1)
+                    if (__shfl_sync(kFull, first, i + step) <= t) i += step;
+                const uint32_t start = __shfl_sync(kFull, first, i);
+                if (b * 32 + lane < n && t >= base && t < end) {
+                    const uint32_t at = (w0 + i) * v.seg_lights + (t - start);
+                    async16(&s.in[b][lane], &lists[at]);
+                    async4(&s.in_idx[b][lane], &lists_i[at]);
+                }
+            }
+        }
+        base = end;
+    }
+    // the last chunk's absent lanes: lights that reach nothing
+    const uint32_t b = n / 32;
+    if (lane >= n % 32 && n % 32) s.in[b][lane] = make_float4(0.f, 0.f, 0.f, __uint_as_float(0xff800000u));
+}
+
+// A warp's pass over the unit of n candidates in s (see fetch_candidates).
+//   kEmit false  counts the lane's hits (no more than lim are needed) and keeps
+//                the mask words and indices
+//   kEmit true   writes the hits to out from place `count` up to lim
+// Returns the number of survivors tested.
+template <bool kEmit>
+__device__ __forceinline__ uint32_t scan_candidates(ScanWarp& s, uint32_t n, uint32_t lane, const GroupLane& q,
+                                                    uint32_t& count, uint32_t lim, uint32_t* __restrict__ out)
+{
+    const float inf = __uint_as_float(0x7f800000u);
+    const float umn[3] = {q.ulo.x, q.ulo.y, q.ulo.z}, umx[3] = {q.uhi.x, q.uhi.y, q.uhi.z};
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    uint32_t ns = 0, done = 0;
+    bool full = __all_sync(kFull, count >= lim);  // every lane has as many hits as its cluster can list
+    auto flush = [&](uint32_t m) {
+        // pad to a multiple of four with lights that reach nothing
+        if ((m & 3u) && lane < 4u - (m & 3u)) {
+            const uint32_t p = (done + m + lane) & 63u;
+            s.x[p] = s.y[p] = s.z[p] = 0.0f;
+            s.r2[p] = -inf;
+        }
+        __syncwarp();
+        const uint32_t r = (done + lane) & 63u;
+        const bool bad = lane < m && !(finite_bits(s.x[r]) && finite_bits(s.y[r]) && finite_bits(s.z[r]));
+        uint32_t word = __any_sync(kFull, bad) ? test_pending_exact(s, done, m, q.lo, q.hi)
+                                               : test_pending(s, done, m, q.box);
+        if (!q.present) word = 0;
+        if constexpr (kEmit) {
+            count = emit_word(word, &s.idx[done], out, count, lim);
+        } else {
+            s.word[done / 32][lane] = word;
+            count += __popc(word);
+        }
+        full = __all_sync(kFull, count >= lim);
+        __syncwarp();
+        done += m;
+    };
+    async_wait_all();
+    for (uint32_t b = 0; b * 32 < n && !full; ++b) {
+        const float4 L = s.in[b][lane];
+        const bool pass = hit_fast(L, umn, umx);
+        const uint32_t m = __ballot_sync(kFull, pass);
+        if (!m) continue;
+        if (pass) {
+            const uint32_t p = ns + __popc(m & lt_mask);
+            s.x[p & 63u] = L.x;
+            s.y[p & 63u] = L.y;
+            s.z[p & 63u] = L.z;
+            s.r2[p & 63u] = L.w;
+            s.idx[p] = s.in_idx[b][lane];
+        }
+        ns += __popc(m);
+        if (ns - done >= 32) flush(32);
+    }
+    if (ns > done && !full) flush(ns - done);
+    return done;
+}
+
+// unit_run: the unit's first batch in the pool and, from bit kBatchShift, its
+// batches less one; or a mark.  A batch is the 32 mask words (one per cluster)
+// of 32 survivors and the survivors' indices.
+constexpr uint32_t kBatchShift = 28;
+constexpr uint32_t kNoHits = 0xffffffffu;  // the unit has no hit
+constexpr uint32_t kNoRun = 0xfffffffeu;   // ... has hits, but the pool had no room for them
+constexpr uint32_t kBatchWords = 64;
+constexpr int kScanWarps = 4;
+
+// Which unit a warp has: run r (of `runs`) of group g in slice k, n candidates
+// from t0 of the slice's list.
+struct Unit {
+    uint32_t u, k, g, r, runs, t0, n;
+};
+
+__device__ __forceinline__ void scan_unit(const ViewCull& v, const Unit& a, ScanWarp& s, uint32_t lane)
+{
+    const uint32_t cap = v.cap, u = a.u, n = a.n;
+    fetch_candidates(v, s, a.k, a.t0, n, lane);
+    const GroupLane q = load_group(v, a.g, a.k, lane);
+    uint32_t count = q.present ? 0u : cap;
+    const uint32_t survivors = scan_candidates<false>(s, n, lane, q, count, cap, nullptr);
+    if (v.work && lane == 0) {
+        atomicAdd(&v.work[0], (unsigned long long)((n + 31) & ~31u));
+        atomicAdd(&v.work[1], 32ull * survivors);
+    }
+    const uint32_t mine = q.present ? min(count, cap) : 0u;
+    const bool hits = __any_sync(kFull, mine != 0);
+    v.unit_count[(size_t)u * kGroup + lane] = (uint8_t)mine;  // at most kMaskMaxRun
+    const uint32_t batches = (survivors + 31) / 32;
+    uint32_t run = kNoHits;
+    if (lane == 0) {
+        if (hits) {
+            const unsigned long long at = atomicAdd(v.pool_head, (unsigned long long)batches);
+            run = at + batches <= v.pool_batches ? (uint32_t)at | (batches - 1) << kBatchShift : kNoRun;
+        }
+        v.unit_run[u] = run;
+    }
+    run = __shfl_sync(kFull, run, 0);
+    if (hits && run != kNoRun) {
+        uint32_t* out = v.pool + (size_t)(run & ((1u << kBatchShift) - 1)) * kBatchWords + lane;
+        for (uint32_t b = 0; b < batches; ++b, out += kBatchWords) {
+            out[0] = s.word[b][lane];
+            out[32] = s.idx[b * 32 + lane];  // past the survivors: never read
+        }
+    }
+    __syncwarp();  // the next unit overwrites the masks
+}
+
+// The units of a view: first[k] is the first unit of slice k, first[slices]
+// their number; total[k] the slice's candidates; `run` the candidates per
+// unit.  Short runs spread a dense group's work over more warps; they are
+// lengthened when the view would then have more units than its workspace
+// holds, which runs of kMaskMaxRun never are.  Every block of the scan makes
+// the same plan; the first one leaves it in the workspace (slice_first, the
+// run last) for the later launches.
+struct Plan {
+    uint32_t first[kMaskMaxSlices + 1];
+    uint32_t total[kMaskMaxSlices];
+    uint32_t warp_units[kScanWarps];
+    uint32_t run;
+};
+
+__device__ __forceinline__ void make_plan(const ViewCull& v, uint32_t gps, Plan& p, bool keep)
+{
+    constexpr uint32_t kThreads = kScanWarps * 32;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (uint32_t run = v.run;; run *= 2) {
+        uint32_t base = 0;
+        for (uint32_t k0 = 0; k0 < v.slices; k0 += kThreads) {
+            const uint32_t k = k0 + tid, total = k < v.slices ? __ldg(&v.slice_total[k]) : 0u;
+            const uint32_t n = (total + run - 1) / run * gps, incl = warp_inclusive_scan(n, lane);
+            if (lane == 31) p.warp_units[warp] = incl;
+            __syncthreads();
+            uint32_t at = base + incl - n;
+#pragma unroll
+            for (uint32_t q = 0; q < (uint32_t)kScanWarps; ++q) {
+                at += q < warp ? p.warp_units[q] : 0u;
+                base += p.warp_units[q];
+            }
+            if (k < v.slices) {
+                p.first[k] = at;
+                p.total[k] = total;
+            }
+            __syncthreads();
+        }
+        if (base <= v.max_units || run >= kMaskMaxRun) {
+            if (tid == 0) {
+                p.first[v.slices] = base;
+                p.run = run;
+            }
+            break;
+        }
+    }
+    __syncthreads();
+    if (keep)
+        for (uint32_t k = tid; k <= v.slices + 1; k += kThreads) v.slice_first[k] = k <= v.slices ? p.first[k] : p.run;
+}
+
+__device__ __forceinline__ Unit unit_of(const ViewCull& v, uint32_t gps, const Plan& p, uint32_t u)
+{
+    Unit a;
+    uint32_t k = 0, hi = v.slices;  // first[k] <= u < first[hi]
+    while (hi - k > 1) {
+        const uint32_t mid = (k + hi) >> 1;
+        if (p.first[mid] <= u) k = mid;
+        else hi = mid;
+    }
+    const uint32_t total = p.total[k], run = p.run;
+    a.u = u;
+    a.k = k;
+    a.runs = (total + run - 1) / run;
+    const uint32_t gl = (u - p.first[k]) / a.runs;
+    a.g = k * gps + gl;
+    a.r = u - p.first[k] - gl * a.runs;
+    a.t0 = a.r * run;
+    a.n = min(run, total - a.t0);
+    return a;
+}
+
+// A block of a view's scan: every warp takes each `step`th unit.  Neighbouring
+// units, of one dense group, so go to different SMs.
+__device__ __forceinline__ void scan_body(const ViewCull& v, uint32_t blk, uint32_t blocks, ScanWarp* sm, Plan& p)
+{
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup;
+    make_plan(v, gps, p, blk == 0);
+    const uint32_t units = p.first[v.slices];
+    for (uint32_t u = blk + warp * blocks; u < units; u += kScanWarps * blocks)
+        scan_unit(v, unit_of(v, gps, p, u), sm[warp], lane);
+}
+
+__global__ void __launch_bounds__(kScanWarps * 32, 8) scan_kernel(const ViewJob* __restrict__ jobs,
+                                                               const uint32_t* __restrict__ prefix, uint32_t n_views,
+                                                               const __grid_constant__ ViewJob single)
+{
+    __shared__ __align__(16) ScanWarp sm[kScanWarps];
+    __shared__ Plan plan;
+    grid_dependency_wait();
+    launch_dependents();
+    if (jobs) {
+        const uint32_t vi = find_view(prefix, n_views, blockIdx.x), b0 = __ldg(&prefix[vi]);
+        scan_body(jobs[vi].v, blockIdx.x - b0, __ldg(&prefix[vi + 1]) - b0, sm, plan);
+    } else {
+        scan_body(single.v, blockIdx.x, gridDim.x, sm, plan);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Group totals.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kSumWarps = 4;
+constexpr uint32_t kSumIlp = 16;
+
+// Group g: the hits each cluster has in the units before each one, the length
+// of its list, the group's total.  Each warp takes a stretch of the group's
+// units, kSumIlp loads in flight.
+__device__ __forceinline__ void sum_group(const ViewCull& v, uint32_t g)
+{
+    __shared__ uint32_t s_sum[kSumWarps][32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = v.cap;
+    const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup, k = g / gps;
+    const uint32_t first = v.segs ? __ldg(&v.slice_first[k]) : 0u, end = v.segs ? __ldg(&v.slice_first[k + 1]) : 0u;
+    const uint32_t runs = (end - first) / gps, u0 = first + (g - k * gps) * runs;
+    const uint32_t j0 = warp * runs / kSumWarps, j1 = (warp + 1) * runs / kSumWarps;
+    const uint8_t* __restrict__ counts = v.unit_count + (size_t)u0 * kGroup + lane;
+    uint16_t* __restrict__ before = v.unit_before + (size_t)u0 * kGroup + lane;
+    uint32_t x[kSumIlp];
+    auto load = [&](uint32_t j) {
+#pragma unroll
+        for (uint32_t e = 0; e < kSumIlp; ++e) x[e] = __ldg(&counts[min(j + e, j1 - 1) * kGroup]);
+#pragma unroll
+        for (uint32_t e = 0; e < kSumIlp; ++e) x[e] = j + e < j1 ? x[e] : 0u;
+    };
+    uint32_t sum = 0;
+    for (uint32_t j = j0; j < j1; j += kSumIlp) {
+        load(j);
+#pragma unroll
+        for (uint32_t e = 0; e < kSumIlp; ++e) sum += x[e];
+    }
+    s_sum[warp][lane] = sum;
+    __syncthreads();
+    uint32_t at = 0, all = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < kSumWarps; ++q) {
+        at += q < warp ? s_sum[q][lane] : 0u;
+        all += s_sum[q][lane];
+    }
+    all = min(all, cap);
+    if (warp == 0) {
+        v.group_count[(size_t)g * kGroup + lane] = (uint16_t)all;
+        const uint32_t total = warp_sum(all);
+        if (lane == 0) {
+            v.group_total[g] = total;
+            if (total) atomicAdd(&v.block_total[g / kGroup], total);
+        }
+    }
+    for (uint32_t j = j0; j < j1; j += kSumIlp) {
+        if (j1 - j0 > kSumIlp) load(j);  // else still in registers
+#pragma unroll
+        for (uint32_t e = 0; e < kSumIlp; ++e) {
+            if (j + e < j1) before[(j + e) * kGroup] = (uint16_t)min(at, cap);
+            at += x[e];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kSumWarps * 32) sum_kernel(const ViewJob* __restrict__ jobs,
+                                                          const uint32_t* __restrict__ prefix, uint32_t n_views,
+                                                          const __grid_constant__ ViewJob single)
+{
+    grid_dependency_wait();
+    launch_dependents();
+    if (jobs) {
+        const uint32_t vi = find_view(prefix, n_views, blockIdx.x);
+        sum_group(jobs[vi].v, blockIdx.x - __ldg(&prefix[vi]));
+    } else {
+        sum_group(single.v, blockIdx.x);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Writing.
+// ---------------------------------------------------------------------------
+constexpr int kEmitWarps = kScanWarps;
+
+// The sum of the totals of the groups before g, in every lane: block sums, then
+// the groups of g's own block of 32.
+__device__ __forceinline__ uint32_t group_base(const ViewCull& v, uint32_t g, uint32_t lane)
+{
+    uint32_t sum = lane < g % kGroup ? __ldg(&v.group_total[g - g % kGroup + lane]) : 0u;
+    for (uint32_t b = lane; b < g / kGroup; b += 32) sum += __ldg(&v.block_total[b]);
+    return warp_sum(sum);
+}
+
+// Moves the hits of a unit to their places.
+__device__ __forceinline__ void emit_unit(const ViewCull& v, const Unit& a, uint32_t run, ScanWarp& s, uint32_t lane)
+{
+    const uint32_t before = __ldg(&v.unit_before[(size_t)a.u * kGroup + lane]);
+    const uint32_t all = __ldg(&v.group_count[(size_t)a.g * kGroup + lane]);
+    const uint32_t first = group_base(v, a.g, lane) + warp_inclusive_scan(all, lane) - all;
+    uint32_t pos = first + before;
+    if (__all_sync(kFull, before >= all)) return;  // past the cap in every cluster
+    if (run == kNoRun) {  // the pool had no room: scan again, writing this time
+        fetch_candidates(v, s, a.k, a.t0, a.n, lane);
+        scan_candidates<true>(s, a.n, lane, load_group(v, a.g, a.k, lane), pos, first + all, v.indices);
+        __syncwarp();
+        return;
+    }
+    const uint32_t batches = (run >> kBatchShift) + 1;
+    const uint32_t* __restrict__ in = v.pool + (size_t)(run & ((1u << kBatchShift) - 1)) * kBatchWords + lane;
+    uint32_t word[kBank], idx[kBank];
+#pragma unroll
+    for (uint32_t b = 0; b < kBank; ++b) {
+        word[b] = b < batches ? __ldg(&in[b * kBatchWords]) : 0u;
+        idx[b] = b < batches ? __ldg(&in[b * kBatchWords + 32]) : 0u;
+    }
+#pragma unroll
+    for (uint32_t b = 0; b < kBank; ++b) s.idx[b * 32 + lane] = idx[b];
+    __syncwarp();
+#pragma unroll
+    for (uint32_t b = 0; b < kBank; ++b) pos = emit_word(word[b], &s.idx[b * 32], v.indices, pos, first + all);
+    __syncwarp();
+}
+
+// A block of a view's writing: every warp takes each `step`th group, for its
+// cells, and each `step`th unit that has hits.
+__device__ __forceinline__ void emit_body(const ViewCull& v, uint32_t blk, uint32_t blocks, ScanWarp* sm, Plan& p)
+{
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, step = kEmitWarps * blocks;
+    const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup;
+    uint32_t units = 0;
+    if (v.segs) {  // without lights there was no scan
+        for (uint32_t k = threadIdx.x; k <= v.slices + 1; k += kEmitWarps * 32) {
+            const uint32_t x = __ldg(&v.slice_first[k]);
+            if (k < v.slices) p.total[k] = __ldg(&v.slice_total[k]);
+            if (k <= v.slices) p.first[k] = x;
+            else p.run = x;
+        }
+        __syncthreads();
+        units = p.first[v.slices];
+    }
+    for (uint32_t u = blk + warp * blocks; u < units; u += step) {
+        const uint32_t run = __ldg(&v.unit_run[u]);
+        if (run != kNoHits) emit_unit(v, unit_of(v, gps, p, u), run, sm[warp], lane);
+    }
+    for (uint32_t g = blk + warp * blocks; g < v.groups; g += step) {
+        const uint32_t k = g / gps, c = k * v.slice_clusters + (g - k * gps) * kGroup + lane;
+        const uint32_t all = __ldg(&v.group_count[(size_t)g * kGroup + lane]);
+        const uint32_t incl = warp_inclusive_scan(all, lane), base = group_base(v, g, lane);
+        if (c < (k + 1) * v.slice_clusters) v.cells[c] = CfLightCell{base + incl - all, all};
+        if (g == v.groups - 1 && lane == 31 && v.total) *v.total = base + incl;
+    }
+}
+
+__global__ void __launch_bounds__(kEmitWarps * 32, 8) emit_kernel(const ViewJob* __restrict__ jobs,
+                                                               const uint32_t* __restrict__ prefix, uint32_t n_views,
+                                                               const __grid_constant__ ViewJob single)
+{
+    __shared__ __align__(16) ScanWarp sm[kEmitWarps];
+    __shared__ Plan plan;
+    grid_dependency_wait();
+    launch_dependents();
+    if (jobs) {
+        const uint32_t vi = find_view(prefix, n_views, blockIdx.x), b0 = __ldg(&prefix[vi]);
+        emit_body(jobs[vi].v, blockIdx.x - b0, __ldg(&prefix[vi + 1]) - b0, sm, plan);
+    } else {
+        emit_body(single.v, blockIdx.x, gridDim.x, sm, plan);
+    }
+}
+
+}  // namespace
+
+MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slices, uint32_t lights, uint32_t cap,
+                       uint32_t seg_lights)
+{
+    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const uint32_t lpad = pad_lights(lights), groups = group_count(clusters, slice_clusters, slices, kMaskGroup, kModeBinned);
+    MaskLayout m{};
+    // The status words, then the words of a one-launch pass over the same
+    // workspace: small counts left there would pass for its tagged totals.
+    size_t off = 256 + al(kOneLaunchMaxCtas * sizeof(unsigned long long));
+    auto take = [&](size_t bytes) {
+        const size_t at = off;
+        off += al(bytes);
+        return at;
+    };
+    m.group_total = take((size_t)groups * sizeof(uint32_t));
+    m.group_count = take((size_t)groups * kMaskGroup * sizeof(uint16_t));
+    m.block_total = take((size_t)(groups + kMaskGroup - 1) / kMaskGroup * sizeof(uint32_t));
+    m.group_boxes = take((size_t)groups * 2 * sizeof(float4));
+    m.slice_boxes = take((size_t)slices * 2 * sizeof(float4));
+    m.seg_count = take((size_t)slices * mask_segments(lpad, seg_lights) * sizeof(uint32_t));
+    const size_t units = (size_t)groups * ((lpad + kMaskMaxRun - 1) / kMaskMaxRun);
+    m.max_units = (uint32_t)units;
+    m.pool_head = take(sizeof(unsigned long long));
+    m.slice_total = take((size_t)slices * sizeof(uint32_t));
+    m.slice_first = take((size_t)(slices + 2) * sizeof(uint32_t));
+    m.unit_run = take(units * sizeof(uint32_t));
+    m.unit_count = take(units * kMaskGroup * sizeof(uint8_t));
+    m.unit_before = take(units * kMaskGroup * sizeof(uint16_t));
+    // Batches of 32 survivors that all units may keep, as many as fit a third
+    // of the largest index list; a unit past that is scanned a second time
+    // when the lists are written.
+    m.pool_batches = lights ? (uint32_t)std::min<uint64_t>(((uint64_t)clusters * cap / 3 + 4096) / kBatchWords, 1u << 27) : 0u;
+    m.pool = take((size_t)m.pool_batches * kBatchWords * sizeof(uint32_t));
+    m.slice_lights = take((size_t)slices * lpad * sizeof(float4));
+    m.slice_idx = take((size_t)slices * lpad * sizeof(uint32_t));
+    m.bytes = off;
+    return m;
+}
+
+static uint32_t mask_list_slices(uint32_t segs, uint32_t slices)
+{
+    // as few slices per CTA as keep the launch to one wave of two CTAs per SM
+    const uint64_t n = ((uint64_t)segs * slices + 303) / 304;
+    return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(n, 4), kListSlices);
+}
+
+void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg_lights, bool batch)
+{
+    v.group_total = reinterpret_cast<uint32_t*>(ws + m.group_total);
+    v.group_count = reinterpret_cast<uint16_t*>(ws + m.group_count);
+    v.block_total = reinterpret_cast<uint32_t*>(ws + m.block_total);
+    v.group_boxes = reinterpret_cast<float4*>(ws + m.group_boxes);
+    v.slice_boxes = reinterpret_cast<float4*>(ws + m.slice_boxes);
+    v.seg_count = reinterpret_cast<uint32_t*>(ws + m.seg_count);
+    v.pool_head = reinterpret_cast<unsigned long long*>(ws + m.pool_head);
+    v.slice_total = reinterpret_cast<uint32_t*>(ws + m.slice_total);
+    v.slice_first = reinterpret_cast<uint32_t*>(ws + m.slice_first);
+    v.unit_run = reinterpret_cast<uint32_t*>(ws + m.unit_run);
+    v.unit_count = ws + m.unit_count;
+    v.unit_before = reinterpret_cast<uint16_t*>(ws + m.unit_before);
+    v.pool = reinterpret_cast<uint32_t*>(ws + m.pool);
+    v.pool_batches = m.pool_batches;
+    v.max_units = m.max_units;
+    v.run = kMaskMaxRun;
+    v.slice_lights = reinterpret_cast<float4*>(ws + m.slice_lights);
+    v.slice_idx = reinterpret_cast<uint32_t*>(ws + m.slice_idx);
+    v.seg_lights = seg_lights;
+    v.segs = mask_segments(v.lpad, seg_lights);
+    v.list_slices = batch ? kListSlices : mask_list_slices(v.segs, v.slices);
+}
+
+uint32_t mask_seg_lights(uint32_t lights) { return lights <= 4096 ? 256u : lights <= 8192 ? 512u : 1024u; }
+uint32_t mask_list_blocks(const ViewCull& v) { return v.segs * ((v.slices + v.list_slices - 1) / v.list_slices); }
+
+// A view's units are rarely more than this part of what its lights could make
+// (every light a candidate in every slice): with 16384 or 65536 lights the
+// 2560x1600 view has one in 50.
+constexpr uint64_t kUnitsPart = 50;
+
+uint32_t mask_scan_blocks(const ViewCull& v, bool batch)
+{
+    const uint64_t most = (uint64_t)v.groups * ((v.lpad + v.run - 1) / v.run);
+    if (most == 0) return 0;
+    // alone: one resident wave (8 CTAs on each of 152 SMs), or fewer for a view
+    // that cannot have as many units; in a batch about two units per warp
+    const uint64_t blocks = batch ? (most / kUnitsPart + 2 * kScanWarps - 1) / (2 * kScanWarps)
+                                  : (most + kScanWarps - 1) / kScanWarps;
+    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(blocks, 152u * 8u));
+}
+uint32_t mask_emit_blocks(const ViewCull& v, bool batch)
+{
+    const uint32_t per = batch ? 4 * kEmitWarps : kEmitWarps;  // groups whose cells a CTA writes, at most
+    return std::max(mask_scan_blocks(v, batch), std::min((v.groups + per - 1) / per, 152u * 8u));
+}
+
+cudaError_t launch_mask_lists(const ViewJob& j, cudaStream_t stream)
+{
+    cudaError_t e = launch_kernel(true, box_kernel<kBoxThreads>, dim3(j.v.slices), dim3(kBoxThreads), 0, stream,
+                                  static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
+    const uint32_t blocks = mask_list_blocks(j.v);
+    if (e == cudaSuccess && blocks)
+        e = launch_kernel(true, list_kernel, dim3(blocks), dim3(j.v.seg_lights), 0, stream,
+                          static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
+    return e;
+}
+
+cudaError_t launch_mask_scan(const ViewJob& j, cudaStream_t stream)
+{
+    if (j.v.segs == 0) return cudaSuccess;
+    return launch_kernel(true, scan_kernel, dim3(mask_scan_blocks(j.v, false)), dim3(kScanWarps * 32), 0, stream,
+                         static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
+}
+
+cudaError_t launch_mask_emit(const ViewJob& j, cudaStream_t stream)
+{
+    const cudaError_t e = launch_kernel(true, sum_kernel, dim3(j.v.groups), dim3(kSumWarps * 32),
+                                        0, stream, static_cast<const ViewJob*>(nullptr),
+                                        static_cast<const uint32_t*>(nullptr), 0u, j);
+    if (e != cudaSuccess) return e;
+    return launch_kernel(true, emit_kernel, dim3(mask_emit_blocks(j.v, false)), dim3(kEmitWarps * 32), 0, stream,
+                         static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
+}
+
+cudaError_t launch_mask_batch(const MaskBatch& b, cudaStream_t stream)
+{
+    if (b.n_views == 0) return cudaSuccess;
+    const ViewJob none{};
+    const uint32_t n = b.n_views, *p = b.prefix;
+    cudaError_t e = launch_kernel(false, box_kernel<kBoxThreadsBatch>, dim3(b.blocks[kMaskBox]), dim3(kBoxThreadsBatch), 0,
+                                  stream, b.jobs, p, n, none);
+    if (e == cudaSuccess && b.blocks[kMaskList])
+        e = launch_kernel(false, list_kernel, dim3(b.blocks[kMaskList]), dim3(b.seg_lights), 0, stream, b.jobs,
+                          p + kMaskList * (n + 1), n, none);
+    if (e == cudaSuccess && b.blocks[kMaskScan])
+        e = launch_kernel(false, scan_kernel, dim3(b.blocks[kMaskScan]), dim3(kScanWarps * 32), 0, stream, b.jobs,
+                          p + kMaskScan * (n + 1), n, none);
+    if (e == cudaSuccess)
+        e = launch_kernel(false, sum_kernel, dim3(b.blocks[kMaskSum]), dim3(kSumWarps * 32), 0, stream, b.jobs,
+                          p + kMaskSum * (n + 1), n, none);
+    if (e == cudaSuccess)
+        e = launch_kernel(false, emit_kernel, dim3(b.blocks[kMaskEmit]), dim3(kEmitWarps * 32), 0, stream, b.jobs,
+                          p + kMaskEmit * (n + 1), n, none);
+    return e;
+}
+
+uint32_t mask_batch_blocks(const ViewCull& v, MaskStage stage)
+{
+    switch (stage) {
+    case kMaskBox: return v.slices;
+    case kMaskList: return mask_list_blocks(v);
+    case kMaskScan: return mask_scan_blocks(v, true);
+    case kMaskSum: return v.groups;
+    default: return mask_emit_blocks(v, true);
+    }
+}
+
+}  // namespace cfk

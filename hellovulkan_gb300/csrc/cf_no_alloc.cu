@@ -129,16 +129,16 @@ extern "C" int cf_cull_lights_static_scratch(const CfClusterForwardUBO* ubo, con
     // the automatic kernel choice when its scratch fits, else the brute-force
     // kernels, which need less (both give the same result)
     cfk::CullConfig cfg = choose_config(*ubo, light_count, nullptr);
-    cfk::WorkspaceLayout L = layout_for(*ubo, light_count, cap, cfg);
-    if (L.bytes > kStaticScratchBytes && cfg.binned) {
+    uint64_t bytes = scratch_bytes(*ubo, light_count, cap, cfg);
+    if (bytes > kStaticScratchBytes && cfg.binned) {
         cfg = cfk::default_cull_config(C, light_count, 1);
-        L = layout_for(*ubo, light_count, cap, cfg);
+        bytes = scratch_bytes(*ubo, light_count, cap, cfg);
     }
-    if (L.bytes > kStaticScratchBytes)
+    if (bytes > kStaticScratchBytes)
         return fail(CF_ERROR_CAPACITY,
                     "this view needs %llu bytes of scratch (%u clusters, %u lights, cap %u); the static scratch of "
                     "cf_cull_lights_static_scratch holds %llu bytes — use cf_cull_lights with a workspace instead",
-                    (unsigned long long)L.bytes, C, light_count, cap, (unsigned long long)kStaticScratchBytes);
+                    (unsigned long long)bytes, C, light_count, cap, (unsigned long long)kStaticScratchBytes);
     unsigned char* ws = nullptr;
     s = scratch_address(&ws);
     if (s) return s;

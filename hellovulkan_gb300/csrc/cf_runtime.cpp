@@ -11,6 +11,7 @@
 // that uses it is the caller's error.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -165,6 +166,51 @@ cfk::WorkspaceLayout layout_for(const CfClusterForwardUBO& ubo, uint32_t light_c
     return cfk::workspace_layout(C, light_count, cap, ubo.sliceCountZ, cfg.binned, groups);
 }
 
+uint64_t scratch_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, const cfk::CullConfig& cfg)
+{
+    const uint64_t needed = cull_bytes(ubo, light_count, cap, cfg);
+    if (!cfk::is_mask_config(cfg)) return needed;
+    return std::max<uint64_t>(needed, layout_for(ubo, light_count, cap, cfk::kStagedConfig).bytes);
+}
+
+uint64_t cull_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, const cfk::CullConfig& cfg)
+{
+    if (!cfk::is_mask_config(cfg)) return layout_for(ubo, light_count, cap, cfg).bytes;
+    const uint32_t xy = ubo.sliceCountX * ubo.sliceCountY;
+    return cfk::mask_layout(xy * ubo.sliceCountZ, xy, ubo.sliceCountZ, light_count, cap, cfk::mask_seg_lights(light_count)).bytes;
+}
+
+namespace {
+
+// The hit-mask path of one view: slabs, candidate lists, culling straight
+// into the packed list.
+int enqueue_mask(cfk::ViewJob& j, const CfClusterForwardUBO& ubo, const CfLightData* d_lights, uint32_t light_count,
+                 unsigned char* ws, cudaStream_t stream, cudaEvent_t* stage_events)
+{
+    cfk::ViewCull& v = j.v;
+    if (!cfk::mask_fits(v.clusters, v.slice_clusters, v.slices))
+        return fail(CF_ERROR_INVALID_ARGUMENT, "%u slices of %u clusters exceed the hit-mask configuration", v.slices,
+                    v.slice_clusters);
+    const uint32_t seg = cfk::mask_seg_lights(light_count);
+    cfk::mask_bind(v, cfk::mask_layout(v.clusters, v.slice_clusters, v.slices, light_count, v.cap, seg), ws, seg, false);
+    j.lights = d_lights;
+    j.light_count = light_count;
+    for (int i = 0; i < 16; ++i) j.view[i] = ubo.cameraView[i];
+    cudaError_t e = stage_events ? cudaEventRecord(stage_events[0], stream) : cudaSuccess;
+    if (e == cudaSuccess) e = cfk::launch_mask_lists(j, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "slice list launch");
+    if (stage_events) e = cudaEventRecord(stage_events[1], stream);
+    if (e == cudaSuccess) e = cfk::launch_mask_scan(j, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "light culling launch");
+    if (stage_events) e = cudaEventRecord(stage_events[2], stream);
+    if (e == cudaSuccess) e = cfk::launch_mask_emit(j, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "light list launch");
+    if (stage_events) e = cudaEventRecord(stage_events[3], stream);
+    return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "stage event");
+}
+
+}  // namespace
+
 int enqueue_cull(const CfClusterForwardUBO& ubo, const CfAABB* d_aabbs, const CfLightData* d_lights,
                  uint32_t light_count, uint32_t cap, CfLightCell* d_cells, uint32_t* d_indices, uint32_t* d_total,
                  unsigned char* ws, uint32_t* dev_error, const cfk::CullConfig& cfg, cudaStream_t stream,
@@ -199,13 +245,10 @@ int enqueue_cull(const CfClusterForwardUBO& ubo, const CfAABB* d_aabbs, const Cf
         if (e == cudaSuccess && stage_events) e = cudaEventRecord(stage_events[3], stream);
         return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "stage event");
     }
-    cfk::ViewCull v{};
+    cfk::ViewJob job{};
+    cfk::ViewCull& v = job.v;
     v.work = work;
-    v.vlights = reinterpret_cast<const float4*>(ws + L.vlights);
-    v.nonfinite = reinterpret_cast<const uint32_t*>(ws + L.nonfinite);
     v.aabbs = reinterpret_cast<const float4*>(d_aabbs);
-    v.counts = reinterpret_cast<uint32_t*>(ws + L.counts);
-    v.staging = reinterpret_cast<uint32_t*>(ws + L.staging);
     v.cells = d_cells;
     v.indices = d_indices;
     v.total = d_total;
@@ -217,6 +260,11 @@ int enqueue_cull(const CfClusterForwardUBO& ubo, const CfAABB* d_aabbs, const Cf
     v.binned = cfg.binned ? 1u : 0u;
     v.group_width = cfk::group_width(cfg);
     v.groups = cfk::group_count(C, v.slice_clusters, v.slices, v.group_width, cfg.binned);
+    if (cfk::is_mask_config(cfg)) return enqueue_mask(job, ubo, d_lights, light_count, ws, stream, stage_events);
+    v.vlights = reinterpret_cast<const float4*>(ws + L.vlights);
+    v.nonfinite = reinterpret_cast<const uint32_t*>(ws + L.nonfinite);
+    v.counts = reinterpret_cast<uint32_t*>(ws + L.counts);
+    v.staging = reinterpret_cast<uint32_t*>(ws + L.staging);
     v.group_sums = reinterpret_cast<uint32_t*>(ws + L.group_sums);
     v.group_offsets = reinterpret_cast<uint32_t*>(ws + L.group_offsets);
     if (cfg.binned) {
@@ -752,8 +800,8 @@ int cf_pipeline_light_culling_fill_command_buffer(CfPipelineLightCulling* p, voi
     DeviceGuard g(p->ctx->device);
     if (g.err()) return cuda_fail(g.err(), "cudaSetDevice");
     const cfk::CullConfig cfg = choose_config(p->ubo, p->lights->count, p->has_cfg ? &p->cfg : nullptr);
-    const cfk::WorkspaceLayout L = layout_for(p->ubo, p->lights->count, r->cap, cfg);
-    int s = grow(reinterpret_cast<void**>(&r->d_ws), &r->ws_capacity, L.bytes, "culling workspace");
+    int s = grow(reinterpret_cast<void**>(&r->d_ws), &r->ws_capacity, cull_bytes(p->ubo, p->lights->count, r->cap, cfg),
+                 "culling workspace");
     if (s) return s;
     return enqueue_cull(p->ubo, r->d_aabbs, p->lights->d_lights, p->lights->count, r->cap, r->d_cells, r->d_indices,
                         r->d_total, r->d_ws, p->ctx->dev_error, cfg, (cudaStream_t)stream,
@@ -811,7 +859,7 @@ int cf_cull_workspace_size(const CfClusterForwardUBO* ubo, uint32_t light_count,
     uint32_t C = 0;
     int s = validate_grid(ubo->sliceCountX, ubo->sliceCountY, ubo->sliceCountZ, cap, &C);
     if (s) return s;
-    *bytes = layout_for(*ubo, light_count, cap, choose_config(*ubo, light_count, nullptr)).bytes;
+    *bytes = scratch_bytes(*ubo, light_count, cap, choose_config(*ubo, light_count, nullptr));
     return CF_SUCCESS;
 }
 
@@ -853,10 +901,10 @@ int cf_cull_lights(const CfClusterForwardUBO* ubo, const CfAABB* d_aabbs, const 
         return fail(CF_ERROR_CAPACITY, "index capacity %llu < clusters x cap = %llu", (unsigned long long)index_capacity,
                     (unsigned long long)C * cap);
     const cfk::CullConfig cfg = choose_config(*ubo, light_count, nullptr);
-    const cfk::WorkspaceLayout L = layout_for(*ubo, light_count, cap, cfg);
-    if (workspace_bytes < L.bytes)
+    const uint64_t needed = scratch_bytes(*ubo, light_count, cap, cfg);
+    if (workspace_bytes < needed)
         return fail(CF_ERROR_CAPACITY, "workspace %llu bytes < %llu needed", (unsigned long long)workspace_bytes,
-                    (unsigned long long)L.bytes);
+                    (unsigned long long)needed);
     unsigned char* ws = static_cast<unsigned char*>(d_workspace);
     return enqueue_cull(*ubo, d_aabbs, d_lights, light_count, cap, d_cells, d_indices, d_total, ws,
                         reinterpret_cast<uint32_t*>(ws), cfg, (cudaStream_t)stream, nullptr);

@@ -182,7 +182,8 @@ CFCULL_API int cf_pipeline_light_culling_fill_command_buffer(CfPipelineLightCull
 /* Tuning: selects the culling kernel configuration (clusters per warp,
  * consumer warps per CTA, lights per shared-memory stage, stages, and the
  * mode: binned = 0 every light against every cluster, 1 the depth-slice
- * candidate lists first, 2 the whole step in one launch, for which the
+ * candidate lists first — (4, 8, 32, 1, 1) by hit masks, the automatic choice
+ * for most views — 2 the whole step in one launch, for which the
  * arguments are clusters per CTA (1..32), warps per CTA, the most lights the
  * launch takes and 1 — (M, 32, 1024, 1, 2), (M, 16, 2048, 1, 2) or
  * (M, 16, 1024, 1, 2); a view with more lights than that is rejected when
