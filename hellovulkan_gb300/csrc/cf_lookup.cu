@@ -4,15 +4,27 @@
 // index list drop into the reference's fragment pass, and the pass's direct
 // clustered lighting (Radiance.glsl) over a G-buffer.
 //
-// One thread per pixel: LinearDepth of the pixel's depth, the exponential
-// slice index from log2 (pinned: cf_log2_pinned), the tile from the pixel
-// centre, then the cluster's cell.  The fragment's view-space position is
-// reconstructed the way AABBGenerator.comp's ScreenToView unprojects a screen
-// point, and every listed light is tested for containing it (the lights a
-// shading loop over the list would find in range).  In check mode every light
-// of the set is tested as well, to count the ones the list lacks.
+// Per pixel: LinearDepth of its depth, the exponential slice index from log2
+// (pinned: cf_log2_pinned), the tile from the pixel centre, then the cluster's
+// cell.  The fragment's view-space position is reconstructed the way
+// AABBGenerator.comp's ScreenToView unprojects a screen point, and every listed
+// light is tested for containing it (the lights a shading loop over the list
+// would find in range).  In check mode the lights of the whole set that contain
+// it are counted as well, to count the ones the list lacks.
+//
+// Both passes take a CTA per square tile of pixels and sort the tile's pixels
+// by depth first, so that the 32 pixels of a warp read the same one or two
+// lists: with every pixel at its own depth, unsorted warps had 5 to 10 of 32
+// lanes active.  A sorted warp's fragments also lie in a small box, which few
+// lights of the whole set reach.  1920x1080, 1024 lights, every pixel at its own
+// depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 61 us,
+// shading 1108 -> 139 us; 480x270 with 3000 lights and the all-lights check
+// 805 -> 60 us.
 #include <cuda_runtime.h>
 
+#include <cmath>
+
+#include "cf_device.cuh"
 #include "cf_pinned_math.h"
 #include "cf_runtime_internal.h"
 #include "cfcull.h"
@@ -32,7 +44,8 @@ __device__ __forceinline__ void light_view(const float* V, const CfLightData* __
 
 // Scene.frag:54-71 for the fragment at pixel (x, y) with window depth z: the
 // linear depth and, when it lies inside the grid, the cluster index.
-__device__ __forceinline__ bool fragment_cluster(const CfClusterForwardUBO& u, uint32_t x, uint32_t y, float z,
+// xf, yf: its tile coordinates, gl_FragCoord.xy / (screenSize / sliceCount).
+__device__ __forceinline__ bool fragment_cluster(const CfClusterForwardUBO& u, float xf, float yf, float z,
                                                  uint32_t* cluster, float* linear_depth)
 {
     const float n = u.cameraNear, f = u.cameraFar;
@@ -40,9 +53,6 @@ __device__ __forceinline__ bool fragment_cluster(const CfClusterForwardUBO& u, u
     const float lin = cf_fdiv(cf_fmul(n, f), cf_fadd(f, cf_fmul(z, cf_fsub(n, f))));
     // zIndex (Scene.frag:63): max(log2(linDepth) * sliceScaling + sliceBias, 0)
     const float zf = cf_glsl_max(cf_fadd(cf_fmul(cf_log2_pinned(lin), u.sliceScaling), u.sliceBias), 0.0f);
-    // tile (Scene.frag:64-70): gl_FragCoord.xy / (screenSize / sliceCount)
-    const float xf = cf_fdiv((float)x + 0.5f, cf_fdiv(u.screenSize[0], (float)u.sliceCountX));
-    const float yf = cf_fdiv((float)y + 0.5f, cf_fdiv(u.screenSize[1], (float)u.sliceCountY));
     *linear_depth = lin;
     // NaN compares false: a NaN index leaves the grid too
     if (!(zf < (float)u.sliceCountZ && xf < (float)u.sliceCountX && yf < (float)u.sliceCountY)) return false;
@@ -57,63 +67,251 @@ __device__ __forceinline__ bool contains(const float f[3], const float c[3], flo
     return cf_fadd(cf_fadd(cf_fmul(dx, dx), cf_fmul(dy, dy)), cf_fmul(dz, dz)) < r2;
 }
 
-__global__ void __launch_bounds__(256) lookup_kernel(const CfClusterForwardUBO u, const float* __restrict__ depth,
-                                                     uint32_t width, uint32_t n_pixels,
-                                                     const CfLightCell* __restrict__ cells,
-                                                     const uint32_t* __restrict__ indices, uint64_t index_count,
-                                                     const CfLightData* __restrict__ lights, uint32_t light_count,
-                                                     uint32_t cap, const float4* __restrict__ aabbs, int check_all,
-                                                     CfFragmentSample* __restrict__ out)
+// ---------------------------------------------------------------------------
+// Tiles of pixels, sorted by depth.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kDepthBins = 64;
+constexpr uint32_t kNoPixel = 0xffffu;
+
+struct Image {
+    uint32_t width, height, n_pixels;
+    uint32_t tiles_x;  // 0: too narrow for square tiles, a tile is a run of pixels in row-major order
+    float tile_w, tile_h;  // pixels per cluster (screenSize / sliceCount)
+};
+
+// The CTA's tile of kSide * kSide pixels.
+template <uint32_t kSide>
+struct Tile {
+    uint32_t x0, y0;  // of a run: x0 is its first pixel
+    __device__ __forceinline__ explicit Tile(const Image& im)
+        : x0(im.tiles_x ? blockIdx.x % im.tiles_x * kSide : blockIdx.x * kSide * kSide),
+          y0(im.tiles_x ? blockIdx.x / im.tiles_x * kSide : 0u)
+    {
+    }
+    // Pixel i of the tile; false past the image.
+    __device__ __forceinline__ bool at(const Image& im, uint32_t i, uint32_t& x, uint32_t& y) const
+    {
+        if (im.tiles_x) {
+            x = x0 + i % kSide;
+            y = y0 + i / kSide;
+            return x < im.width && y < im.height;
+        }
+        const uint32_t p = x0 + i;  // below 2^31 + 1024
+        x = p % im.width;
+        y = p / im.width;
+        return p < im.n_pixels;
+    }
+};
+
+// What a pixel's column and row give, which a square tile's pixels share: the
+// cluster tile coordinate and the clip coordinate of the pixel centre (a run's
+// pixels compute them where they are used).
+template <uint32_t kSide>
+struct TileAxes {
+    float tile[2][kSide], clip[2][kSide];
+};
+// gl_FragCoord / (screenSize / sliceCount) (Scene.frag:64-70)
+__device__ __forceinline__ float tile_coord(uint32_t p, float pixels) { return cf_fdiv((float)p + 0.5f, pixels); }
+// ScreenToView's clip coordinate of the pixel centre
+__device__ __forceinline__ float clip_coord(uint32_t p, float size)
 {
-    const uint32_t pix = blockIdx.x * 256u + threadIdx.x;
-    if (pix >= n_pixels) return;
-    const uint32_t x = pix % width, y = pix / width;
-    const float z = __ldg(&depth[pix]);
-    uint32_t c = 0;
-    float lin = 0.0f;
-    const bool inside = fragment_cluster(u, x, y, z, &c, &lin);
-    const float fx = (float)x + 0.5f, fy = (float)y + 0.5f;
-    // the fragment in view space: ScreenToView of (fx / width, fy / height, z, 1)
-    const float cx = cf_fsub(cf_fmul(cf_fdiv(fx, u.screenSize[0]), 2.0f), 1.0f);
-    const float cy = cf_fsub(cf_fmul(cf_fdiv(fy, u.screenSize[1]), 2.0f), 1.0f);
+    return cf_fsub(cf_fmul(cf_fdiv((float)p + 0.5f, size), 2.0f), 1.0f);
+}
+template <uint32_t kSide>
+__device__ __forceinline__ void fill_axes(const CfClusterForwardUBO& u, const Image& im, const Tile<kSide>& tile,
+                                          TileAxes<kSide>& a)
+{
+    if (im.tiles_x == 0 || threadIdx.x >= 2 * kSide) return;
+    const uint32_t axis = threadIdx.x / kSide, i = threadIdx.x % kSide, p = (axis ? tile.y0 : tile.x0) + i;
+    a.tile[axis][i] = tile_coord(p, axis ? im.tile_h : im.tile_w);
+    a.clip[axis][i] = clip_coord(p, u.screenSize[axis]);
+}
+
+// A pixel's depth bin: a quarter of an octave of the denominator of
+// LinearDepth, so of the linear depth itself.  It orders the work and nothing
+// else; a depth outside [0, 1] or a NaN gets some bin.
+__device__ __forceinline__ uint32_t depth_bin(const CfClusterForwardUBO& u, float z)
+{
+    const float t = u.cameraFar + z * (u.cameraNear - u.cameraFar);
+    const int b = ((int)__float_as_uint(t) - (int)__float_as_uint(u.cameraNear)) >> 21;
+    return (uint32_t)min(max(b, 0), (int)kDepthBins - 2);
+}
+
+struct TileSort {
+    uint32_t start[kDepthBins];
+    uint32_t next;  // unit not yet taken
+};
+
+// order[]: the tile's pixels by depth bin, those past the image (kNoPixel)
+// last.  `depth` gives a pixel's depth.  Every thread of the CTA takes part.
+template <uint32_t kSide, uint32_t kThreads, typename Depth>
+__device__ __forceinline__ void sort_tile(const CfClusterForwardUBO& u, const Image& im, const Tile<kSide>& tile,
+                                          TileSort& s, uint16_t* order, Depth depth)
+{
+    constexpr uint32_t kPer = kSide * kSide / kThreads;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    if (tid < kDepthBins) s.start[tid] = 0;
+    uint32_t bin[kPer], rank[kPer];
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) {
+        uint32_t x, y;
+        bin[q] = tile.at(im, q * kThreads + tid, x, y) ? depth_bin(u, depth(y * im.width + x)) : kDepthBins - 1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) {  // one count per bin and warp
+        const uint32_t same = __match_any_sync(cfk::kFull, bin[q]), first = __ffs(same) - 1;
+        uint32_t at = 0;
+        if (lane == first) at = atomicAdd(&s.start[bin[q]], (uint32_t)__popc(same));
+        rank[q] = __shfl_sync(cfk::kFull, at, first) + __popc(same & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    if (tid < 32) {
+        const uint32_t a = s.start[2 * tid], b = s.start[2 * tid + 1];
+        const uint32_t incl = cfk::warp_inclusive_scan(a + b, tid);
+        s.start[2 * tid] = incl - a - b;
+        s.start[2 * tid + 1] = incl - b;
+        if (tid == 0) s.next = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q)
+        order[s.start[bin[q]] + rank[q]] = (uint16_t)(bin[q] == kDepthBins - 1 ? kNoPixel : q * kThreads + tid);
+    __syncthreads();
+}
+
+// The next 32 pixels of the sorted tile, as units are taken by the CTA's warps
+// one after another: a tile's long lists lie at neighbouring depths, so fixed
+// shares would leave them to one warp.
+__device__ __forceinline__ uint32_t next_unit(TileSort& s, uint32_t lane)
+{
+    uint32_t unit = 0;
+    if (lane == 0) unit = atomicAdd(&s.next, 1u);
+    return __shfl_sync(cfk::kFull, unit, 0);
+}
+
+// ---------------------------------------------------------------------------
+// Lookup.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kTableLights = 1024;  // view-space lights kept in shared memory at a time
+
+struct LookupArgs {
+    CfClusterForwardUBO u;
+    Image im;
+    const float* depth;
+    const CfLightCell* cells;
+    const uint32_t* indices;
+    uint64_t index_count;
+    const CfLightData* lights;
+    const float4* aabbs;
+    CfFragmentSample* out;
+    uint32_t light_count, cap;
+    int out_aligned;
+};
+
+// Lights [first, first + n) of the set in view space: (x, y, z, r^2).
+__device__ __forceinline__ void fill_table(const LookupArgs& A, float4* table, uint32_t first, uint32_t n)
+{
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        float p[3], r2;
+        light_view(A.u.cameraView, &A.lights[first + i], p, &r2);
+        table[i] = make_float4(p[0], p[1], p[2], r2);
+    }
+}
+
+// The view-space position of the fragment at clip coordinates (cx, cy) with
+// window depth z: ScreenToView of (x / width, y / height, z, 1).
+__device__ __forceinline__ void fragment_view(const CfClusterForwardUBO& u, float cx, float cy, float z, float frag[3])
+{
     const float* IP = u.cameraInverseProjection;
     const float vw = cf_mat4_row(IP, 3, cx, cy, z, 1.0f);
-    const float frag[3] = {cf_fdiv(cf_mat4_row(IP, 0, cx, cy, z, 1.0f), vw),
-                           cf_fdiv(cf_mat4_row(IP, 1, cx, cy, z, 1.0f), vw),
-                           cf_fdiv(cf_mat4_row(IP, 2, cx, cy, z, 1.0f), vw)};
-    CfFragmentSample s;
+    frag[0] = cf_fdiv(cf_mat4_row(IP, 0, cx, cy, z, 1.0f), vw);
+    frag[1] = cf_fdiv(cf_mat4_row(IP, 1, cx, cy, z, 1.0f), vw);
+    frag[2] = cf_fdiv(cf_mat4_row(IP, 2, cx, cy, z, 1.0f), vw);
+}
+
+// How many lights of table[0, n) contain each lane's fragment.  The warp's
+// fragments lie in the box [lo, hi]; a light that does not reach it contains
+// none of them (its distance to the box is never larger than to a fragment in
+// it, rounded operation by rounded operation).
+__device__ __forceinline__ uint32_t count_containing(const float4* table, uint32_t n, const float frag[3], const float lo[3],
+                                                     const float hi[3], uint32_t lane)
+{
+    uint32_t count = 0;
+    for (uint32_t c = 0; c < n; c += 32) {
+        const bool in = c + lane < n;
+        const float4 L = table[in ? c + lane : c];
+        for (uint32_t m = __ballot_sync(cfk::kFull, in && cfk::hit_fast(L, lo, hi)); m; m &= m - 1) {
+            const float4 q = table[c + __ffs(m) - 1];
+            const float p[3] = {q.x, q.y, q.z};
+            count += contains(frag, p, q.w) ? 1u : 0u;
+        }
+    }
+    return count;
+}
+
+// The lookup of one pixel whose fragment is at frag; `missing` of s holds the
+// lights of the whole set that contain it, or 0 without the check.  Four list
+// entries are read ahead of their tests.
+constexpr uint32_t kListIlp = 4;
+template <bool kCheck>
+__device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table, bool whole, float xf, float yf, float z,
+                                        const float frag[3], CfFragmentSample& s)
+{
+    const CfClusterForwardUBO& u = A.u;
+    uint32_t c = 0, off = 0, cnt = 0, in_list = 0;
+    const bool inside = fragment_cluster(u, xf, yf, z, &c, &s.linear_depth);
     s.view_z = frag[2];
-    s.linear_depth = lin;
     s.covering = 0;
-    s.missing = 0;
     s.flags = 0;
-    uint32_t off = 0, cnt = 0;
-    const float* V = u.cameraView;
     if (inside) {
-        const CfLightCell cell = cells[c];
+        const CfLightCell cell = A.cells[c];
         off = cell.offset;
         cnt = cell.count;
         s.cluster = c;
-        if ((uint64_t)off + cnt > index_count) {  // not a cell of this index list: read nothing through it
+        if ((uint64_t)off + cnt > A.index_count) {  // not a cell of this index list: read nothing through it
             s.flags |= CF_FRAGMENT_BAD_CELL;
             cnt = 0;
         }
-        if (cnt >= cap) s.flags |= CF_FRAGMENT_CAPPED;
-        if (aabbs) {
-            const float4 lo = aabbs[2 * (size_t)c], hi = aabbs[2 * (size_t)c + 1];
-            if (frag[0] < lo.x || frag[1] < lo.y || frag[2] < lo.z || frag[0] > hi.x || frag[1] > hi.y ||
-                frag[2] > hi.z)
+        if (cnt >= A.cap) s.flags |= CF_FRAGMENT_CAPPED;
+        if (A.aabbs) {
+            const float4 lo = __ldg(&A.aabbs[2 * (size_t)c]), hi = __ldg(&A.aabbs[2 * (size_t)c + 1]);
+            if (frag[0] < lo.x || frag[1] < lo.y || frag[2] < lo.z || frag[0] > hi.x || frag[1] > hi.y || frag[2] > hi.z)
                 s.flags |= CF_FRAGMENT_OUTSIDE_AABB;
         }
-        for (uint32_t j = 0; j < cnt; ++j) {
-            const uint32_t li = indices[off + j];
-            if (li >= light_count) {
-                s.flags |= CF_FRAGMENT_BAD_CELL;
-                continue;
+        // A light is missing when it is not in the part of the list that a
+        // walk over all lights in order would match: the entries up to the
+        // first that does not ascend or is no light.
+        bool walked = true;
+        uint32_t before = 0;
+        for (uint32_t j = 0; j < cnt; j += kListIlp) {
+            uint32_t li[kListIlp];
+#pragma unroll
+            for (uint32_t e = 0; e < kListIlp; ++e) li[e] = __ldg(&A.indices[off + min(j + e, cnt - 1)]);
+#pragma unroll
+            for (uint32_t e = 0; e < kListIlp; ++e) {
+                if (j + e >= cnt) break;
+                const bool light = li[e] < A.light_count;
+                if (!light) s.flags |= CF_FRAGMENT_BAD_CELL;
+                if (kCheck) {
+                    walked = walked && light && (j + e == 0 || li[e] > before);
+                    before = li[e];
+                }
+                if (!light) continue;
+                float p[3], r2;
+                if (whole) {
+                    const float4 L = table[li[e]];
+                    p[0] = L.x;
+                    p[1] = L.y;
+                    p[2] = L.z;
+                    r2 = L.w;
+                } else {
+                    light_view(u.cameraView, &A.lights[li[e]], p, &r2);
+                }
+                const uint32_t hit = contains(frag, p, r2) ? 1u : 0u;
+                s.covering += hit;
+                if (kCheck) in_list += walked ? hit : 0u;
             }
-            float p[3], r2;
-            light_view(V, &lights[li], p, &r2);
-            s.covering += contains(frag, p, r2) ? 1u : 0u;
         }
     } else {
         s.cluster = 0xFFFFFFFFu;
@@ -121,21 +319,102 @@ __global__ void __launch_bounds__(256) lookup_kernel(const CfClusterForwardUBO u
     }
     s.offset = off;
     s.count = (s.flags & CF_FRAGMENT_BAD_CELL) ? 0u : cnt;
-    if (check_all) {
-        uint32_t j = 0;  // the list is ascending: walk it beside the lights
-        for (uint32_t i = 0; i < light_count; ++i) {
-            if (j < cnt && indices[off + j] == i) {
-                ++j;
-                continue;
-            }
-            float p[3], r2;
-            light_view(V, &lights[i], p, &r2);
-            s.missing += contains(frag, p, r2) ? 1u : 0u;
-        }
-    }
-    out[pix] = s;
+    if (kCheck) s.missing -= in_list;
 }
 
+// One CTA per tile.  Bound by issue: some 300 instructions a pixel apart from
+// its list, six of them IEEE divisions.  A sorted warp's listed loop runs about
+// as long as its mean list; lights come from the table where the whole set fits
+// it.  The all-lights check runs the set through the table in pieces, a filter
+// of 32 lights at a time against the box of the warp's fragments.
+template <uint32_t kSide, uint32_t kThreads, bool kCheck>
+__global__ void __launch_bounds__(kThreads) lookup_kernel(const __grid_constant__ LookupArgs A)
+{
+    constexpr uint32_t kPixels = kSide * kSide, kUnits = kPixels / 32;
+    __shared__ __align__(16) float4 table[kTableLights];
+    __shared__ uint32_t missing[kCheck ? kPixels : 1];  // by place in the order, between pieces
+    __shared__ uint16_t order[kPixels];
+    __shared__ TileSort sort;
+    __shared__ TileAxes<kSide> axes;
+    const uint32_t lane = threadIdx.x & 31;
+    const CfClusterForwardUBO& u = A.u;
+    const Tile<kSide> tile(A.im);
+    const bool whole = A.light_count <= kTableLights;  // the set fits the table
+    if (whole) fill_table(A, table, 0, A.light_count);
+    fill_axes(u, A.im, tile, axes);
+    sort_tile<kSide, kThreads>(u, A.im, tile, sort, order, [&](uint32_t p) { return __ldg(&A.depth[p]); });
+    const uint32_t pieces = kCheck ? (A.light_count + kTableLights - 1) / kTableLights : 0u;
+    for (uint32_t piece = 0; piece < max(pieces, 1u); ++piece) {
+        const uint32_t n = pieces ? min(kTableLights, A.light_count - piece * kTableLights) : 0u;
+        if (!whole && pieces) {
+            if (piece) {
+                __syncthreads();
+                if (threadIdx.x == 0) sort.next = 0;
+            }
+            fill_table(A, table, piece * kTableLights, n);
+            __syncthreads();
+        }
+        for (uint32_t unit; (unit = next_unit(sort, lane)) < kUnits;) {
+            const uint32_t i = order[unit * 32 + lane];
+            const bool valid = i != kNoPixel;
+            if (!__any_sync(cfk::kFull, valid)) continue;
+            uint32_t x = 0, y = 0;
+            float z = 0.0f, cx = 0.0f, cy = 0.0f, xf = 0.0f, yf = 0.0f;
+            if (valid) {
+                tile.at(A.im, i, x, y);
+                z = __ldg(&A.depth[y * A.im.width + x]);
+                if (A.im.tiles_x) {
+                    cx = axes.clip[0][i % kSide];
+                    cy = axes.clip[1][i / kSide];
+                    xf = axes.tile[0][i % kSide];
+                    yf = axes.tile[1][i / kSide];
+                } else {
+                    cx = clip_coord(x, u.screenSize[0]);
+                    cy = clip_coord(y, u.screenSize[1]);
+                    xf = tile_coord(x, A.im.tile_w);
+                    yf = tile_coord(y, A.im.tile_h);
+                }
+            }
+            float frag[3];
+            fragment_view(u, cx, cy, z, frag);
+            CfFragmentSample s;
+            s.missing = 0;
+            if (kCheck && pieces) {
+                const float inf = __uint_as_float(0x7f800000u);
+                float lo[3], hi[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {  // a NaN coordinate is in no sphere: fminf and fmaxf pass it over
+                    lo[a] = valid ? frag[a] : inf;
+                    hi[a] = valid ? frag[a] : -inf;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        lo[a] = fminf(lo[a], __shfl_xor_sync(cfk::kFull, lo[a], o));
+                        hi[a] = fmaxf(hi[a], __shfl_xor_sync(cfk::kFull, hi[a], o));
+                    }
+                }
+                s.missing = count_containing(table, n, frag, lo, hi, lane) + (piece ? missing[unit * 32 + lane] : 0u);
+                if (piece + 1 < pieces) {
+                    missing[unit * 32 + lane] = s.missing;
+                    continue;
+                }
+            }
+            if (!valid) continue;
+            look_up<kCheck>(A, table, whole, xf, yf, z, frag, s);
+            CfFragmentSample* out = &A.out[y * A.im.width + x];
+            if (A.out_aligned) {
+                uint4* o = reinterpret_cast<uint4*>(out);
+                o[0] = make_uint4(s.cluster, s.offset, s.count, s.covering);
+                o[1] = make_uint4(s.missing, s.flags, __float_as_uint(s.view_z), __float_as_uint(s.linear_depth));
+            } else {
+                *out = s;
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Shading.
+// ---------------------------------------------------------------------------
 struct V3 {
     float x, y, z;
 };
@@ -155,16 +434,28 @@ __device__ __forceinline__ V3 v3_normalize(V3 v)
 
 constexpr float kPi = 3.14159265358979323846f;  // PBRHeader.glsl's PI as a GLSL float
 
-// Radiance (Radiance.glsl:2-57) of one light at world position P, in the
-// shader's operation order; adds to lo.
-__device__ __forceinline__ void radiance(const CfLightData* __restrict__ light, V3 P, V3 N, V3 V, V3 albedo, V3 F0,
-                                         float metallic, float roughness, float alpha_r, float NoV,
-                                         const CfPBRPushConstant& pc, V3& lo)
+// What Radiance reads of a texel, one array per field over the texels of a warp.
+enum TexelField { kPx, kPy, kPz, kNx, kNy, kNz, kVx, kVy, kVz, kAx, kAy, kAz, kFx, kFy, kFz, kA2, kAlphaR, kGv, kNoV4, kKm,
+                  kTexelFields };
+
+// Shared memory of one shading warp.
+struct ShadeWarp {
+    float f[kTexelFields][32];
+    float lo[3][32];       // the texels' sums so far
+    uint32_t light[64];    // ring of (light, texel) pairs to evaluate
+    uint32_t texel[64];
+};
+
+// Radiance (Radiance.glsl:2-57) of one light at texel t of w, in the shader's
+// operation order, plus the zero its Lo starts from.
+__device__ __forceinline__ void radiance(const CfLightData* __restrict__ light, const ShadeWarp& w, uint32_t t,
+                                         const CfPBRPushConstant& pc, float out[3])
 {
     const float4 q = __ldg(reinterpret_cast<const float4*>(&light->position[0]));
     const float4 col = __ldg(reinterpret_cast<const float4*>(&light->color[0]));
     const float radius = __ldg(&light->radius);
-    const V3 d = v3_sub(V3{q.x, q.y, q.z}, P);
+    const V3 N = {w.f[kNx][t], w.f[kNy][t], w.f[kNz][t]}, V = {w.f[kVx][t], w.f[kVy][t], w.f[kVz][t]};
+    const V3 d = v3_sub(V3{q.x, q.y, q.z}, V3{w.f[kPx][t], w.f[kPy][t], w.f[kPz][t]});
     const V3 L = v3_normalize(d);
     const V3 H = v3_normalize(v3_add(V, L));
     const float NoH = cf_glsl_max(v3_dot(N, H), 0.0f);
@@ -172,81 +463,275 @@ __device__ __forceinline__ void radiance(const CfLightData* __restrict__ light, 
     const float HoV = cf_glsl_max(v3_dot(H, V), 0.0f);
     const float dist = cf_fsqrt(v3_dot(d, d));
     const float att = cf_fdiv(cf_glsl_max(cf_fsub(1.0f, cf_fdiv(dist, radius)), 0.0f), cf_pow_pinned(dist, pc.lightFalloff));
-    const V3 rad = {cf_fmul(cf_fmul(col.x, att), pc.lightIntensity), cf_fmul(cf_fmul(col.y, att), pc.lightIntensity),
-                    cf_fmul(cf_fmul(col.z, att), pc.lightIntensity)};
+    const float rad[3] = {cf_fmul(cf_fmul(col.x, att), pc.lightIntensity), cf_fmul(cf_fmul(col.y, att), pc.lightIntensity),
+                          cf_fmul(cf_fmul(col.z, att), pc.lightIntensity)};
     // DistributionGGX (PBRHeader.glsl:17-28)
-    const float a = cf_fmul(roughness, roughness);
-    const float a2 = cf_fmul(a, a);
+    const float a2 = w.f[kA2][t];
     const float den0 = cf_fadd(cf_fmul(cf_fmul(NoH, NoH), cf_fsub(a2, 1.0f)), 1.0f);
     const float D = cf_fdiv(a2, cf_fmul(cf_fmul(kPi, den0), den0));
-    // GeometrySchlickGGX (PBRHeader.glsl:41-46)
-    const float one_a = cf_fsub(1.0f, alpha_r);
-    const float G = cf_fmul(cf_fdiv(NoL, cf_fadd(cf_fmul(NoL, one_a), alpha_r)),
-                            cf_fdiv(NoV, cf_fadd(cf_fmul(NoV, one_a), alpha_r)));
+    // GeometrySchlickGGX (PBRHeader.glsl:41-46); the texel's factor is kGv
+    const float alpha_r = w.f[kAlphaR][t];
+    const float G = cf_fmul(cf_fdiv(NoL, cf_fadd(cf_fmul(NoL, cf_fsub(1.0f, alpha_r)), alpha_r)), w.f[kGv][t]);
     // FresnelSchlick (PBRHeader.glsl:50-53)
     const float p5 = cf_pow_pinned(cf_glsl_min(cf_glsl_max(cf_fsub(1.0f, HoV), 0.0f), 1.0f), 5.0f);
-    const V3 F = {cf_fadd(F0.x, cf_fmul(cf_fsub(1.0f, F0.x), p5)), cf_fadd(F0.y, cf_fmul(cf_fsub(1.0f, F0.y), p5)),
-                  cf_fadd(F0.z, cf_fmul(cf_fsub(1.0f, F0.z), p5))};
     const float DG = cf_fmul(D, G);
-    const float denom = cf_fadd(cf_fmul(cf_fmul(4.0f, NoV), NoL), 0.0001f);
-    const float km = cf_fsub(1.0f, metallic);
-    const float fc[3] = {F.x, F.y, F.z}, ac[3] = {albedo.x, albedo.y, albedo.z}, rc[3] = {rad.x, rad.y, rad.z};
-    float out[3];
+    const float denom = cf_fadd(cf_fmul(w.f[kNoV4][t], NoL), 0.0001f);
+    const float km = w.f[kKm][t];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const float spec = cf_fdiv(cf_fmul(DG, fc[c]), denom);
-        const float kd = cf_fmul(cf_fsub(1.0f, fc[c]), km);
-        const float diff = cf_fdiv(cf_fmul(kd, ac[c]), kPi);
+        const float f0 = w.f[kFx + c][t];
+        const float F = cf_fadd(f0, cf_fmul(cf_fsub(1.0f, f0), p5));
+        const float spec = cf_fdiv(cf_fmul(DG, F), denom);
+        const float kd = cf_fmul(cf_fsub(1.0f, F), km);
+        const float diff = cf_fdiv(cf_fmul(kd, w.f[kAx + c][t]), kPi);
         // Radiance's own Lo starts at vec3(0.0) (Radiance.glsl:13,55): the
         // term is added to zero before Scene.frag adds it to its Lo, which
         // turns a -0 term into +0
-        out[c] = cf_fadd(0.0f, cf_fmul(cf_fmul(cf_fadd(diff, spec), rc[c]), NoL));
+        out[c] = cf_fadd(0.0f, cf_fmul(cf_fmul(cf_fadd(diff, spec), rad[c]), NoL));
     }
-    lo = V3{cf_fadd(lo.x, out[0]), cf_fadd(lo.y, out[1]), cf_fadd(lo.z, out[2])};
 }
 
-__global__ void __launch_bounds__(256) shade_kernel(const CfClusterForwardUBO u, const float3 cam,
-                                                    const CfPBRPushConstant pc,
-                                                    const CfGBufferTexel* __restrict__ gbuf, uint32_t width,
-                                                    uint32_t n_pixels, const CfLightCell* __restrict__ cells,
-                                                    const uint32_t* __restrict__ indices, uint64_t index_count,
-                                                    const CfLightData* __restrict__ lights, uint32_t light_count,
-                                                    float4* __restrict__ out)
+// A light as the tests of out_of_reach see it: its position and the squared
+// distance from which it is out of reach, +inf for a light whose colour or
+// radius rules the tests out.
+struct ReachLimits {
+    float dd_min, dd_max;  // squared distances between which pow(dist, falloff) is in [2^-20, 2^20]; dd_max < 0: none
+};
+constexpr float kMost = 1048576.0f;     // 2^20: largest colour component and intensity the tests take
+constexpr float kMostTexel = 1024.0f;   // ... and largest albedo, F0 and metallic
+__device__ __forceinline__ float4 reach_entry(const CfLightData* __restrict__ light)
 {
-    const uint32_t pix = blockIdx.x * 256u + threadIdx.x;
-    if (pix >= n_pixels) return;
-    const float4* t = reinterpret_cast<const float4*>(&gbuf[pix]);
-    const float4 pos = __ldg(&t[0]), nrm = __ldg(&t[1]), alb = __ldg(&t[2]);
-    const V3 P = {pos.x, pos.y, pos.z}, N = {nrm.x, nrm.y, nrm.z}, A = {alb.x, alb.y, alb.z};
-    const float metallic = nrm.w, roughness = alb.w;
-    // Scene.frag:82-115: V, NoV, F0 = mix(baseReflectivity, albedo, metallic), Lo = albedo * albedoMultipler
-    const V3 V = v3_normalize(v3_sub(V3{cam.x, cam.y, cam.z}, P));
-    const float NoV = cf_glsl_max(v3_dot(N, V), 0.0f);
-    const float mi = cf_fsub(1.0f, metallic);
-    const V3 F0 = {cf_fadd(cf_fmul(pc.baseReflectivity, mi), cf_fmul(A.x, metallic)),
-                   cf_fadd(cf_fmul(pc.baseReflectivity, mi), cf_fmul(A.y, metallic)),
-                   cf_fadd(cf_fmul(pc.baseReflectivity, mi), cf_fmul(A.z, metallic))};
-    const float r1 = cf_fadd(roughness, 1.0f);
-    const float alpha_r = cf_fdiv(cf_fmul(r1, r1), 8.0f);  // AlphaDirectLighting (PBRHeader.glsl:32-37)
-    V3 lo = {cf_fmul(A.x, pc.albedoMultipler), cf_fmul(A.y, pc.albedoMultipler), cf_fmul(A.z, pc.albedoMultipler)};
-    uint32_t c = 0;
-    float lin = 0.0f;
-    float alpha = 0.0f;
-    if (fragment_cluster(u, pix % width, pix / width, pos.w, &c, &lin)) {
-        const CfLightCell cell = cells[c];
-        if ((uint64_t)cell.offset + cell.count <= index_count) {
-            alpha = 1.0f;
-            for (uint32_t j = 0; j < cell.count; ++j) {
-                const uint32_t li = indices[cell.offset + j];
-                if (li >= light_count) {
-                    alpha = 0.0f;
-                    continue;
-                }
-                radiance(&lights[li], P, N, V, A, F0, metallic, roughness, alpha_r, NoV, pc, lo);
+    const float4 q = __ldg(reinterpret_cast<const float4*>(&light->position[0]));
+    const float4 col = __ldg(reinterpret_cast<const float4*>(&light->color[0]));
+    const float r = __ldg(&light->radius);
+    const bool plain = r > 0.0f && r <= 1e18f && fabsf(col.x) <= kMost && fabsf(col.y) <= kMost && fabsf(col.z) <= kMost;
+    // a little above r^2: the product is rounded
+    return make_float4(q.x, q.y, q.z, plain ? r * r * 1.000001f : __uint_as_float(0x7f800000u));
+}
+
+// Whether a light adds exactly +0 to a texel.  Its term is ((diff + spec) *
+// rad) * NoL with rad = (color * att) * intensity and att = max(1 - dist /
+// radius, 0) / pow(dist, falloff).
+//   At or beyond the radius the numerator is +0 and att +0: rad is a zero.
+//   Behind the texel's surface, N.d below zero by more than rounding can turn
+//   (the shader's N.L is within 1e-6 of it), NoL is +0.
+// Either way the term is a zero, as long as every other factor is finite, and
+// Radiance's 0 + term is +0.  They are: the distance is inside the limits, so
+// att is at most 2^20 and rad at most 2^60; the light is not opposite the
+// camera, so V + L keeps a length of at least 0.1 and H is a unit vector up to
+// rounding; and the texel is `tame` (see shade_kernel), which bounds diff + spec.
+__device__ __forceinline__ bool out_of_reach(const float4& e, const ReachLimits& lim, V3 P, V3 V, V3 N)
+{
+    const V3 d = v3_sub(V3{e.x, e.y, e.z}, P);
+    const float dd = v3_dot(d, d), vd = v3_dot(V, d), nd = v3_dot(N, d);
+    const bool far = dd >= e.w, behind = nd < 0.0f && nd * nd > 1e-10f * dd && e.w <= 3e38f;
+    return (far || behind) && dd >= lim.dd_min && dd <= lim.dd_max && (vd >= 0.0f || vd * vd <= 0.98f * dd);
+}
+
+struct ShadeArgs {
+    CfClusterForwardUBO u;
+    Image im;
+    CfPBRPushConstant pc;
+    float cam[3];
+    ReachLimits lim;
+    const CfGBufferTexel* gbuf;
+    const CfLightCell* cells;
+    const uint32_t* indices;
+    uint64_t index_count;
+    const CfLightData* lights;
+    float4* out;
+    uint32_t light_count;
+};
+
+// Evaluates the ring's pairs [at, at + n) and adds their terms to the texels'
+// sums, each texel's in the ring's order: pairs of one texel take turns.
+__device__ __forceinline__ void evaluate_pairs(const ShadeArgs& A, ShadeWarp& w, uint32_t at, uint32_t n, uint32_t lane)
+{
+    __syncwarp();
+    const uint32_t t = lane < n ? w.texel[(at + lane) & 63u] : 32u + lane;
+    const uint32_t earlier = __match_any_sync(cfk::kFull, t) & ((1u << lane) - 1u);
+    float term[3] = {0.0f, 0.0f, 0.0f};
+    if (lane < n) radiance(&A.lights[w.light[(at + lane) & 63u]], w, t, A.pc, term);
+    const uint32_t turn = __popc(earlier), turns = __reduce_max_sync(cfk::kFull, turn);
+    for (uint32_t k = 0; k <= turns; ++k) {
+        if (turn == k && lane < n) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) w.lo[c][t] = cf_fadd(w.lo[c][t], term[c]);
+        }
+        __syncwarp();
+    }
+}
+
+// One CTA per tile of texels.  Bound by issue: about 450 instructions a light
+// evaluated, with some twenty IEEE divisions and square roots.  Most listed
+// lights add nothing (of 20 listed on surfaces 3 reach the texel), so each is
+// tested first (out_of_reach, about 35 instructions, from a table in shared
+// memory where the set fits it) and the pairs that may add something are
+// gathered per warp and evaluated 32 at a time, so that no lane idles while
+// others evaluate.  A 1920x1080 G-buffer of surfaces, 20 listed lights a texel:
+// every light evaluated 683 us, with the test 227 us (3600 instructions per 32
+// texels at 3.3 per cycle: 60 % of them in 3.7 evaluations).
+template <uint32_t kSide, uint32_t kThreads>
+__global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__ ShadeArgs A)
+{
+    constexpr uint32_t kPixels = kSide * kSide, kUnits = kPixels / 32;
+    __shared__ __align__(16) float4 table[kTableLights];
+    __shared__ uint16_t order[kPixels];
+    __shared__ TileSort sort;
+    __shared__ TileAxes<kSide> axes;
+    __shared__ ShadeWarp warps[kThreads / 32];
+    const uint32_t lane = threadIdx.x & 31, lt_mask = (1u << lane) - 1u;
+    ShadeWarp& w = warps[threadIdx.x >> 5];
+    const Tile<kSide> tile(A.im);
+    const bool whole = A.light_count <= kTableLights;
+    if (whole)
+        for (uint32_t i = threadIdx.x; i < A.light_count; i += kThreads) table[i] = reach_entry(&A.lights[i]);
+    fill_axes(A.u, A.im, tile, axes);
+    sort_tile<kSide, kThreads>(A.u, A.im, tile, sort, order, [&](uint32_t p) { return __ldg(&A.gbuf[p].position[3]); });
+    for (uint32_t unit; (unit = next_unit(sort, lane)) < kUnits;) {
+        const uint32_t i = order[unit * 32 + lane];
+        const bool valid = i != kNoPixel;
+        if (!__any_sync(cfk::kFull, valid)) continue;
+        uint32_t x = 0, y = 0;
+        float xf = 0.0f, yf = 0.0f;
+        if (valid) {
+            tile.at(A.im, i, x, y);
+            xf = A.im.tiles_x ? axes.tile[0][i % kSide] : tile_coord(x, A.im.tile_w);
+            yf = A.im.tiles_x ? axes.tile[1][i / kSide] : tile_coord(y, A.im.tile_h);
+        }
+        const uint32_t pix = y * A.im.width + x;
+        const float4* t = reinterpret_cast<const float4*>(&A.gbuf[pix]);
+        const float4 pos = __ldg(&t[0]), nrm = __ldg(&t[1]), alb = __ldg(&t[2]);
+        const V3 P = {pos.x, pos.y, pos.z}, N = {nrm.x, nrm.y, nrm.z};
+        const float al[3] = {alb.x, alb.y, alb.z};
+        const float metallic = nrm.w, roughness = alb.w;
+        // Scene.frag:82-115: V, NoV, F0 = mix(baseReflectivity, albedo, metallic), Lo = albedo * albedoMultipler
+        const V3 V = v3_normalize(v3_sub(V3{A.cam[0], A.cam[1], A.cam[2]}, P));
+        const float NoV = cf_glsl_max(v3_dot(N, V), 0.0f);
+        const float mi = cf_fsub(1.0f, metallic);
+        const float r1 = cf_fadd(roughness, 1.0f);
+        const float alpha_r = cf_fdiv(cf_fmul(r1, r1), 8.0f);  // AlphaDirectLighting (PBRHeader.glsl:32-37)
+        const float a = cf_fmul(roughness, roughness), a2 = cf_fmul(a, a);
+        w.f[kPx][lane] = P.x, w.f[kPy][lane] = P.y, w.f[kPz][lane] = P.z;
+        w.f[kNx][lane] = N.x, w.f[kNy][lane] = N.y, w.f[kNz][lane] = N.z;
+        w.f[kVx][lane] = V.x, w.f[kVy][lane] = V.y, w.f[kVz][lane] = V.z;
+        bool colours = true;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float f0 = cf_fadd(cf_fmul(A.pc.baseReflectivity, mi), cf_fmul(al[c], metallic));
+            w.f[kAx + c][lane] = al[c];
+            w.f[kFx + c][lane] = f0;
+            w.lo[c][lane] = cf_fmul(al[c], A.pc.albedoMultipler);
+            colours = colours && fabsf(al[c]) <= kMostTexel && fabsf(f0) <= kMostTexel;
+        }
+        w.f[kA2][lane] = a2;
+        w.f[kAlphaR][lane] = alpha_r;
+        w.f[kGv][lane] = cf_fdiv(NoV, cf_fadd(cf_fmul(NoV, cf_fsub(1.0f, alpha_r)), alpha_r));
+        w.f[kNoV4][lane] = cf_fmul(4.0f, NoV);
+        w.f[kKm][lane] = mi;
+        // Tame: diff + spec is bounded.  V is a unit vector up to rounding, N
+        // hardly longer than one, roughness in [0, 1.8] (alpha_r in [1/8, 1),
+        // so both factors of G are at most 8), colours and metallic moderate
+        // (diff at most 2^31).  NoH^2 is at most nn * (1 + 1.1e-6)
+        // for any unit H, so DistributionGGX's denominator NoH^2 * (a2 - 1) + 1
+        // stays above 3e-6 by the last condition, D below 2^39 and spec below
+        // 2^70.  (All false for NaN.)
+        const float vv = v3_dot(V, V), nn = v3_dot(N, N);
+        const bool tame = colours && vv >= 0.999f && vv <= 1.001f && nn <= 1.0001f && roughness >= 0.0f &&
+                          roughness <= 1.8f && fabsf(metallic) <= kMostTexel && a2 * nn + (1.0f - nn * 1.000002f) > 4e-6f;
+        uint32_t c = 0, off = 0, cnt = 0;
+        float lin = 0.0f, alpha = 0.0f;
+        if (valid && fragment_cluster(A.u, xf, yf, pos.w, &c, &lin)) {
+            const CfLightCell cell = A.cells[c];
+            if ((uint64_t)cell.offset + cell.count <= A.index_count) {
+                alpha = 1.0f;
+                off = cell.offset;
+                cnt = cell.count;
             }
         }
+        bool lit = false;  // a light of the list is one of the set
+        uint32_t put = 0, done = 0;
+        const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
+        for (uint32_t j = 0; j < longest; ++j) {
+            bool need = false;
+            uint32_t li = 0;
+            if (j < cnt) {
+                li = __ldg(&A.indices[off + j]);
+                if (li >= A.light_count) {
+                    alpha = 0.0f;
+                } else {
+                    lit = true;
+                    need = !(tame && out_of_reach(whole ? table[li] : reach_entry(&A.lights[li]), A.lim, P, V, N));
+                }
+            }
+            const uint32_t m = __ballot_sync(cfk::kFull, need);
+            if (!m) continue;
+            if (need) {
+                const uint32_t at = (put + __popc(m & lt_mask)) & 63u;
+                w.light[at] = li;
+                w.texel[at] = lane;
+            }
+            put += __popc(m);
+            if (put - done >= 32) {
+                evaluate_pairs(A, w, done, 32, lane);
+                done += 32;
+            }
+        }
+        if (put > done) evaluate_pairs(A, w, done, put - done, lane);
+        __syncwarp();
+        if (valid) {
+            // the lights out of reach added +0, which turns a -0 sum into +0
+            float lo[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) lo[k] = lit ? cf_fadd(w.lo[k][lane], 0.0f) : w.lo[k][lane];
+            A.out[pix] = make_float4(lo[0], lo[1], lo[2], alpha);
+        }
+        __syncwarp();
     }
-    out[pix] = make_float4(lo.x, lo.y, lo.z, alpha);
+}
+
+// Tiles of 32x32 pixels with 256 threads where an image has enough of them to
+// fill the GPU four times over.  Smaller images take them with 1024 threads
+// (lookup: the finer a tile's depths are sorted, the smaller the box that the
+// all-lights check filters by) or take tiles of 16x16 (shading, whose warps
+// need 3.5 KB of shared memory each; and lookups of less than one small tile
+// per SM).
+constexpr uint64_t kLargePixels = 152ull * 4 * 1024, kSmallPixels = 152ull * 256;
+
+Image image_of(const CfClusterForwardUBO& u, uint32_t width, uint32_t height, uint32_t side)
+{
+    Image im;
+    im.width = width;
+    im.height = height;
+    im.n_pixels = width * height;
+    im.tiles_x = width >= side && height >= side ? (width + side - 1) / side : 0u;
+    im.tile_w = u.screenSize[0] / (float)u.sliceCountX;
+    im.tile_h = u.screenSize[1] / (float)u.sliceCountY;
+    return im;
+}
+
+unsigned image_blocks(const Image& im, uint32_t side)
+{
+    const uint64_t n = (uint64_t)side * side;
+    return im.tiles_x ? im.tiles_x * ((im.height + side - 1) / side) : (unsigned)((im.n_pixels + n - 1) / n);
+}
+
+// Squared distances between which pow(dist, falloff) is in [2^-20, 2^20]:
+// |log2 dist| <= k with k * |falloff| <= 20.
+ReachLimits reach_limits(const CfPBRPushConstant& pc)
+{
+    const float f = std::fabs(pc.lightFalloff);
+    if (!(f <= 20.0f) || !(std::fabs(pc.lightIntensity) <= kMost)) return {0.0f, -1.0f};
+    const int k = f * 62.0f <= 20.0f ? 62 : (int)(20.0f / f);
+    return {std::ldexp(1.0f, -2 * k), std::ldexp(1.0f, 2 * k)};
+}
+
+template <bool kCheck>
+void launch_lookup(const LookupArgs& A, bool large, bool small, cudaStream_t stream)
+{
+    if (large) lookup_kernel<32, 256, kCheck><<<image_blocks(A.im, 32), 256, 0, stream>>>(A);
+    else if (!small) lookup_kernel<32, 1024, kCheck><<<image_blocks(A.im, 32), 1024, 0, stream>>>(A);
+    else lookup_kernel<16, 256, kCheck><<<image_blocks(A.im, 16), 256, 0, stream>>>(A);
 }
 
 }  // namespace
@@ -273,9 +758,22 @@ extern "C" int cf_shade_clusters(const CfClusterForwardUBO* ubo, const float cam
     if ((reinterpret_cast<uintptr_t>(d_lights) | reinterpret_cast<uintptr_t>(d_gbuffer) |
          reinterpret_cast<uintptr_t>(d_out)) & 15)
         return fail(CF_ERROR_INVALID_ARGUMENT, "lights, G-buffer and output must be 16-byte aligned");
-    shade_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        *ubo, make_float3(camera_position[0], camera_position[1], camera_position[2]), *pc, d_gbuffer, width,
-        (uint32_t)n, d_cells, d_indices, index_count, d_lights, light_count, reinterpret_cast<float4*>(d_out));
+    const bool large = n >= kLargePixels;
+    ShadeArgs A;
+    A.u = *ubo;
+    A.im = image_of(*ubo, width, height, large ? 32 : 16);
+    A.pc = *pc;
+    for (int i = 0; i < 3; ++i) A.cam[i] = camera_position[i];
+    A.lim = reach_limits(*pc);
+    A.gbuf = d_gbuffer;
+    A.cells = d_cells;
+    A.indices = d_indices;
+    A.index_count = index_count;
+    A.lights = d_lights;
+    A.out = reinterpret_cast<float4*>(d_out);
+    A.light_count = light_count;
+    if (large) shade_kernel<32, 256><<<image_blocks(A.im, 32), 256, 0, (cudaStream_t)stream>>>(A);
+    else shade_kernel<16, 256><<<image_blocks(A.im, 16), 256, 0, (cudaStream_t)stream>>>(A);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "clustered shading launch");
 }
@@ -299,10 +797,22 @@ extern "C" int cf_lookup_clusters(const CfClusterForwardUBO* ubo, const float* d
     if (n > (1ull << 31)) return fail(CF_ERROR_INVALID_ARGUMENT, "depth buffer of %llu pixels", (unsigned long long)n);
     if (reinterpret_cast<uintptr_t>(d_lights) & 15 || reinterpret_cast<uintptr_t>(d_aabbs) & 15)
         return fail(CF_ERROR_INVALID_ARGUMENT, "lights and AABBs must be 16-byte aligned");
-    lookup_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        *ubo, d_depth, width, (uint32_t)n, d_cells, d_indices, index_count, d_lights, light_count,
-        cap ? cap : 0xFFFFFFFFu,
-        reinterpret_cast<const float4*>(d_aabbs), check_all_lights, d_out);
+    const bool large = n >= kLargePixels, small = n < kSmallPixels;
+    LookupArgs A;
+    A.u = *ubo;
+    A.im = image_of(*ubo, width, height, small ? 16 : 32);
+    A.depth = d_depth;
+    A.cells = d_cells;
+    A.indices = d_indices;
+    A.index_count = index_count;
+    A.lights = d_lights;
+    A.aabbs = reinterpret_cast<const float4*>(d_aabbs);
+    A.out = d_out;
+    A.light_count = light_count;
+    A.cap = cap ? cap : 0xFFFFFFFFu;
+    A.out_aligned = (reinterpret_cast<uintptr_t>(d_out) & 15) == 0;
+    if (check_all_lights) launch_lookup<true>(A, large, small, (cudaStream_t)stream);
+    else launch_lookup<false>(A, large, small, (cudaStream_t)stream);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "cluster lookup launch");
 }
