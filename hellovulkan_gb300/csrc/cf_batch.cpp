@@ -209,7 +209,7 @@ int rebuild(CfBatch* b)
     std::stable_sort(mask_views.begin(), mask_views.end(),
                      [&](uint32_t x, uint32_t y) { return b->views[x].light_count > b->views[y].light_count; });
     for (size_t r = 0; r < mask_views.size(); ++r) b->pos[mask_views[r]] = ns + (uint32_t)r;
-    const uint32_t nm = (uint32_t)mask_views.size(), seg = cfk::mask_seg_lights(most_lights);
+    const uint32_t nm = (uint32_t)mask_views.size(), seg = cfk::mask_seg_lights(most_lights, nm);
     b->staged = ns;
     std::vector<uint32_t> prefix(4 * (size_t)ns), mask_prefix(cfk::kMaskStages * ((size_t)nm + 1));
     size_t ws = 0;
@@ -273,7 +273,7 @@ int rebuild(CfBatch* b)
         cfk::ViewJob& j = b->jobs[b->pos[i]];
         unsigned char* w = b->d_ws + ws_off[i];
         if (b->pos[i] >= ns) {
-            cfk::mask_bind(j.v, mask_lay[i], w, seg, true);
+            cfk::mask_bind(j.v, mask_lay[i], w, seg, nm);
             continue;
         }
         const cfk::WorkspaceLayout& L = lay[i];
@@ -297,7 +297,7 @@ int rebuild(CfBatch* b)
         uint64_t blocks = 0;
         for (uint32_t r = 0; r < nm; ++r) {
             p[r] = (uint32_t)blocks;
-            blocks += cfk::mask_batch_blocks(b->jobs[ns + r].v, (cfk::MaskStage)q);
+            blocks += cfk::mask_batch_blocks(b->jobs[ns + r].v, (cfk::MaskStage)q, nm);
         }
         if (blocks > 0x7fffffffull) return fail(CF_ERROR_INVALID_ARGUMENT, "the batch needs more blocks than a launch holds");
         p[nm] = b->mask.blocks[q] = (uint32_t)blocks;
@@ -321,7 +321,7 @@ int rebuild(CfBatch* b)
         auto on_mask = [&](uint32_t q) { return q >= ns; };
         for (uint32_t q : vs)
             if (on_mask(q)) {
-                mask_ctas += cfk::mask_batch_blocks(b->jobs[q].v, cfk::kMaskScan);
+                mask_ctas += cfk::mask_batch_blocks(b->jobs[q].v, cfk::kMaskScan, nm);
                 mask_groups += b->jobs[q].v.groups;
             }
         vs.erase(std::remove_if(vs.begin(), vs.end(), on_mask), vs.end());

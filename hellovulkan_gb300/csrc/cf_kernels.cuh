@@ -90,8 +90,6 @@ struct ViewCull {
     uint32_t* pool;                  // the units' masks and light indices, in batches
     unsigned long long* pool_head;   // batches asked for
     uint32_t pool_batches;
-    uint32_t max_units;              // units the workspace holds
-    uint32_t run;                    // candidates per unit, at first (see Plan)
     uint32_t seg_lights;
     uint32_t segs;
     uint32_t list_slices;            // slices a list CTA takes
@@ -161,7 +159,7 @@ constexpr CullConfig kStagedConfig{2, 8, 1024, 2, kModeBinned};  // the staged b
 // Most groups the automatic choice gives the hit-mask path: a group reads the
 // totals of earlier groups as sums of 32, so their number grows with the view.
 constexpr uint32_t kMaskMaxGroups = 32768;
-constexpr uint32_t kMaskMaxSlices = 1024;  // slices whose first units a scanning CTA keeps in shared memory
+constexpr uint32_t kMaskMaxSlices = 256;  // slices whose first units a scanning CTA keeps in shared memory
 constexpr uint32_t kMaskMaxRun = 128;      // most candidates per scanning unit
 constexpr uint32_t kMaskGroup = 32;      // clusters per group
 constexpr uint32_t kMaxSegLights = 1024; // most lights per list segment
@@ -177,14 +175,13 @@ struct MaskLayout {
     size_t slice_first, group_total, group_count, block_total, group_boxes, slice_boxes, seg_count, pool_head, slice_total, unit_run,
         unit_count, unit_before, pool, slice_lights, slice_idx, bytes;
     uint32_t pool_batches;
-    uint32_t max_units;
 };
 MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slices, uint32_t lights, uint32_t cap,
                        uint32_t seg_lights);
 // Points v's hit-mask buffers into a workspace (v.lpad set).
-void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg_lights, bool batch);
-// Lights per list segment for a view of its own.
-uint32_t mask_seg_lights(uint32_t lights);
+void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg_lights, uint32_t views);
+// Lights per list segment for a view of `lights` (a batch: the most of its views).
+uint32_t mask_seg_lights(uint32_t lights, uint32_t views);
 
 // Workspace carve-up for one view (cf_cull_lights).  A one-launch view needs
 // only the status block and one 8-byte word per CTA (`partials`).
@@ -325,7 +322,7 @@ struct MaskBatch {
     uint32_t n_views, seg_lights;
     uint32_t blocks[kMaskStages];
 };
-uint32_t mask_batch_blocks(const ViewCull& v, MaskStage stage);
+uint32_t mask_batch_blocks(const ViewCull& v, MaskStage stage, uint32_t views);
 cudaError_t launch_mask_batch(const MaskBatch& b, cudaStream_t stream);
 cudaError_t batch_cull_resident_ctas(const CullConfig& cfg, int* ctas);
 cudaError_t launch_batch_scan(const ViewJob* jobs, uint32_t n_views, cudaStream_t stream);

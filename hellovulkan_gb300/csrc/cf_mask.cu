@@ -17,7 +17,7 @@
 //                  in shared memory.  The masks and the lights' indices go to
 //                  the view's pool.  No warp waits for another, and a dense
 //                  group's work spreads over many.
-//   sum_kernel     one CTA per group: adds up the units' counts
+//   sum_kernel     one CTA per group, or four: adds up the units' counts
 //   emit_kernel    warps write the groups' cells, and the units' hits from
 //                  their masks straight to their places in the packed list
 //
@@ -29,11 +29,11 @@
 // nothing reaches cost nothing.  What is left is latency: the five launches of
 // a single view overlap by programmatic dependent launch, and each is a chain
 // of two to five L2 round trips (0.5 us each) with 0.9 us to the next launch.
-// Batches are bound by issue (2.2 to 2.8 of 4 instructions per cycle in the
-// list and scan launches).  Measured, back-to-back passes, against the staged
-// path: that view 33.8 -> 22.8 us; 65536 lights 77.4 -> 36.5 us; 64 views of the
-// benchmark's mix 367 -> 188 us; 256 animated views of 4096 lights
-// 1474 -> 537 us.
+// Batches are bound by issue (2.3 to 2.5 of 4 instructions per cycle in the
+// list, scan and sum launches).  Measured, back-to-back passes, against the
+// staged path: that view 33.8 -> 22.3 us; 65536 lights 77.4 -> 36.5 us; 64 views
+// of the benchmark's mix 371 -> 130 us; 256 animated views of 4096 lights
+// 1485 -> 346 us.
 //
 // The tests are the ones of cf_device.cuh; pruning by union box is exact: per
 // axis the distance to a box that contains another is never larger, and the
@@ -55,8 +55,10 @@ constexpr uint32_t kGroup = kMaskGroup;  // clusters per group: one per lane
 // Slice and group boxes.
 // ---------------------------------------------------------------------------
 // threads per slice: a view's own launch reduces up to 1024 clusters in one
-// step; a batch has slices enough to fill the GPU with smaller CTAs
-constexpr uint32_t kBoxThreads = 1024, kBoxThreadsBatch = 256;
+// step; a batch has slices enough to fill the GPU with smaller CTAs, whose
+// warps wait less for one another (256 animated views: 359 us with 256 threads,
+// 350 with 128, 346 with 64)
+constexpr uint32_t kBoxThreads = 1024, kBoxThreadsBatch = 64;
 
 __device__ __forceinline__ float4 min4(float4 a, float4 b)
 {
@@ -154,11 +156,17 @@ __global__ void __launch_bounds__(kThreads) box_kernel(const ViewJob* __restrict
 // ---------------------------------------------------------------------------
 constexpr uint32_t kListSlices = 16;         // most slices per CTA
 
+__device__ __forceinline__ bool reaches(const float4& L, const float4& lo, const float4& hi)
+{
+    const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
+    return hit_fast(L, mn, mx);
+}
+
 __device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
 {
     __shared__ uint32_t s_mask[kListSlices][32];
     __shared__ uint32_t s_off[kListSlices][32];
-    __shared__ float4 s_box[2 * kListSlices];
+    __shared__ float4 s_box[2 * kListSlices], s_quad[2 * kListSlices / 4];
     const ViewCull& v = j.v;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     const uint32_t seg = blk % v.segs, z0 = (blk / v.segs) * v.list_slices;
@@ -180,17 +188,31 @@ __device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
     launch_dependents();
     if (tid < 2 * nz) s_box[tid] = v.slice_boxes[2 * z0 + tid];
     __syncthreads();
-    const bool lights = seg * v.seg_lights + warp * 32 < j.light_count;  // whether the warp has any
-    for (uint32_t q = 0; q < nz; ++q) {
-        if (!lights) {
-            if (lane == 0) s_mask[q][warp] = 0u;
-            continue;
+    if (tid < (nz + 3) / 4) {  // the union of every four slices
+        float4 lo = s_box[8 * tid], hi = s_box[8 * tid + 1];
+        for (uint32_t q = 4 * tid + 1; q < min(4 * tid + 4, nz); ++q) {
+            lo = min4(lo, s_box[2 * q]);
+            hi = max4(hi, s_box[2 * q + 1]);
         }
-        const float4 lo = s_box[2 * q], hi = s_box[2 * q + 1];
-        const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
-        const uint32_t m = __ballot_sync(kFull, hit_fast(L, mn, mx));
-        if (lane == 0) s_mask[q][warp] = m;
+        s_quad[2 * tid] = lo;
+        s_quad[2 * tid + 1] = hi;
     }
+    __syncthreads();
+    // The warp's masks; a light that does not reach four slices' union reaches
+    // none of them (most warps reach few slices of the near half).
+    uint32_t reached = 0;  // bit q: slice q lists a light of the warp
+    if (seg * v.seg_lights + warp * 32 < j.light_count)
+        for (uint32_t q0 = 0; q0 < nz; q0 += 4) {
+            if (!__any_sync(kFull, reaches(L, s_quad[q0 / 2], s_quad[q0 / 2 + 1]))) continue;
+            for (uint32_t q = q0; q < min(q0 + 4, nz); ++q) {
+                const uint32_t m = __ballot_sync(kFull, reaches(L, s_box[2 * q], s_box[2 * q + 1]));
+                if (m) {
+                    reached |= 1u << q;
+                    if (lane == 0) s_mask[q][warp] = m;
+                }
+            }
+        }
+    if (lane < nz && !((reached >> lane) & 1u)) s_mask[lane][warp] = 0u;
     __syncthreads();
     for (uint32_t q = warp; q < nz; q += nw) {
         const uint32_t c = lane < nw ? __popc(s_mask[q][lane]) : 0u;
@@ -202,8 +224,8 @@ __device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
         }
     }
     __syncthreads();
-    for (uint32_t q = 0; lights && q < nz; ++q) {
-        const uint32_t m = s_mask[q][warp];
+    for (; reached; reached &= reached - 1) {
+        const uint32_t q = __ffs(reached) - 1, m = s_mask[q][warp];
         if ((m >> lane) & 1u) {
             const size_t at = (size_t)(z0 + q) * v.lpad + seg * v.seg_lights + s_off[q][warp] +
                               __popc(m & ((1u << lane) - 1u));
@@ -493,53 +515,41 @@ __device__ __forceinline__ void scan_unit(const ViewCull& v, const Unit& a, Scan
 }
 
 // The units of a view: first[k] is the first unit of slice k, first[slices]
-// their number; total[k] the slice's candidates; `run` the candidates per
-// unit.  Short runs spread a dense group's work over more warps; they are
-// lengthened when the view would then have more units than its workspace
-// holds, which runs of kMaskMaxRun never are.  Every block of the scan makes
-// the same plan; the first one leaves it in the workspace (slice_first, the
-// run last) for the later launches.
+// their number; total[k] the slice's candidates, kMaskMaxRun to a unit.  Every
+// block of the scan makes the same plan; the first one leaves it in the
+// workspace (slice_first) for the later launches.
 struct Plan {
     uint32_t first[kMaskMaxSlices + 1];
     uint32_t total[kMaskMaxSlices];
     uint32_t warp_units[kScanWarps];
-    uint32_t run;
 };
 
 __device__ __forceinline__ void make_plan(const ViewCull& v, uint32_t gps, Plan& p, bool keep)
 {
     constexpr uint32_t kThreads = kScanWarps * 32;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (uint32_t run = v.run;; run *= 2) {
-        uint32_t base = 0;
-        for (uint32_t k0 = 0; k0 < v.slices; k0 += kThreads) {
-            const uint32_t k = k0 + tid, total = k < v.slices ? __ldg(&v.slice_total[k]) : 0u;
-            const uint32_t n = (total + run - 1) / run * gps, incl = warp_inclusive_scan(n, lane);
-            if (lane == 31) p.warp_units[warp] = incl;
-            __syncthreads();
-            uint32_t at = base + incl - n;
+    uint32_t base = 0;
+    for (uint32_t k0 = 0; k0 < v.slices; k0 += kThreads) {
+        const uint32_t k = k0 + tid, total = k < v.slices ? __ldg(&v.slice_total[k]) : 0u;
+        const uint32_t n = (total + kMaskMaxRun - 1) / kMaskMaxRun * gps, incl = warp_inclusive_scan(n, lane);
+        if (lane == 31) p.warp_units[warp] = incl;
+        __syncthreads();
+        uint32_t at = base + incl - n;
 #pragma unroll
-            for (uint32_t q = 0; q < (uint32_t)kScanWarps; ++q) {
-                at += q < warp ? p.warp_units[q] : 0u;
-                base += p.warp_units[q];
-            }
-            if (k < v.slices) {
-                p.first[k] = at;
-                p.total[k] = total;
-            }
-            __syncthreads();
+        for (uint32_t q = 0; q < (uint32_t)kScanWarps; ++q) {
+            at += q < warp ? p.warp_units[q] : 0u;
+            base += p.warp_units[q];
         }
-        if (base <= v.max_units || run >= kMaskMaxRun) {
-            if (tid == 0) {
-                p.first[v.slices] = base;
-                p.run = run;
-            }
-            break;
+        if (k < v.slices) {
+            p.first[k] = at;
+            p.total[k] = total;
         }
+        __syncthreads();
     }
+    if (tid == 0) p.first[v.slices] = base;
     __syncthreads();
     if (keep)
-        for (uint32_t k = tid; k <= v.slices + 1; k += kThreads) v.slice_first[k] = k <= v.slices ? p.first[k] : p.run;
+        for (uint32_t k = tid; k <= v.slices; k += kThreads) v.slice_first[k] = p.first[k];
 }
 
 __device__ __forceinline__ Unit unit_of(const ViewCull& v, uint32_t gps, const Plan& p, uint32_t u)
@@ -551,15 +561,15 @@ __device__ __forceinline__ Unit unit_of(const ViewCull& v, uint32_t gps, const P
         if (p.first[mid] <= u) k = mid;
         else hi = mid;
     }
-    const uint32_t total = p.total[k], run = p.run;
+    const uint32_t total = p.total[k];
     a.u = u;
     a.k = k;
-    a.runs = (total + run - 1) / run;
+    a.runs = (total + kMaskMaxRun - 1) / kMaskMaxRun;
     const uint32_t gl = (u - p.first[k]) / a.runs;
     a.g = k * gps + gl;
     a.r = u - p.first[k] - gl * a.runs;
-    a.t0 = a.r * run;
-    a.n = min(run, total - a.t0);
+    a.t0 = a.r * kMaskMaxRun;
+    a.n = min(kMaskMaxRun, total - a.t0);
     return a;
 }
 
@@ -575,7 +585,10 @@ __device__ __forceinline__ void scan_body(const ViewCull& v, uint32_t blk, uint3
         scan_unit(v, unit_of(v, gps, p, u), sm[warp], lane);
 }
 
-__global__ void __launch_bounds__(kScanWarps * 32, 8) scan_kernel(const ViewJob* __restrict__ jobs,
+// CTAs per SM: eight leave 64 registers per thread; ten spill nothing but issue
+// more to hide less (256 animated views 395 -> 410 us, one view 23.7 -> 25.1 us)
+constexpr int kScanCtas = 8;
+__global__ void __launch_bounds__(kScanWarps * 32, kScanCtas) scan_kernel(const ViewJob* __restrict__ jobs,
                                                                const uint32_t* __restrict__ prefix, uint32_t n_views,
                                                                const __grid_constant__ ViewJob single)
 {
@@ -595,60 +608,100 @@ __global__ void __launch_bounds__(kScanWarps * 32, 8) scan_kernel(const ViewJob*
 // Group totals.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kSumWarps = 4;
-constexpr uint32_t kSumIlp = 16;
+constexpr uint32_t kSumIlp = 8;  // loads in flight per warp
 
-// Group g: the hits each cluster has in the units before each one, the length
-// of its list, the group's total.  Each warp takes a stretch of the group's
-// units, kSumIlp loads in flight.
-__device__ __forceinline__ void sum_group(const ViewCull& v, uint32_t g)
-{
-    __shared__ uint32_t s_sum[kSumWarps][32];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = v.cap;
-    const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup, k = g / gps;
-    const uint32_t first = v.segs ? __ldg(&v.slice_first[k]) : 0u, end = v.segs ? __ldg(&v.slice_first[k + 1]) : 0u;
-    const uint32_t runs = (end - first) / gps, u0 = first + (g - k * gps) * runs;
-    const uint32_t j0 = warp * runs / kSumWarps, j1 = (warp + 1) * runs / kSumWarps;
-    const uint8_t* __restrict__ counts = v.unit_count + (size_t)u0 * kGroup + lane;
-    uint16_t* __restrict__ before = v.unit_before + (size_t)u0 * kGroup + lane;
-    uint32_t x[kSumIlp];
-    auto load = [&](uint32_t j) {
+// One warp's part of a group's sums: units [j0, j1) of those from u0.  load()
+// gives the lane's cluster's hits in kSumIlp of them.
+struct GroupUnits {
+    const uint8_t* __restrict__ counts;
+    uint16_t* __restrict__ before;
+    uint32_t j0, j1;
+
+    __device__ __forceinline__ void load(uint32_t j, uint32_t x[kSumIlp]) const
+    {
 #pragma unroll
         for (uint32_t e = 0; e < kSumIlp; ++e) x[e] = __ldg(&counts[min(j + e, j1 - 1) * kGroup]);
 #pragma unroll
         for (uint32_t e = 0; e < kSumIlp; ++e) x[e] = j + e < j1 ? x[e] : 0u;
-    };
-    uint32_t sum = 0;
-    for (uint32_t j = j0; j < j1; j += kSumIlp) {
-        load(j);
-#pragma unroll
-        for (uint32_t e = 0; e < kSumIlp; ++e) sum += x[e];
     }
-    s_sum[warp][lane] = sum;
-    __syncthreads();
-    uint32_t at = 0, all = 0;
+    __device__ __forceinline__ uint32_t sum(uint32_t x[kSumIlp]) const
+    {
+        uint32_t s = 0;
+        for (uint32_t j = j0; j < j1; j += kSumIlp) {
+            load(j, x);
 #pragma unroll
-    for (uint32_t q = 0; q < kSumWarps; ++q) {
-        at += q < warp ? s_sum[q][lane] : 0u;
-        all += s_sum[q][lane];
+            for (uint32_t e = 0; e < kSumIlp; ++e) s += x[e];
+        }
+        return s;
     }
-    all = min(all, cap);
-    if (warp == 0) {
-        v.group_count[(size_t)g * kGroup + lane] = (uint16_t)all;
-        const uint32_t total = warp_sum(all);
-        if (lane == 0) {
-            v.group_total[g] = total;
-            if (total) atomicAdd(&v.block_total[g / kGroup], total);
+    // x: as the last load left it
+    __device__ __forceinline__ void write_before(uint32_t x[kSumIlp], uint32_t at, uint32_t cap) const
+    {
+        for (uint32_t j = j0; j < j1; j += kSumIlp) {
+            if (j1 - j0 > kSumIlp) load(j, x);  // else still in registers
+#pragma unroll
+            for (uint32_t e = 0; e < kSumIlp; ++e) {
+                if (j + e < j1) before[(j + e) * kGroup] = (uint16_t)min(at, cap);
+                at += x[e];
+            }
         }
     }
-    for (uint32_t j = j0; j < j1; j += kSumIlp) {
-        if (j1 - j0 > kSumIlp) load(j);  // else still in registers
-#pragma unroll
-        for (uint32_t e = 0; e < kSumIlp; ++e) {
-            if (j + e < j1) before[(j + e) * kGroup] = (uint16_t)min(at, cap);
-            at += x[e];
-        }
+};
+
+__device__ __forceinline__ void write_group(const ViewCull& v, uint32_t g, uint32_t all, uint32_t lane)
+{
+    v.group_count[(size_t)g * kGroup + lane] = (uint16_t)all;
+    const uint32_t total = warp_sum(all);
+    if (lane == 0) {
+        v.group_total[g] = total;
+        if (total) atomicAdd(&v.block_total[g / kGroup], total);
     }
 }
+
+// A CTA's kSumGroups groups: the hits each cluster has in the units before each
+// one, the lengths of the lists, the groups' totals.  A group of few units is
+// one warp's; the CTA's warps share the units of a larger one.
+template <uint32_t kSumGroups>
+__device__ __forceinline__ void sum_groups(const ViewCull& v, uint32_t blk)
+{
+    __shared__ uint32_t s_sum[kSumWarps][32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = v.cap;
+    const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup;
+    uint32_t x[kSumIlp];
+    for (uint32_t q = 0; q < kSumGroups; ++q) {
+        const uint32_t g = blk * kSumGroups + q;
+        if (g >= v.groups) break;
+        const uint32_t k = g / gps;
+        const uint32_t first = v.segs ? __ldg(&v.slice_first[k]) : 0u, end = v.segs ? __ldg(&v.slice_first[k + 1]) : 0u;
+        const uint32_t runs = (end - first) / gps, u0 = first + (g - k * gps) * runs;
+        const bool alone = kSumGroups > 1 && runs <= kSumIlp;
+        if (alone && warp != q) continue;
+        const GroupUnits a = {v.unit_count + (size_t)u0 * kGroup + lane, v.unit_before + (size_t)u0 * kGroup + lane,
+                              alone ? 0u : warp * runs / kSumWarps, alone ? runs : (warp + 1) * runs / kSumWarps};
+        uint32_t sum = a.sum(x);
+        if (alone) {
+            write_group(v, g, min(sum, cap), lane);
+            a.write_before(x, 0, cap);
+            continue;
+        }
+        s_sum[warp][lane] = sum;
+        __syncthreads();
+        uint32_t at = 0, all = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kSumWarps; ++w) {
+            at += w < warp ? s_sum[w][lane] : 0u;
+            all += s_sum[w][lane];
+        }
+        if (warp == 0) write_group(v, g, min(all, cap), lane);
+        a.write_before(x, at, cap);
+        if (kSumGroups > 1) __syncthreads();  // s_sum is the next group's
+    }
+}
+
+// Groups per CTA in a batch: most have a unit or two, or none, and a CTA for
+// each was half launch overhead (the sum launch of 64 mixed views: 42 -> 19 us).
+constexpr uint32_t kSumGroupsBatch = 4;
+static_assert(kSumGroupsBatch <= kSumWarps, "a group of few units is one warp's");
 
 __global__ void __launch_bounds__(kSumWarps * 32) sum_kernel(const ViewJob* __restrict__ jobs,
                                                           const uint32_t* __restrict__ prefix, uint32_t n_views,
@@ -658,9 +711,9 @@ __global__ void __launch_bounds__(kSumWarps * 32) sum_kernel(const ViewJob* __re
     launch_dependents();
     if (jobs) {
         const uint32_t vi = find_view(prefix, n_views, blockIdx.x);
-        sum_group(jobs[vi].v, blockIdx.x - __ldg(&prefix[vi]));
+        sum_groups<kSumGroupsBatch>(jobs[vi].v, blockIdx.x - __ldg(&prefix[vi]));
     } else {
-        sum_group(single.v, blockIdx.x);
+        sum_groups<1>(single.v, blockIdx.x);
     }
 }
 
@@ -678,6 +731,16 @@ __device__ __forceinline__ uint32_t group_base(const ViewCull& v, uint32_t g, ui
     return warp_sum(sum);
 }
 
+// Writes the hits of a unit whose masks were not kept by scanning it again.
+// (Not inlined: the registers it needs would be every warp's.)
+__device__ __noinline__ void emit_unkept(const ViewCull& v, const Unit& a, ScanWarp& s, uint32_t lane, uint32_t pos,
+                                         uint32_t lim)
+{
+    fetch_candidates(v, s, a.k, a.t0, a.n, lane);
+    scan_candidates<true>(s, a.n, lane, load_group(v, a.g, a.k, lane), pos, lim, v.indices);
+    __syncwarp();
+}
+
 // Moves the hits of a unit to their places.
 __device__ __forceinline__ void emit_unit(const ViewCull& v, const Unit& a, uint32_t run, ScanWarp& s, uint32_t lane)
 {
@@ -686,10 +749,8 @@ __device__ __forceinline__ void emit_unit(const ViewCull& v, const Unit& a, uint
     const uint32_t first = group_base(v, a.g, lane) + warp_inclusive_scan(all, lane) - all;
     uint32_t pos = first + before;
     if (__all_sync(kFull, before >= all)) return;  // past the cap in every cluster
-    if (run == kNoRun) {  // the pool had no room: scan again, writing this time
-        fetch_candidates(v, s, a.k, a.t0, a.n, lane);
-        scan_candidates<true>(s, a.n, lane, load_group(v, a.g, a.k, lane), pos, first + all, v.indices);
-        __syncwarp();
+    if (run == kNoRun) {  // the pool had no room
+        emit_unkept(v, a, s, lane, pos, first + all);
         return;
     }
     const uint32_t batches = (run >> kBatchShift) + 1;
@@ -704,23 +765,26 @@ __device__ __forceinline__ void emit_unit(const ViewCull& v, const Unit& a, uint
     for (uint32_t b = 0; b < kBank; ++b) s.idx[b * 32 + lane] = idx[b];
     __syncwarp();
 #pragma unroll
-    for (uint32_t b = 0; b < kBank; ++b) pos = emit_word(word[b], &s.idx[b * 32], v.indices, pos, first + all);
+    for (uint32_t b = 0; b < kBank; ++b) {
+        if (b >= batches) break;
+        pos = emit_word(word[b], &s.idx[b * 32], v.indices, pos, first + all);
+    }
     __syncwarp();
 }
 
-// A block of a view's writing: every warp takes each `step`th group, for its
-// cells, and each `step`th unit that has hits.
+// A block of a view's writing: every warp takes each `step`th unit that has
+// hits, and each `step`th run of kCellGroups groups, for their cells: the base
+// of a group is a sum over all before it, which eight groups share.
+constexpr uint32_t kCellGroups = 8;
 __device__ __forceinline__ void emit_body(const ViewCull& v, uint32_t blk, uint32_t blocks, ScanWarp* sm, Plan& p)
 {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, step = kEmitWarps * blocks;
     const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup;
     uint32_t units = 0;
     if (v.segs) {  // without lights there was no scan
-        for (uint32_t k = threadIdx.x; k <= v.slices + 1; k += kEmitWarps * 32) {
-            const uint32_t x = __ldg(&v.slice_first[k]);
+        for (uint32_t k = threadIdx.x; k <= v.slices; k += kEmitWarps * 32) {
+            p.first[k] = __ldg(&v.slice_first[k]);
             if (k < v.slices) p.total[k] = __ldg(&v.slice_total[k]);
-            if (k <= v.slices) p.first[k] = x;
-            else p.run = x;
         }
         __syncthreads();
         units = p.first[v.slices];
@@ -729,16 +793,29 @@ __device__ __forceinline__ void emit_body(const ViewCull& v, uint32_t blk, uint3
         const uint32_t run = __ldg(&v.unit_run[u]);
         if (run != kNoHits) emit_unit(v, unit_of(v, gps, p, u), run, sm[warp], lane);
     }
-    for (uint32_t g = blk + warp * blocks; g < v.groups; g += step) {
-        const uint32_t k = g / gps, c = k * v.slice_clusters + (g - k * gps) * kGroup + lane;
-        const uint32_t all = __ldg(&v.group_count[(size_t)g * kGroup + lane]);
-        const uint32_t incl = warp_inclusive_scan(all, lane), base = group_base(v, g, lane);
-        if (c < (k + 1) * v.slice_clusters) v.cells[c] = CfLightCell{base + incl - all, all};
-        if (g == v.groups - 1 && lane == 31 && v.total) *v.total = base + incl;
+    for (uint32_t g0 = (blk + warp * blocks) * kCellGroups; g0 < v.groups; g0 += step * kCellGroups) {
+        uint32_t all[kCellGroups];
+#pragma unroll
+        for (uint32_t e = 0; e < kCellGroups; ++e)
+            all[e] = g0 + e < v.groups ? __ldg(&v.group_count[(size_t)(g0 + e) * kGroup + lane]) : 0u;
+        uint32_t base = group_base(v, g0, lane), k = g0 / gps, in_slice = g0 - k * gps;
+#pragma unroll
+        for (uint32_t e = 0; e < kCellGroups; ++e) {
+            if (g0 + e >= v.groups) break;
+            const uint32_t incl = warp_inclusive_scan(all[e], lane), i = in_slice * kGroup + lane;
+            if (i < v.slice_clusters) v.cells[k * v.slice_clusters + i] = CfLightCell{base + incl - all[e], all[e]};
+            base += __shfl_sync(kFull, incl, 31);
+            if (++in_slice == gps) {
+                in_slice = 0;
+                ++k;
+            }
+        }
+        if (g0 + kCellGroups >= v.groups && lane == 0 && v.total) *v.total = base;
     }
 }
 
-__global__ void __launch_bounds__(kEmitWarps * 32, 8) emit_kernel(const ViewJob* __restrict__ jobs,
+constexpr int kEmitCtas = 8;  // per SM, as in the scan
+__global__ void __launch_bounds__(kEmitWarps * 32, kEmitCtas) emit_kernel(const ViewJob* __restrict__ jobs,
                                                                const uint32_t* __restrict__ prefix, uint32_t n_views,
                                                                const __grid_constant__ ViewJob single)
 {
@@ -777,10 +854,9 @@ MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slic
     m.slice_boxes = take((size_t)slices * 2 * sizeof(float4));
     m.seg_count = take((size_t)slices * mask_segments(lpad, seg_lights) * sizeof(uint32_t));
     const size_t units = (size_t)groups * ((lpad + kMaskMaxRun - 1) / kMaskMaxRun);
-    m.max_units = (uint32_t)units;
     m.pool_head = take(sizeof(unsigned long long));
     m.slice_total = take((size_t)slices * sizeof(uint32_t));
-    m.slice_first = take((size_t)(slices + 2) * sizeof(uint32_t));
+    m.slice_first = take((size_t)(slices + 1) * sizeof(uint32_t));
     m.unit_run = take(units * sizeof(uint32_t));
     m.unit_count = take(units * kMaskGroup * sizeof(uint8_t));
     m.unit_before = take(units * kMaskGroup * sizeof(uint16_t));
@@ -795,14 +871,14 @@ MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slic
     return m;
 }
 
-static uint32_t mask_list_slices(uint32_t segs, uint32_t slices)
+static uint32_t mask_list_slices(uint32_t segs, uint32_t slices, uint32_t views)
 {
     // as few slices per CTA as keep the launch to one wave of two CTAs per SM
-    const uint64_t n = ((uint64_t)segs * slices + 303) / 304;
+    const uint64_t n = ((uint64_t)segs * slices * views + 303) / 304;
     return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(n, 4), kListSlices);
 }
 
-void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg_lights, bool batch)
+void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg_lights, uint32_t views)
 {
     v.group_total = reinterpret_cast<uint32_t*>(ws + m.group_total);
     v.group_count = reinterpret_cast<uint16_t*>(ws + m.group_count);
@@ -818,37 +894,44 @@ void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg
     v.unit_before = reinterpret_cast<uint16_t*>(ws + m.unit_before);
     v.pool = reinterpret_cast<uint32_t*>(ws + m.pool);
     v.pool_batches = m.pool_batches;
-    v.max_units = m.max_units;
-    v.run = kMaskMaxRun;
     v.slice_lights = reinterpret_cast<float4*>(ws + m.slice_lights);
     v.slice_idx = reinterpret_cast<uint32_t*>(ws + m.slice_idx);
     v.seg_lights = seg_lights;
     v.segs = mask_segments(v.lpad, seg_lights);
-    v.list_slices = batch ? kListSlices : mask_list_slices(v.segs, v.slices);
+    v.list_slices = mask_list_slices(v.segs, v.slices, views);
 }
 
-uint32_t mask_seg_lights(uint32_t lights) { return lights <= 4096 ? 256u : lights <= 8192 ? 512u : 1024u; }
+// A view alone: as many CTAs as keep the launch to about a wave.  A batch has
+// CTAs enough, and half the threads wait half as long at its barriers: 64
+// views of the benchmark's mix 140.9 us with 1024 lights per segment, 137.6
+// with 512.
+uint32_t mask_seg_lights(uint32_t lights, uint32_t views)
+{
+    return lights <= 4096 ? 256u : lights <= 8192 || views > 1 ? 512u : 1024u;
+}
 uint32_t mask_list_blocks(const ViewCull& v) { return v.segs * ((v.slices + v.list_slices - 1) / v.list_slices); }
 
-// A view's units are rarely more than this part of what its lights could make
-// (every light a candidate in every slice): with 16384 or 65536 lights the
-// 2560x1600 view has one in 50.
-constexpr uint64_t kUnitsPart = 50;
+// Scan CTAs per view.  Each makes the view's plan first, so few are better once
+// there are enough for the GPU: a view gets its share of one resident wave
+// (8 CTAs on each of 152 SMs), and more only where the units that its lights
+// could make (every light a candidate in every slice; with 16384 lights the
+// 2560x1600 view has one in 50) would leave a warp with more than this many.
+// Measured with 200 / 400 / 800 / 1600: 64 mixed views 142.8 / 140.9 / 152.2 /
+// 206.4 us, 256 views of 4096 lights 367.6 / 358.8 / 357.2 / 354.4 us.
+constexpr uint64_t kUnitsPerWarp = 400;
 
-uint32_t mask_scan_blocks(const ViewCull& v, bool batch)
+uint32_t mask_scan_blocks(const ViewCull& v, uint32_t views)
 {
-    const uint64_t most = (uint64_t)v.groups * ((v.lpad + v.run - 1) / v.run);
+    const uint64_t most = (uint64_t)v.groups * ((v.lpad + kMaskMaxRun - 1) / kMaskMaxRun);
     if (most == 0) return 0;
-    // alone: one resident wave (8 CTAs on each of 152 SMs), or fewer for a view
-    // that cannot have as many units; in a batch about two units per warp
-    const uint64_t blocks = batch ? (most / kUnitsPart + 2 * kScanWarps - 1) / (2 * kScanWarps)
-                                  : (most + kScanWarps - 1) / kScanWarps;
-    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(blocks, 152u * 8u));
+    const uint64_t wave = 152u * 8u, one_each = (most + kScanWarps - 1) / kScanWarps;
+    const uint64_t share = std::max((wave + views - 1) / views, one_each / kUnitsPerWarp);
+    return (uint32_t)std::min(std::min(share, one_each), wave);
 }
-uint32_t mask_emit_blocks(const ViewCull& v, bool batch)
+uint32_t mask_emit_blocks(const ViewCull& v, uint32_t views)
 {
-    const uint32_t per = batch ? 4 * kEmitWarps : kEmitWarps;  // groups whose cells a CTA writes, at most
-    return std::max(mask_scan_blocks(v, batch), std::min((v.groups + per - 1) / per, 152u * 8u));
+    const uint32_t per = kCellGroups * kEmitWarps;  // groups whose cells a CTA writes in one step
+    return std::max(mask_scan_blocks(v, views), std::min((v.groups + per - 1) / per, 152u * 8u));
 }
 
 cudaError_t launch_mask_lists(const ViewJob& j, cudaStream_t stream)
@@ -865,7 +948,7 @@ cudaError_t launch_mask_lists(const ViewJob& j, cudaStream_t stream)
 cudaError_t launch_mask_scan(const ViewJob& j, cudaStream_t stream)
 {
     if (j.v.segs == 0) return cudaSuccess;
-    return launch_kernel(true, scan_kernel, dim3(mask_scan_blocks(j.v, false)), dim3(kScanWarps * 32), 0, stream,
+    return launch_kernel(true, scan_kernel, dim3(mask_scan_blocks(j.v, 1)), dim3(kScanWarps * 32), 0, stream,
                          static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
 }
 
@@ -875,7 +958,7 @@ cudaError_t launch_mask_emit(const ViewJob& j, cudaStream_t stream)
                                         0, stream, static_cast<const ViewJob*>(nullptr),
                                         static_cast<const uint32_t*>(nullptr), 0u, j);
     if (e != cudaSuccess) return e;
-    return launch_kernel(true, emit_kernel, dim3(mask_emit_blocks(j.v, false)), dim3(kEmitWarps * 32), 0, stream,
+    return launch_kernel(true, emit_kernel, dim3(mask_emit_blocks(j.v, 1)), dim3(kEmitWarps * 32), 0, stream,
                          static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
 }
 
@@ -901,14 +984,14 @@ cudaError_t launch_mask_batch(const MaskBatch& b, cudaStream_t stream)
     return e;
 }
 
-uint32_t mask_batch_blocks(const ViewCull& v, MaskStage stage)
+uint32_t mask_batch_blocks(const ViewCull& v, MaskStage stage, uint32_t views)
 {
     switch (stage) {
     case kMaskBox: return v.slices;
     case kMaskList: return mask_list_blocks(v);
-    case kMaskScan: return mask_scan_blocks(v, true);
-    case kMaskSum: return v.groups;
-    default: return mask_emit_blocks(v, true);
+    case kMaskScan: return mask_scan_blocks(v, views);
+    case kMaskSum: return (v.groups + kSumGroupsBatch - 1) / kSumGroupsBatch;
+    default: return mask_emit_blocks(v, views);
     }
 }
 

@@ -177,7 +177,7 @@ uint64_t cull_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32
 {
     if (!cfk::is_mask_config(cfg)) return layout_for(ubo, light_count, cap, cfg).bytes;
     const uint32_t xy = ubo.sliceCountX * ubo.sliceCountY;
-    return cfk::mask_layout(xy * ubo.sliceCountZ, xy, ubo.sliceCountZ, light_count, cap, cfk::mask_seg_lights(light_count)).bytes;
+    return cfk::mask_layout(xy * ubo.sliceCountZ, xy, ubo.sliceCountZ, light_count, cap, cfk::mask_seg_lights(light_count, 1)).bytes;
 }
 
 namespace {
@@ -191,8 +191,8 @@ int enqueue_mask(cfk::ViewJob& j, const CfClusterForwardUBO& ubo, const CfLightD
     if (!cfk::mask_fits(v.clusters, v.slice_clusters, v.slices))
         return fail(CF_ERROR_INVALID_ARGUMENT, "%u slices of %u clusters exceed the hit-mask configuration", v.slices,
                     v.slice_clusters);
-    const uint32_t seg = cfk::mask_seg_lights(light_count);
-    cfk::mask_bind(v, cfk::mask_layout(v.clusters, v.slice_clusters, v.slices, light_count, v.cap, seg), ws, seg, false);
+    const uint32_t seg = cfk::mask_seg_lights(light_count, 1);
+    cfk::mask_bind(v, cfk::mask_layout(v.clusters, v.slice_clusters, v.slices, light_count, v.cap, seg), ws, seg, 1);
     j.lights = d_lights;
     j.light_count = light_count;
     for (int i = 0; i < 16; ++i) j.view[i] = ubo.cameraView[i];

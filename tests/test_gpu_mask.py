@@ -90,3 +90,27 @@ def test_sums_are_rounded_as_the_shader_rounds_them(gpu, oracle):
     b.cull(s)
     assert_matches_oracle(oracle, v, *bufs.read(0))
     b.close()
+
+
+@pytest.mark.parametrize("grid", [(8, 8, 2), (15, 9, 13), (33, 1, 7), (5, 1, 255), (3, 1, 257)])
+def test_batches_of_few_and_many_units(gpu, oracle, grid):
+    """A batch whose groups have from no unit to more than a warp adds up by
+    itself (eight of 128 candidates), side by side in one block, with slices
+    that the quick test of four at a time passes over; numbers of groups and of
+    slices that are no multiple of four; the most slices of the hit-mask path
+    and one more."""
+    from hellovulkan_gb300.batch import Batch, BatchBuffers
+    views = []
+    for n in (0, 90, 1100, 3000):
+        rng = np.random.default_rng(n)
+        near = scenes.uniform_box_lights(rng, n, [-3, -2, -4], [3, 2, -3.5], 0.1, 0.6)
+        far = scenes.uniform_box_lights(rng, 60, [-60, -30, -200], [60, 30, -5], 1.0, 9.0)
+        views.append(scenes.custom_view(grid, 1920, 1080, 0.1, 300.0, lights=np.concatenate([far[:30], near, far[30:]])))
+    bufs = BatchBuffers(views)
+    b = Batch(gpu)
+    b.set_views(bufs.batch_views())
+    b.generate_aabbs()
+    b.cull()
+    for q, v in enumerate(views):
+        assert_matches_oracle(oracle, v, *bufs.read(q))
+    b.close()
