@@ -93,6 +93,8 @@ struct ViewCull {
     uint32_t seg_lights;
     uint32_t segs;
     uint32_t list_slices;            // slices a list CTA takes
+    uint32_t scan_groups;            // groups a scanning warp tests a run of candidates against
+    uint32_t sum_groups;             // groups whose units a warp of a batch adds up
     uint32_t lpad;
     uint32_t clusters;
     uint32_t cap;

@@ -17,7 +17,7 @@
 //                  in shared memory.  The masks and the lights' indices go to
 //                  the view's pool.  No warp waits for another, and a dense
 //                  group's work spreads over many.
-//   sum_kernel     one CTA per group, or four: adds up the units' counts
+//   sum_kernel     one CTA per group, or 32: adds up the units' counts
 //   emit_kernel    warps write the groups' cells, and the units' hits from
 //                  their masks straight to their places in the packed list
 //
@@ -29,11 +29,11 @@
 // nothing reaches cost nothing.  What is left is latency: the five launches of
 // a single view overlap by programmatic dependent launch, and each is a chain
 // of two to five L2 round trips (0.5 us each) with 0.9 us to the next launch.
-// Batches are bound by issue (2.3 to 2.5 of 4 instructions per cycle in the
-// list, scan and sum launches).  Measured, back-to-back passes, against the
-// staged path: that view 33.8 -> 22.3 us; 65536 lights 77.4 -> 36.5 us; 64 views
-// of the benchmark's mix 371 -> 130 us; 256 animated views of 4096 lights
-// 1485 -> 346 us.
+// Batches are bound by issue (1.9 to 2.9 of 4 instructions per cycle in the
+// list, scan and write launches).  Measured, back-to-back passes, against the
+// staged path: that view 33.8 -> 21.9 us; 65536 lights 77.4 -> 35.5 us; 64 views
+// of the benchmark's mix 371 -> 106 us; 256 animated views of 4096 lights
+// 1485 -> 234 us.
 //
 // The tests are the ones of cf_device.cuh; pruning by union box is exact: per
 // axis the distance to a box that contains another is never larger, and the
@@ -69,19 +69,28 @@ __device__ __forceinline__ float4 max4(float4 a, float4 b)
     return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), 0.f);
 }
 
-// The union of the lanes' boxes, in every lane.
+__device__ __forceinline__ float warp_min(float x)
+{
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float x)
+{
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The union of the lanes' boxes, in every lane: six instructions, for sixty of a
+// butterfly of shuffles.
 __device__ __forceinline__ void warp_union(float4& lo, float4& hi)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo.x = fminf(lo.x, __shfl_xor_sync(kFull, lo.x, o));
-        lo.y = fminf(lo.y, __shfl_xor_sync(kFull, lo.y, o));
-        lo.z = fminf(lo.z, __shfl_xor_sync(kFull, lo.z, o));
-        hi.x = fmaxf(hi.x, __shfl_xor_sync(kFull, hi.x, o));
-        hi.y = fmaxf(hi.y, __shfl_xor_sync(kFull, hi.y, o));
-        hi.z = fmaxf(hi.z, __shfl_xor_sync(kFull, hi.z, o));
-    }
+    lo = make_float4(warp_min(lo.x), warp_min(lo.y), warp_min(lo.z), 0.f);
+    hi = make_float4(warp_max(hi.x), warp_max(hi.y), warp_max(hi.z), 0.f);
 }
+
+constexpr uint32_t kBoxIlp = 4;  // groups a warp has loads in flight for (256 views: 43 -> 34 us, the traffic's 19)
 
 template <uint32_t kThreads>
 __device__ __forceinline__ void box_body(const ViewCull& v, uint32_t k)
@@ -98,24 +107,32 @@ __device__ __forceinline__ void box_body(const ViewCull& v, uint32_t k)
         if (k == 0) *v.pool_head = 0ull;
     }
     float4 lo = make_float4(inf, inf, inf, 0.f), hi = make_float4(-inf, -inf, -inf, 0.f);
-    for (uint32_t g = warp; g < gps; g += kWarps) {
-        const uint32_t c = g * kGroup + lane;
-        float4 a = make_float4(inf, inf, inf, 0.f), b = make_float4(-inf, -inf, -inf, 0.f);
-        if (c < xy) {
-            a = __ldg(&v.aabbs[2 * ((size_t)k * xy + c)]);
-            b = __ldg(&v.aabbs[2 * ((size_t)k * xy + c) + 1]);
+    for (uint32_t g0 = warp; g0 < gps; g0 += kBoxIlp * kWarps) {
+        float4 a[kBoxIlp], b[kBoxIlp];
+#pragma unroll
+        for (uint32_t e = 0; e < kBoxIlp; ++e) {
+            const uint32_t c = (g0 + e * kWarps) * kGroup + lane;
+            a[e] = make_float4(inf, inf, inf, 0.f);
+            b[e] = make_float4(-inf, -inf, -inf, 0.f);
+            if (c < xy) {
+                a[e] = __ldg(&v.aabbs[2 * ((size_t)k * xy + c)]);
+                b[e] = __ldg(&v.aabbs[2 * ((size_t)k * xy + c) + 1]);
+            }
         }
-        const bool nan = (a.x != a.x) | (a.y != a.y) | (a.z != a.z) | (b.x != b.x) | (b.y != b.y) | (b.z != b.z);
-        warp_union(a, b);
-        if (__any_sync(kFull, nan)) {
-            a = make_float4(-inf, -inf, -inf, 0.f);
-            b = make_float4(inf, inf, inf, 0.f);
-        }
-        lo = min4(lo, a);
-        hi = max4(hi, b);
-        if (lane == 0) {
-            v.group_boxes[2 * ((size_t)k * gps + g)] = a;
-            v.group_boxes[2 * ((size_t)k * gps + g) + 1] = b;
+#pragma unroll
+        for (uint32_t e = 0; e < kBoxIlp; ++e) {
+            const uint32_t g = g0 + e * kWarps;
+            if (g >= gps) break;
+            const bool nan = (a[e].x != a[e].x) | (a[e].y != a[e].y) | (a[e].z != a[e].z) | (b[e].x != b[e].x) |
+                             (b[e].y != b[e].y) | (b[e].z != b[e].z);
+            warp_union(a[e], b[e]);
+            if (__any_sync(kFull, nan)) {
+                a[e] = make_float4(-inf, -inf, -inf, 0.f);
+                b[e] = make_float4(inf, inf, inf, 0.f);
+            }
+            lo = min4(lo, a[e]);
+            hi = max4(hi, b[e]);
+            if (lane < 2) v.group_boxes[2 * ((size_t)k * gps + g) + lane] = lane ? b[e] : a[e];
         }
     }
     if (lane == 0) {
@@ -154,7 +171,9 @@ __global__ void __launch_bounds__(kThreads) box_kernel(const ViewJob* __restrict
 // ---------------------------------------------------------------------------
 // Candidate lists.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kListSlices = 16;         // most slices per CTA
+// Most slices per CTA: its lights are read and transformed once for all of them
+// (256 animated views: 289 us with 16, 279 with 32).
+constexpr uint32_t kListSlices = 32;
 
 __device__ __forceinline__ bool reaches(const float4& L, const float4& lo, const float4& hi)
 {
@@ -236,9 +255,12 @@ __device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
     if (v.work && tid == 0) atomicAdd(&v.work[0], (unsigned long long)nz * blockDim.x);
 }
 
-__global__ void __launch_bounds__(kMaxSegLights, 2) list_kernel(const ViewJob* __restrict__ jobs,
-                                                             const uint32_t* __restrict__ prefix, uint32_t n_views,
-                                                             const __grid_constant__ ViewJob single)
+// Segments of up to 512 lights have CTAs of their own size, four to an SM.
+constexpr uint32_t kSmallSegLights = 512, kSmallListCtas = 4;
+template <uint32_t kThreads, uint32_t kCtas>
+__global__ void __launch_bounds__(kThreads, kCtas) list_kernel(const ViewJob* __restrict__ jobs,
+                                                            const uint32_t* __restrict__ prefix, uint32_t n_views,
+                                                            const __grid_constant__ ViewJob single)
 {
     if (jobs) {
         const uint32_t vi = find_view(prefix, n_views, blockIdx.x);
@@ -273,20 +295,21 @@ constexpr uint32_t kBank = kMaskMaxRun / 32;  // most chunks of 32 candidates pe
 // survivors and their mask words.
 struct ScanWarp {
     float4 in[kBank][32];
-    float x[64], y[64], z[64], r2[64];
+    float x[64], y[64], z[64], r2[64], zz[64];
     uint32_t in_idx[kBank][32];
     uint32_t idx[32 * kBank];
     uint32_t word[kBank][32];
 };
 
-// One lane's cluster box, each bound in both halves of a packed pair.
+// One lane's cluster box, each x and y bound in both halves of a packed pair.
 struct LaneBox {
-    f2 mnx, mny, mnz, mxx, mxy, mxz;
+    f2 mnx, mny, mxx, mxy;
 };
 
 // Mask of the n pending survivors from ring position `at` that reach this
-// lane's box.  Four lights per step, two per packed operation; the ring is
-// padded with never-hit lights to a multiple of four.
+// lane's box, one of a group whose boxes share their z bounds: the ring holds
+// each light's squared z distance.  Four lights per step, two per packed
+// operation; the ring is padded with never-hit lights to a multiple of four.
 __device__ __forceinline__ uint32_t test_pending(const ScanWarp& s, uint32_t at, uint32_t n, const LaneBox& b)
 {
     uint32_t word = 0;
@@ -295,35 +318,37 @@ __device__ __forceinline__ uint32_t test_pending(const ScanWarp& s, uint32_t at,
         const uint32_t p = (at + j) & 63u;  // `at` is a multiple of 32
         const float4 x = *reinterpret_cast<const float4*>(&s.x[p]);
         const float4 y = *reinterpret_cast<const float4*>(&s.y[p]);
-        const float4 z = *reinterpret_cast<const float4*>(&s.z[p]);
+        const float4 zz = *reinterpret_cast<const float4*>(&s.zz[p]);
         const float4 r2 = *reinterpret_cast<const float4*>(&s.r2[p]);
         bool h0, h1, h2, h3;
-        hit_pair_twice_rounded(f2_pack(x.x, x.y), f2_pack(y.x, y.y), f2_pack(z.x, z.y), r2.x, r2.y, b.mnx, b.mny, b.mnz,
-                               b.mxx, b.mxy, b.mxz, h0, h1);
-        hit_pair_twice_rounded(f2_pack(x.z, x.w), f2_pack(y.z, y.w), f2_pack(z.z, z.w), r2.z, r2.w, b.mnx, b.mny, b.mnz,
-                               b.mxx, b.mxy, b.mxz, h2, h3);
+        hit_pair_flat(f2_pack(x.x, x.y), f2_pack(y.x, y.y), zz.x, zz.y, r2.x, r2.y, b.mnx, b.mny, b.mxx, b.mxy, h0, h1);
+        hit_pair_flat(f2_pack(x.z, x.w), f2_pack(y.z, y.w), zz.z, zz.w, r2.z, r2.w, b.mnx, b.mny, b.mxx, b.mxy, h2, h3);
         word |= ((h0 ? 1u : 0u) | (h1 ? 2u : 0u) | (h2 ? 4u : 0u) | (h3 ? 8u : 0u)) << j;
     }
     return word;
 }
 
-// The same with the shader's branchy test, for survivors that include a
-// non-finite coordinate.
-__device__ __noinline__ uint32_t test_pending_exact(const ScanWarp& s, uint32_t at, uint32_t n, const float4 lo,
-                                                    const float4 hi)
+// The same for any boxes and lights, with the shader's branchy test if `exact`
+// (survivors that include a non-finite coordinate).  Out of line and reading
+// the lane's box again: rare, and its registers would be every unit's.
+__device__ __noinline__ uint32_t test_pending_general(const ScanWarp& s, uint32_t at, uint32_t n,
+                                                      const float4* __restrict__ box, bool exact)
 {
+    const float4 lo = __ldg(box), hi = __ldg(box + 1);
     const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
     uint32_t word = 0;
     for (uint32_t j = 0; j < n; ++j) {
         const uint32_t p = (at + j) & 63u;
-        if (hit_exact(make_float4(s.x[p], s.y[p], s.z[p], s.r2[p]), mn, mx)) word |= 1u << j;
+        const float4 L = make_float4(s.x[p], s.y[p], s.z[p], s.r2[p]);
+        if (exact ? hit_exact(L, mn, mx) : hit_fast(L, mn, mx)) word |= 1u << j;
     }
     return word;
 }
 
 // Writes the hits of 32 lights (`word`: the lane's cluster's mask, idx: the
 // lights' indices) in light order at the lane's next place `pos`, up to `lim`,
-// four at a time; returns the place after them.
+// four at a time; returns the place after them.  (All lanes walking the lights
+// of dense words is no faster: a word's fullest lane has 7 to 11 hits.)
 __device__ __forceinline__ uint32_t emit_word(uint32_t word, const uint32_t* idx, uint32_t* __restrict__ out,
                                               uint32_t pos, uint32_t lim)
 {
@@ -344,27 +369,25 @@ __device__ __forceinline__ uint32_t emit_word(uint32_t word, const uint32_t* idx
 
 // One group as a warp sees it: lane i holds cluster i.
 struct GroupLane {
-    float4 lo, hi, ulo, uhi;  // the lane's box (+inf past the slice), the group's union box
+    float4 ulo, uhi;  // the group's union box
     LaneBox box;
+    const float4* at;  // the lane's box (the group's first one past the slice)
     bool present;
+    bool flat;  // the group's boxes share their z bounds (generated clusters of one slice do)
 };
 
 __device__ __forceinline__ GroupLane load_group(const ViewCull& v, uint32_t g, uint32_t k, uint32_t lane)
 {
     const uint32_t xy = v.slice_clusters, gps = (xy + kGroup - 1) / kGroup;
-    const uint32_t c = k * xy + (g - k * gps) * kGroup + lane;
-    const float inf = __uint_as_float(0x7f800000u);
+    const uint32_t c0 = k * xy + (g - k * gps) * kGroup;
     GroupLane q;
-    q.present = c < (k + 1) * xy;
-    q.lo = q.hi = make_float4(inf, inf, inf, 0.f);
-    if (q.present) {
-        q.lo = __ldg(&v.aabbs[2 * (size_t)c]);
-        q.hi = __ldg(&v.aabbs[2 * (size_t)c + 1]);
-    }
+    q.present = c0 + lane < (k + 1) * xy;
+    q.at = &v.aabbs[2 * (size_t)(q.present ? c0 + lane : c0)];
+    const float4 lo = __ldg(q.at), hi = __ldg(q.at + 1);
     q.ulo = __ldg(&v.group_boxes[2 * (size_t)g]);
     q.uhi = __ldg(&v.group_boxes[2 * (size_t)g + 1]);
-    q.box = LaneBox{f2_pack(q.lo.x, q.lo.x), f2_pack(q.lo.y, q.lo.y), f2_pack(q.lo.z, q.lo.z),
-                    f2_pack(q.hi.x, q.hi.x), f2_pack(q.hi.y, q.hi.y), f2_pack(q.hi.z, q.hi.z)};
+    q.box = LaneBox{f2_pack(lo.x, lo.x), f2_pack(lo.y, lo.y), f2_pack(hi.x, hi.x), f2_pack(hi.y, hi.y)};
+    q.flat = __all_sync(kFull, lo.z == q.ulo.z && hi.z == q.uhi.z);
     return q;
 }
 
@@ -425,14 +448,14 @@ __device__ __forceinline__ uint32_t scan_candidates(ScanWarp& s, uint32_t n, uin
         // pad to a multiple of four with lights that reach nothing
         if ((m & 3u) && lane < 4u - (m & 3u)) {
             const uint32_t p = (done + m + lane) & 63u;
-            s.x[p] = s.y[p] = s.z[p] = 0.0f;
+            s.x[p] = s.y[p] = s.z[p] = s.zz[p] = 0.0f;
             s.r2[p] = -inf;
         }
         __syncwarp();
         const uint32_t r = (done + lane) & 63u;
         const bool bad = lane < m && !(finite_bits(s.x[r]) && finite_bits(s.y[r]) && finite_bits(s.z[r]));
-        uint32_t word = __any_sync(kFull, bad) ? test_pending_exact(s, done, m, q.lo, q.hi)
-                                               : test_pending(s, done, m, q.box);
+        const bool exact = __any_sync(kFull, bad);
+        uint32_t word = exact || !q.flat ? test_pending_general(s, done, m, q.at, exact) : test_pending(s, done, m, q.box);
         if (!q.present) word = 0;
         if constexpr (kEmit) {
             count = emit_word(word, &s.idx[done], out, count, lim);
@@ -456,6 +479,8 @@ __device__ __forceinline__ uint32_t scan_candidates(ScanWarp& s, uint32_t n, uin
             s.y[p & 63u] = L.y;
             s.z[p & 63u] = L.z;
             s.r2[p & 63u] = L.w;
+            const float dz = max3f(cf_fsub(q.ulo.z, L.z), cf_fsub(L.z, q.uhi.z), 0.0f);
+            s.zz[p & 63u] = cf_fmul(dz, dz);
             s.idx[p] = s.in_idx[b][lane];
         }
         ns += __popc(m);
@@ -474,17 +499,17 @@ constexpr uint32_t kNoRun = 0xfffffffeu;   // ... has hits, but the pool had no 
 constexpr uint32_t kBatchWords = 64;
 constexpr int kScanWarps = 4;
 
-// Which unit a warp has: run r (of `runs`) of group g in slice k, n candidates
-// from t0 of the slice's list.
+// A unit: group g of slice k, n candidates from t0 of the slice's list.
 struct Unit {
-    uint32_t u, k, g, r, runs, t0, n;
+    uint32_t u, k, g, t0, n;
 };
 
-__device__ __forceinline__ void scan_unit(const ViewCull& v, const Unit& a, ScanWarp& s, uint32_t lane)
+// A warp's unit u: the n candidates in s against group g of slice k.
+__device__ __forceinline__ void scan_unit(const ViewCull& v, uint32_t u, uint32_t g, uint32_t k, uint32_t n, ScanWarp& s,
+                                          uint32_t lane)
 {
-    const uint32_t cap = v.cap, u = a.u, n = a.n;
-    fetch_candidates(v, s, a.k, a.t0, n, lane);
-    const GroupLane q = load_group(v, a.g, a.k, lane);
+    const uint32_t cap = v.cap;
+    const GroupLane q = load_group(v, g, k, lane);
     uint32_t count = q.present ? 0u : cap;
     const uint32_t survivors = scan_candidates<false>(s, n, lane, q, count, cap, nullptr);
     if (v.work && lane == 0) {
@@ -514,31 +539,32 @@ __device__ __forceinline__ void scan_unit(const ViewCull& v, const Unit& a, Scan
     __syncwarp();  // the next unit overwrites the masks
 }
 
-// The units of a view: first[k] is the first unit of slice k, first[slices]
-// their number; total[k] the slice's candidates, kMaskMaxRun to a unit.  Every
-// block of the scan makes the same plan; the first one leaves it in the
-// workspace (slice_first) for the later launches.
+// The runs of a view: slice k's total[k] candidates in runs of kMaskMaxRun,
+// numbered from first[k]; first[slices] is their number.  A run and a group of
+// its slice are a unit: first[k] * groups per slice + group * runs of the
+// slice + run.  Every block of the scan makes the same plan; the first one
+// leaves it in the workspace (slice_first) for the later launches.
 struct Plan {
     uint32_t first[kMaskMaxSlices + 1];
     uint32_t total[kMaskMaxSlices];
-    uint32_t warp_units[kScanWarps];
+    uint32_t warp_runs[kScanWarps];
 };
 
-__device__ __forceinline__ void make_plan(const ViewCull& v, uint32_t gps, Plan& p, bool keep)
+__device__ __forceinline__ void make_plan(const ViewCull& v, Plan& p, bool keep)
 {
     constexpr uint32_t kThreads = kScanWarps * 32;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t base = 0;
     for (uint32_t k0 = 0; k0 < v.slices; k0 += kThreads) {
         const uint32_t k = k0 + tid, total = k < v.slices ? __ldg(&v.slice_total[k]) : 0u;
-        const uint32_t n = (total + kMaskMaxRun - 1) / kMaskMaxRun * gps, incl = warp_inclusive_scan(n, lane);
-        if (lane == 31) p.warp_units[warp] = incl;
+        const uint32_t n = (total + kMaskMaxRun - 1) / kMaskMaxRun, incl = warp_inclusive_scan(n, lane);
+        if (lane == 31) p.warp_runs[warp] = incl;
         __syncthreads();
         uint32_t at = base + incl - n;
 #pragma unroll
         for (uint32_t q = 0; q < (uint32_t)kScanWarps; ++q) {
-            at += q < warp ? p.warp_units[q] : 0u;
-            base += p.warp_units[q];
+            at += q < warp ? p.warp_runs[q] : 0u;
+            base += p.warp_runs[q];
         }
         if (k < v.slices) {
             p.first[k] = at;
@@ -552,41 +578,64 @@ __device__ __forceinline__ void make_plan(const ViewCull& v, uint32_t gps, Plan&
         for (uint32_t k = tid; k <= v.slices; k += kThreads) v.slice_first[k] = p.first[k];
 }
 
-__device__ __forceinline__ Unit unit_of(const ViewCull& v, uint32_t gps, const Plan& p, uint32_t u)
+// The slice of run r (of all).
+__device__ __forceinline__ uint32_t slice_of(const ViewCull& v, const Plan& p, uint32_t r)
 {
-    Unit a;
-    uint32_t k = 0, hi = v.slices;  // first[k] <= u < first[hi]
+    uint32_t k = 0, hi = v.slices;  // first[k] <= r < first[hi]
     while (hi - k > 1) {
         const uint32_t mid = (k + hi) >> 1;
-        if (p.first[mid] <= u) k = mid;
+        if (p.first[mid] <= r) k = mid;
         else hi = mid;
     }
-    const uint32_t total = p.total[k];
-    a.u = u;
-    a.k = k;
-    a.runs = (total + kMaskMaxRun - 1) / kMaskMaxRun;
-    const uint32_t gl = (u - p.first[k]) / a.runs;
-    a.g = k * gps + gl;
-    a.r = u - p.first[k] - gl * a.runs;
-    a.t0 = a.r * kMaskMaxRun;
-    a.n = min(kMaskMaxRun, total - a.t0);
-    return a;
+    return k;
 }
 
-// A block of a view's scan: every warp takes each `step`th unit.  Neighbouring
-// units, of one dense group, so go to different SMs.
+__device__ __forceinline__ Unit unit_of(const ViewCull& v, uint32_t gps, const Plan& p, uint32_t u)
+{
+    const uint32_t k = slice_of(v, p, u / gps), runs = p.first[k + 1] - p.first[k], at = u - p.first[k] * gps;
+    const uint32_t gl = at / runs, t0 = (at - gl * runs) * kMaskMaxRun;
+    return Unit{u, k, k * gps + gl, t0, min(kMaskMaxRun, p.total[k] - t0)};
+}
+
+// Lane i's unit, in every lane.
+__device__ __forceinline__ Unit unit_from(const Unit& a, uint32_t i)
+{
+    return Unit{__shfl_sync(kFull, a.u, i), __shfl_sync(kFull, a.k, i), __shfl_sync(kFull, a.g, i),
+                __shfl_sync(kFull, a.t0, i), __shfl_sync(kFull, a.n, i)};
+}
+
+// A block of a view's scan: every warp takes each `step`th item, a run of
+// candidates against v.scan_groups neighbouring groups.  Neighbouring items, of
+// the same dense groups, so go to different SMs.  The lanes look up 32 items at
+// once.
+template <bool kBatch>
 __device__ __forceinline__ void scan_body(const ViewCull& v, uint32_t blk, uint32_t blocks, ScanWarp* sm, Plan& p)
 {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup;
-    make_plan(v, gps, p, blk == 0);
-    const uint32_t units = p.first[v.slices];
-    for (uint32_t u = blk + warp * blocks; u < units; u += kScanWarps * blocks)
-        scan_unit(v, unit_of(v, gps, p, u), sm[warp], lane);
+    const uint32_t per = kBatch ? v.scan_groups : 1u, parts = (gps + per - 1) / per;  // items per run
+    make_plan(v, p, blk == 0);
+    const uint32_t items = p.first[v.slices] * parts, step = kScanWarps * blocks;
+    for (uint32_t w0 = blk + warp * blocks; w0 < items; w0 += 32 * step) {
+        // the lane's item: part `part` of the groups, run r of slice k
+        const uint32_t w = min(w0 + lane * step, items - 1), k = slice_of(v, p, w / parts);
+        const uint32_t runs = p.first[k + 1] - p.first[k], at = w - p.first[k] * parts, part = at / runs, r = at - part * runs;
+        for (uint32_t i = 0; i < 32 && w0 + i * step < items; ++i) {
+            const uint32_t ik = __shfl_sync(kFull, k, i), ir = __shfl_sync(kFull, r, i);
+            const uint32_t g0 = __shfl_sync(kFull, part, i) * per, g1 = min(g0 + per, gps);
+            const uint32_t iruns = p.first[ik + 1] - p.first[ik], u0 = p.first[ik] * gps + ir;
+            const uint32_t in = min(kMaskMaxRun, p.total[ik] - ir * kMaskMaxRun);
+            fetch_candidates(v, sm[warp], ik, ir * kMaskMaxRun, in, lane);
+            if constexpr (kBatch) {
+                for (uint32_t g = g0; g < g1; ++g)
+                    scan_unit(v, u0 + g * iruns, ik * gps + g, ik, in, sm[warp], lane);
+            } else {
+                scan_unit(v, u0 + g0 * iruns, ik * gps + g0, ik, in, sm[warp], lane);
+            }
+        }
+    }
 }
 
-// CTAs per SM: eight leave 64 registers per thread; ten spill nothing but issue
-// more to hide less (256 animated views 395 -> 410 us, one view 23.7 -> 25.1 us)
 constexpr int kScanCtas = 8;
 __global__ void __launch_bounds__(kScanWarps * 32, kScanCtas) scan_kernel(const ViewJob* __restrict__ jobs,
                                                                const uint32_t* __restrict__ prefix, uint32_t n_views,
@@ -598,9 +647,9 @@ __global__ void __launch_bounds__(kScanWarps * 32, kScanCtas) scan_kernel(const 
     launch_dependents();
     if (jobs) {
         const uint32_t vi = find_view(prefix, n_views, blockIdx.x), b0 = __ldg(&prefix[vi]);
-        scan_body(jobs[vi].v, blockIdx.x - b0, __ldg(&prefix[vi + 1]) - b0, sm, plan);
+        scan_body<true>(jobs[vi].v, blockIdx.x - b0, __ldg(&prefix[vi + 1]) - b0, sm, plan);
     } else {
-        scan_body(single.v, blockIdx.x, gridDim.x, sm, plan);
+        scan_body<false>(single.v, blockIdx.x, gridDim.x, sm, plan);
     }
 }
 
@@ -608,10 +657,13 @@ __global__ void __launch_bounds__(kScanWarps * 32, kScanCtas) scan_kernel(const 
 // Group totals.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kSumWarps = 4;
-constexpr uint32_t kSumIlp = 8;  // loads in flight per warp
+constexpr uint32_t kSumIlp = 8;       // loads in flight per warp
+constexpr uint32_t kSumAlone = 16;    // most units that a warp of a batch adds up by itself
+constexpr uint32_t kSumPerWarp = 8;   // most groups per warp of a batch
 
-// One warp's part of a group's sums: units [j0, j1) of those from u0.  load()
-// gives the lane's cluster's hits in kSumIlp of them.
+// One warp's part of a group's sums: units [j0, j1) of those whose counts start
+// at `counts`.  load() gives the lane's cluster's hits in kSumIlp of them, all
+// asked for at once.
 struct GroupUnits {
     const uint8_t* __restrict__ counts;
     uint16_t* __restrict__ before;
@@ -620,9 +672,7 @@ struct GroupUnits {
     __device__ __forceinline__ void load(uint32_t j, uint32_t x[kSumIlp]) const
     {
 #pragma unroll
-        for (uint32_t e = 0; e < kSumIlp; ++e) x[e] = __ldg(&counts[min(j + e, j1 - 1) * kGroup]);
-#pragma unroll
-        for (uint32_t e = 0; e < kSumIlp; ++e) x[e] = j + e < j1 ? x[e] : 0u;
+        for (uint32_t e = 0; e < kSumIlp; ++e) x[e] = j + e < j1 ? __ldg(&counts[(j + e) * kGroup]) : 0u;
     }
     __device__ __forceinline__ uint32_t sum(uint32_t x[kSumIlp]) const
     {
@@ -634,74 +684,106 @@ struct GroupUnits {
         }
         return s;
     }
-    // x: as the last load left it
-    __device__ __forceinline__ void write_before(uint32_t x[kSumIlp], uint32_t at, uint32_t cap) const
+    // Writes the hits before each unit, `at` before the first one; returns the
+    // hits of all.  `loaded`: x is as the last load left it.
+    __device__ __forceinline__ uint32_t write_before(uint32_t x[kSumIlp], uint32_t at, uint32_t cap, bool loaded) const
     {
         for (uint32_t j = j0; j < j1; j += kSumIlp) {
-            if (j1 - j0 > kSumIlp) load(j, x);  // else still in registers
+            if (!loaded || j1 - j0 > kSumIlp) load(j, x);  // else still in registers
 #pragma unroll
             for (uint32_t e = 0; e < kSumIlp; ++e) {
                 if (j + e < j1) before[(j + e) * kGroup] = (uint16_t)min(at, cap);
                 at += x[e];
             }
         }
+        return at;
     }
 };
 
-__device__ __forceinline__ void write_group(const ViewCull& v, uint32_t g, uint32_t all, uint32_t lane)
+// A group's units: the first one, and how many.
+__device__ __forceinline__ uint2 group_units(const ViewCull& v, uint32_t g, uint32_t gps)
 {
-    v.group_count[(size_t)g * kGroup + lane] = (uint16_t)all;
-    const uint32_t total = warp_sum(all);
-    if (lane == 0) {
-        v.group_total[g] = total;
-        if (total) atomicAdd(&v.block_total[g / kGroup], total);
-    }
+    if (!v.segs) return make_uint2(0u, 0u);
+    const uint32_t k = g / gps, first = __ldg(&v.slice_first[k]), runs = __ldg(&v.slice_first[k + 1]) - first;
+    return make_uint2(first * gps + (g - k * gps) * runs, runs);
 }
 
-// A CTA's kSumGroups groups: the hits each cluster has in the units before each
-// one, the lengths of the lists, the groups' totals.  A group of few units is
-// one warp's; the CTA's warps share the units of a larger one.
-template <uint32_t kSumGroups>
-__device__ __forceinline__ void sum_groups(const ViewCull& v, uint32_t blk)
+// Group g by all warps of the CTA.
+__device__ __forceinline__ void sum_group(const ViewCull& v, uint32_t g, uint2 units, uint32_t lane, uint32_t warp)
 {
     __shared__ uint32_t s_sum[kSumWarps][32];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = v.cap;
-    const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup;
+    const GroupUnits a = {v.unit_count + (size_t)units.x * kGroup + lane, v.unit_before + (size_t)units.x * kGroup + lane,
+                          warp * units.y / kSumWarps, (warp + 1) * units.y / kSumWarps};
     uint32_t x[kSumIlp];
-    for (uint32_t q = 0; q < kSumGroups; ++q) {
-        const uint32_t g = blk * kSumGroups + q;
-        if (g >= v.groups) break;
-        const uint32_t k = g / gps;
-        const uint32_t first = v.segs ? __ldg(&v.slice_first[k]) : 0u, end = v.segs ? __ldg(&v.slice_first[k + 1]) : 0u;
-        const uint32_t runs = (end - first) / gps, u0 = first + (g - k * gps) * runs;
-        const bool alone = kSumGroups > 1 && runs <= kSumIlp;
-        if (alone && warp != q) continue;
-        const GroupUnits a = {v.unit_count + (size_t)u0 * kGroup + lane, v.unit_before + (size_t)u0 * kGroup + lane,
-                              alone ? 0u : warp * runs / kSumWarps, alone ? runs : (warp + 1) * runs / kSumWarps};
-        uint32_t sum = a.sum(x);
-        if (alone) {
-            write_group(v, g, min(sum, cap), lane);
-            a.write_before(x, 0, cap);
-            continue;
-        }
-        s_sum[warp][lane] = sum;
-        __syncthreads();
-        uint32_t at = 0, all = 0;
+    s_sum[warp][lane] = a.sum(x);
+    __syncthreads();
+    uint32_t at = 0, all = 0;
 #pragma unroll
-        for (uint32_t w = 0; w < kSumWarps; ++w) {
-            at += w < warp ? s_sum[w][lane] : 0u;
-            all += s_sum[w][lane];
-        }
-        if (warp == 0) write_group(v, g, min(all, cap), lane);
-        a.write_before(x, at, cap);
-        if (kSumGroups > 1) __syncthreads();  // s_sum is the next group's
+    for (uint32_t w = 0; w < kSumWarps; ++w) {
+        at += w < warp ? s_sum[w][lane] : 0u;
+        all += s_sum[w][lane];
     }
+    if (warp == 0) {
+        all = min(all, v.cap);
+        v.group_count[(size_t)g * kGroup + lane] = (uint16_t)all;
+        const uint32_t total = warp_sum(all);
+        if (lane == 0) {
+            v.group_total[g] = total;
+            if (total) atomicAdd(&v.block_total[g / kGroup], total);
+        }
+    }
+    a.write_before(x, at, v.cap, true);
 }
 
-// Groups per CTA in a batch: most have a unit or two, or none, and a CTA for
-// each was half launch overhead (the sum launch of 64 mixed views: 42 -> 19 us).
-constexpr uint32_t kSumGroupsBatch = 4;
-static_assert(kSumGroupsBatch <= kSumWarps, "a group of few units is one warp's");
+// A block of a batch's groups.  Where most have a unit or two, or none, each warp
+// takes eight, whose first units' counts it asks for at once; the block shares
+// the groups of many units.  A block for each group was mostly its own start: the
+// sum launch of 256 animated views 67 us, 26 with this.
+__device__ __forceinline__ void sum_block(const ViewCull& v, uint32_t blk)
+{
+    __shared__ uint32_t s_large[kSumWarps];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cap = v.cap;
+    const uint32_t gps = (v.slice_clusters + kGroup - 1) / kGroup;
+    const uint32_t g0 = (blk * kSumWarps + warp) * v.sum_groups;
+    const uint32_t n = g0 < v.groups ? min(v.sum_groups, v.groups - g0) : 0u;
+    const uint2 mine = lane < n ? group_units(v, g0 + lane, gps) : make_uint2(0u, 0u);  // lane e: of group g0 + e
+    const uint32_t large = __ballot_sync(kFull, mine.y > kSumAlone);
+    uint32_t first[kSumPerWarp], x[kSumIlp], total = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < kSumPerWarp; ++e) {
+        if (e >= v.sum_groups) break;
+        const uint32_t u = __shfl_sync(kFull, mine.x, e), runs = __shfl_sync(kFull, mine.y, e);
+        first[e] = runs ? __ldg(&v.unit_count[(size_t)u * kGroup + lane]) : 0u;
+    }
+#pragma unroll
+    for (uint32_t e = 0; e < kSumPerWarp; ++e) {
+        if (e >= n) break;
+        const uint32_t u = __shfl_sync(kFull, mine.x, e), runs = __shfl_sync(kFull, mine.y, e);
+        if (runs > kSumAlone) continue;
+        uint32_t all = first[e];
+        if (runs > 1) {  // (that none is before the first unit need not be written)
+            const GroupUnits a = {v.unit_count + (size_t)u * kGroup + lane, v.unit_before + (size_t)u * kGroup + lane, 1, runs};
+            all = a.write_before(x, all, cap, false);
+        }
+        all = min(all, cap);
+        v.group_count[(size_t)(g0 + e) * kGroup + lane] = (uint16_t)all;
+        const uint32_t sum = warp_sum(all);
+        if (lane == e) total = sum;
+    }
+    if (lane < n && !((large >> lane) & 1u)) v.group_total[g0 + lane] = total;
+    const uint32_t sum = warp_sum(total);
+    if (lane == 0) {
+        if (sum) atomicAdd(&v.block_total[g0 / kGroup], sum);
+        s_large[warp] = large;
+    }
+    __syncthreads();
+    for (uint32_t w = 0; w < kSumWarps; ++w)
+        for (uint32_t m = s_large[w]; m; m &= m - 1) {
+            const uint32_t g = (blk * kSumWarps + w) * v.sum_groups + __ffs(m) - 1;
+            sum_group(v, g, group_units(v, g, gps), lane, warp);
+            __syncthreads();  // s_sum is the next group's
+        }
+}
 
 __global__ void __launch_bounds__(kSumWarps * 32) sum_kernel(const ViewJob* __restrict__ jobs,
                                                           const uint32_t* __restrict__ prefix, uint32_t n_views,
@@ -711,9 +793,10 @@ __global__ void __launch_bounds__(kSumWarps * 32) sum_kernel(const ViewJob* __re
     launch_dependents();
     if (jobs) {
         const uint32_t vi = find_view(prefix, n_views, blockIdx.x);
-        sum_groups<kSumGroupsBatch>(jobs[vi].v, blockIdx.x - __ldg(&prefix[vi]));
+        sum_block(jobs[vi].v, blockIdx.x - __ldg(&prefix[vi]));
     } else {
-        sum_groups<1>(single.v, blockIdx.x);
+        const uint32_t gps = (single.v.slice_clusters + kGroup - 1) / kGroup;
+        sum_group(single.v, blockIdx.x, group_units(single.v, blockIdx.x, gps), threadIdx.x & 31, threadIdx.x >> 5);
     }
 }
 
@@ -733,7 +816,7 @@ __device__ __forceinline__ uint32_t group_base(const ViewCull& v, uint32_t g, ui
 
 // Writes the hits of a unit whose masks were not kept by scanning it again.
 // (Not inlined: the registers it needs would be every warp's.)
-__device__ __noinline__ void emit_unkept(const ViewCull& v, const Unit& a, ScanWarp& s, uint32_t lane, uint32_t pos,
+__device__ __noinline__ void emit_unkept(const ViewCull& v, const Unit a, ScanWarp& s, uint32_t lane, uint32_t pos,
                                          uint32_t lim)
 {
     fetch_candidates(v, s, a.k, a.t0, a.n, lane);
@@ -744,22 +827,24 @@ __device__ __noinline__ void emit_unkept(const ViewCull& v, const Unit& a, ScanW
 // Moves the hits of a unit to their places.
 __device__ __forceinline__ void emit_unit(const ViewCull& v, const Unit& a, uint32_t run, ScanWarp& s, uint32_t lane)
 {
-    const uint32_t before = __ldg(&v.unit_before[(size_t)a.u * kGroup + lane]);
+    const uint32_t before = a.t0 ? __ldg(&v.unit_before[(size_t)a.u * kGroup + lane]) : 0u;  // of the first run: none
     const uint32_t all = __ldg(&v.group_count[(size_t)a.g * kGroup + lane]);
-    const uint32_t first = group_base(v, a.g, lane) + warp_inclusive_scan(all, lane) - all;
-    uint32_t pos = first + before;
-    if (__all_sync(kFull, before >= all)) return;  // past the cap in every cluster
-    if (run == kNoRun) {  // the pool had no room
-        emit_unkept(v, a, s, lane, pos, first + all);
-        return;
-    }
-    const uint32_t batches = (run >> kBatchShift) + 1;
-    const uint32_t* __restrict__ in = v.pool + (size_t)(run & ((1u << kBatchShift) - 1)) * kBatchWords + lane;
+    // the masks are asked for with the counts: one round trip
+    const bool kept = run != kNoRun;
+    const uint32_t batches = kept ? (run >> kBatchShift) + 1 : 0u;
+    const uint32_t* __restrict__ in = v.pool + (kept ? (size_t)(run & ((1u << kBatchShift) - 1)) * kBatchWords : 0) + lane;
     uint32_t word[kBank], idx[kBank];
 #pragma unroll
     for (uint32_t b = 0; b < kBank; ++b) {
         word[b] = b < batches ? __ldg(&in[b * kBatchWords]) : 0u;
         idx[b] = b < batches ? __ldg(&in[b * kBatchWords + 32]) : 0u;
+    }
+    const uint32_t first = group_base(v, a.g, lane) + warp_inclusive_scan(all, lane) - all;
+    uint32_t pos = first + before;
+    if (__all_sync(kFull, before >= all)) return;  // past the cap in every cluster
+    if (!kept) {  // the pool had no room
+        emit_unkept(v, a, s, lane, pos, first + all);
+        return;
     }
 #pragma unroll
     for (uint32_t b = 0; b < kBank; ++b) s.idx[b * 32 + lane] = idx[b];
@@ -787,11 +872,15 @@ __device__ __forceinline__ void emit_body(const ViewCull& v, uint32_t blk, uint3
             if (k < v.slices) p.total[k] = __ldg(&v.slice_total[k]);
         }
         __syncthreads();
-        units = p.first[v.slices];
+        units = p.first[v.slices] * gps;
     }
-    for (uint32_t u = blk + warp * blocks; u < units; u += step) {
-        const uint32_t run = __ldg(&v.unit_run[u]);
-        if (run != kNoHits) emit_unit(v, unit_of(v, gps, p, u), run, sm[warp], lane);
+    for (uint32_t u0 = blk + warp * blocks; u0 < units; u0 += 32 * step) {
+        const uint32_t u = u0 + lane * step, run = u < units ? __ldg(&v.unit_run[u]) : kNoHits;
+        const Unit mine = unit_of(v, gps, p, min(u, units - 1));
+        for (uint32_t m = __ballot_sync(kFull, run != kNoHits); m; m &= m - 1) {
+            const uint32_t i = __ffs(m) - 1;
+            emit_unit(v, unit_from(mine, i), __shfl_sync(kFull, run, i), sm[warp], lane);
+        }
     }
     for (uint32_t g0 = (blk + warp * blocks) * kCellGroups; g0 < v.groups; g0 += step * kCellGroups) {
         uint32_t all[kCellGroups];
@@ -871,11 +960,23 @@ MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slic
     return m;
 }
 
+// A view alone has a warp for each unit.  In a batch a warp takes a run of
+// candidates against four groups: a third of a unit's instructions were the
+// look-up and copy of its candidates (256 animated views: 251 us with one
+// group, 237 with two, 234 with four, 236 with eight).
+constexpr uint32_t kScanGroupsBatch = 4;
+// Lights up to which a group of a batch mostly has few units, and a summing warp
+// takes eight groups; past it, one (64 views of up to 65536 lights: 113 us with
+// eight for all, 106 with this line; 8192 or 32768 make no difference there).
+constexpr uint32_t kSumManyLights = 8192;
+
 static uint32_t mask_list_slices(uint32_t segs, uint32_t slices, uint32_t views)
 {
     // as few slices per CTA as keep the launch to one wave of two CTAs per SM
     const uint64_t n = ((uint64_t)segs * slices * views + 303) / 304;
-    return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(n, 4), kListSlices);
+    const uint32_t most = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(n, 4), kListSlices);
+    const uint32_t blocks = (slices + most - 1) / most;
+    return (slices + blocks - 1) / blocks;
 }
 
 void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg_lights, uint32_t views)
@@ -898,6 +999,8 @@ void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg
     v.slice_idx = reinterpret_cast<uint32_t*>(ws + m.slice_idx);
     v.seg_lights = seg_lights;
     v.segs = mask_segments(v.lpad, seg_lights);
+    v.scan_groups = views > 1 ? kScanGroupsBatch : 1;
+    v.sum_groups = v.lpad <= kSumManyLights ? kSumPerWarp : 1;
     v.list_slices = mask_list_slices(v.segs, v.slices, views);
 }
 
@@ -934,13 +1037,18 @@ uint32_t mask_emit_blocks(const ViewCull& v, uint32_t views)
     return std::max(mask_scan_blocks(v, views), std::min((v.groups + per - 1) / per, 152u * 8u));
 }
 
+static auto list_function(uint32_t seg_lights)
+{
+    return seg_lights <= kSmallSegLights ? list_kernel<kSmallSegLights, kSmallListCtas> : list_kernel<kMaxSegLights, 2>;
+}
+
 cudaError_t launch_mask_lists(const ViewJob& j, cudaStream_t stream)
 {
     cudaError_t e = launch_kernel(true, box_kernel<kBoxThreads>, dim3(j.v.slices), dim3(kBoxThreads), 0, stream,
                                   static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
     const uint32_t blocks = mask_list_blocks(j.v);
     if (e == cudaSuccess && blocks)
-        e = launch_kernel(true, list_kernel, dim3(blocks), dim3(j.v.seg_lights), 0, stream,
+        e = launch_kernel(true, list_function(j.v.seg_lights), dim3(blocks), dim3(j.v.seg_lights), 0, stream,
                           static_cast<const ViewJob*>(nullptr), static_cast<const uint32_t*>(nullptr), 0u, j);
     return e;
 }
@@ -970,7 +1078,7 @@ cudaError_t launch_mask_batch(const MaskBatch& b, cudaStream_t stream)
     cudaError_t e = launch_kernel(false, box_kernel<kBoxThreadsBatch>, dim3(b.blocks[kMaskBox]), dim3(kBoxThreadsBatch), 0,
                                   stream, b.jobs, p, n, none);
     if (e == cudaSuccess && b.blocks[kMaskList])
-        e = launch_kernel(false, list_kernel, dim3(b.blocks[kMaskList]), dim3(b.seg_lights), 0, stream, b.jobs,
+        e = launch_kernel(false, list_function(b.seg_lights), dim3(b.blocks[kMaskList]), dim3(b.seg_lights), 0, stream, b.jobs,
                           p + kMaskList * (n + 1), n, none);
     if (e == cudaSuccess && b.blocks[kMaskScan])
         e = launch_kernel(false, scan_kernel, dim3(b.blocks[kMaskScan]), dim3(kScanWarps * 32), 0, stream, b.jobs,
@@ -990,7 +1098,7 @@ uint32_t mask_batch_blocks(const ViewCull& v, MaskStage stage, uint32_t views)
     case kMaskBox: return v.slices;
     case kMaskList: return mask_list_blocks(v);
     case kMaskScan: return mask_scan_blocks(v, views);
-    case kMaskSum: return (v.groups + kSumGroupsBatch - 1) / kSumGroupsBatch;
+    case kMaskSum: return (v.groups + kSumWarps * v.sum_groups - 1) / (kSumWarps * v.sum_groups);
     default: return mask_emit_blocks(v, views);
     }
 }

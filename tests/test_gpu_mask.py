@@ -114,3 +114,37 @@ def test_batches_of_few_and_many_units(gpu, oracle, grid):
     for q, v in enumerate(views):
         assert_matches_oracle(oracle, v, *bufs.read(q))
     b.close()
+
+
+@pytest.mark.parametrize("grid", [(16, 9, 24), (33, 1, 13)])
+def test_boxes_of_other_shapes(gpu, oracle, grid):
+    """Boxes that a caller made, not the generator: z bounds that differ within
+    a group (no squared z distance to share), one group whose bounds differ in
+    a single cluster, a box with a NaN bound; in a batch, and with more lights
+    than a warp's groups of few units go with."""
+    from hellovulkan_gb300.batch import Batch, BatchBuffers
+    rng = np.random.default_rng(53)
+    views = [scenes.custom_view(grid, 1920, 1080, 0.1, 300.0,
+                                lights=scenes.uniform_box_lights(rng, n, [-30, -15, -60], [30, 15, -5], 1.0, 6.0))
+             for n in (300, 9000)]
+    bufs = BatchBuffers(views)
+    b = Batch(gpu)
+    b.set_views(bufs.batch_views())
+    b.generate_aabbs()
+    given = []
+    for q, v in enumerate(views):
+        a = oracle.generate_aabbs(v.ubo)
+        xy = grid[0] * grid[1]
+        a[:5 * xy, 2] -= rng.uniform(0, 2, 5 * xy).astype(np.float32)
+        a[5 * xy: 9 * xy, 6] += rng.uniform(0, 1, 4 * xy).astype(np.float32)
+        a[9 * xy + 7, 6] += np.float32(0.5)
+        a[10 * xy + 3, 0] = np.nan
+        import torch
+        bufs.aabbs[q].copy_(torch.from_numpy(a).reshape(bufs.aabbs[q].shape))
+        given.append(a)
+    b.cull()
+    for q, v in enumerate(views):
+        _, cells, idx = bufs.read(q)
+        oc, oi, _ = oracle.cull(v.ubo, given[q], v.lights, v.cap)
+        assert np.array_equal(cells, oc) and np.array_equal(idx, oi), q
+    b.close()
