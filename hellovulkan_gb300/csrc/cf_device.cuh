@@ -65,6 +65,20 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t x, uint32_t lan
     return x;
 }
 
+// The least and greatest of the lanes' values (a NaN only where all are).
+__device__ __forceinline__ float warp_min(float x)
+{
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float x)
+{
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Index of the view whose range [prefix[v], prefix[v+1]) holds block b.  Every
 // lane takes part: each step narrows the range to a 32nd with one load (a
 // binary search's eight dependent loads were a quarter of a short block's time).

@@ -17,9 +17,9 @@
 // lists: with every pixel at its own depth, unsorted warps had 5 to 10 of 32
 // lanes active.  A sorted warp's fragments also lie in a small box, which few
 // lights of the whole set reach.  1920x1080, 1024 lights, every pixel at its own
-// depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 61 us,
-// shading 1108 -> 139 us; 480x270 with 3000 lights and the all-lights check
-// 805 -> 60 us.
+// depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 55 us,
+// shading 1108 -> 150 us; 480x270 with 3000 lights and the all-lights check
+// 812 -> 52 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -159,11 +159,13 @@ __device__ __forceinline__ void sort_tile(const CfClusterForwardUBO& u, const Im
     }
     __syncthreads();
 #pragma unroll
-    for (uint32_t q = 0; q < kPer; ++q) {  // one count per bin and warp
-        const uint32_t same = __match_any_sync(cfk::kFull, bin[q]), first = __ffs(same) - 1;
-        uint32_t at = 0;
-        if (lane == first) at = atomicAdd(&s.start[bin[q]], (uint32_t)__popc(same));
-        rank[q] = __shfl_sync(cfk::kFull, at, first) + __popc(same & ((1u << lane) - 1u));
+    for (uint32_t q = 0; q < kPer; ++q) {  // the order within a bin is of no account
+        if (__all_sync(cfk::kFull, bin[q] == __shfl_sync(cfk::kFull, bin[q], 0))) {  // a surface: one count for the warp
+            if (lane == 0) rank[q] = atomicAdd(&s.start[bin[q]], 32u);
+            rank[q] = __shfl_sync(cfk::kFull, rank[q], 0) + lane;
+        } else {
+            rank[q] = atomicAdd(&s.start[bin[q]], 1u);
+        }
     }
     __syncthreads();
     if (tid < 32) {
@@ -250,25 +252,71 @@ __device__ __forceinline__ uint32_t count_containing(const float4* table, uint32
     return count;
 }
 
-// The lookup of one pixel whose fragment is at frag; `missing` of s holds the
-// lights of the whole set that contain it, or 0 without the check.  Four list
-// entries are read ahead of their tests.
-constexpr uint32_t kListIlp = 4;
+// 32 lights of a list in view space, one array per component so that four
+// lights' x are one 16-byte read.
+struct ListWarp {
+    float x[32], y[32], z[32], r2[32];
+};
+
+// Mask of the first n lights of w that contain the fragment (those past them,
+// to a multiple of four, reach nothing).  Four lights per step, two per packed
+// operation; the products are rounded before scalar additions.
+__device__ __forceinline__ uint32_t containing(const ListWarp& w, uint32_t n, const float frag[3])
+{
+    const cfk::f2 fx = cfk::f2_pack(frag[0], frag[0]), fy = cfk::f2_pack(frag[1], frag[1]),
+                  fz = cfk::f2_pack(frag[2], frag[2]);
+    uint32_t word = 0;
+#pragma unroll 2
+    for (uint32_t j = 0; j < n; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(&w.x[j]);
+        const float4 y = *reinterpret_cast<const float4*>(&w.y[j]);
+        const float4 z = *reinterpret_cast<const float4*>(&w.z[j]);
+        const float4 r2 = *reinterpret_cast<const float4*>(&w.r2[j]);
+        float xx[4], yy[4], zz[4];
+        cfk::f2 d = cfk::f2_sub(fx, cfk::f2_pack(x.x, x.y));
+        cfk::f2_unpack(cfk::f2_mul(d, d), xx[0], xx[1]);
+        d = cfk::f2_sub(fx, cfk::f2_pack(x.z, x.w));
+        cfk::f2_unpack(cfk::f2_mul(d, d), xx[2], xx[3]);
+        d = cfk::f2_sub(fy, cfk::f2_pack(y.x, y.y));
+        cfk::f2_unpack(cfk::f2_mul(d, d), yy[0], yy[1]);
+        d = cfk::f2_sub(fy, cfk::f2_pack(y.z, y.w));
+        cfk::f2_unpack(cfk::f2_mul(d, d), yy[2], yy[3]);
+        d = cfk::f2_sub(fz, cfk::f2_pack(z.x, z.y));
+        cfk::f2_unpack(cfk::f2_mul(d, d), zz[0], zz[1]);
+        d = cfk::f2_sub(fz, cfk::f2_pack(z.z, z.w));
+        cfk::f2_unpack(cfk::f2_mul(d, d), zz[2], zz[3]);
+        const float lim[4] = {r2.x, r2.y, r2.z, r2.w};
+        uint32_t m = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) m |= cf_fadd(cf_fadd(xx[e], yy[e]), zz[e]) < lim[e] ? 1u << e : 0u;
+        word |= m << j;
+    }
+    return word;
+}
+
+// The lookup of a warp's pixels, whose fragments are at frag; with the check,
+// `missing` of s holds the lights of the whole set that contain the fragment.
+// The warp reads the list of each cluster that its pixels lie in together: a
+// lane fetches and transforms an entry; then each pixel of the cluster tests
+// 32 of them, or, where the cluster has few of the warp's pixels, the lanes
+// test their entries against one pixel after another.
+constexpr uint32_t kFewPixels = 3;  // entries per pixel from which a pixel's turn is cheaper than four entries' test
+constexpr uint32_t kBoxList = 8;    // a list up to this long is not worth a box
 template <bool kCheck>
-__device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table, bool whole, float xf, float yf, float z,
-                                        const float frag[3], CfFragmentSample& s)
+__device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table, bool whole, ListWarp& w, uint32_t lane,
+                                        bool valid, float xf, float yf, float z, const float frag[3], CfFragmentSample& s)
 {
     const CfClusterForwardUBO& u = A.u;
     uint32_t c = 0, off = 0, cnt = 0, in_list = 0;
-    const bool inside = fragment_cluster(u, xf, yf, z, &c, &s.linear_depth);
+    const bool inside = fragment_cluster(u, xf, yf, z, &c, &s.linear_depth) && valid;
     s.view_z = frag[2];
     s.covering = 0;
     s.flags = 0;
+    s.cluster = c;
     if (inside) {
         const CfLightCell cell = A.cells[c];
         off = cell.offset;
         cnt = cell.count;
-        s.cluster = c;
         if ((uint64_t)off + cnt > A.index_count) {  // not a cell of this index list: read nothing through it
             s.flags |= CF_FRAGMENT_BAD_CELL;
             cnt = 0;
@@ -279,59 +327,109 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
             if (frag[0] < lo.x || frag[1] < lo.y || frag[2] < lo.z || frag[0] > hi.x || frag[1] > hi.y || frag[2] > hi.z)
                 s.flags |= CF_FRAGMENT_OUTSIDE_AABB;
         }
+    } else {
+        s.cluster = 0xFFFFFFFFu;
+        s.flags |= CF_FRAGMENT_OUTSIDE_GRID;
+    }
+    for (uint32_t todo = __ballot_sync(cfk::kFull, cnt != 0); todo;) {
+        const uint32_t leader = __ffs(todo) - 1;
+        const uint32_t list_c = __shfl_sync(cfk::kFull, c, leader), list = __shfl_sync(cfk::kFull, off, leader),
+                       n = __shfl_sync(cfk::kFull, cnt, leader);
+        const bool mine = cnt != 0 && c == list_c;
+        const uint32_t pixels = __ballot_sync(cfk::kFull, mine);
+        const uint32_t n_pixels = __popc(pixels);
+        // the box of the cluster's fragments, where the list is worth it
+        const float inf = __uint_as_float(0x7f800000u);
+        float lo[3] = {-inf, -inf, -inf}, hi[3] = {inf, inf, inf};
+        if (n > kBoxList) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {  // a NaN coordinate is in no sphere: the reductions pass it over
+                lo[a] = cfk::warp_min(mine ? frag[a] : inf);
+                hi[a] = cfk::warp_max(mine ? frag[a] : -inf);
+            }
+        }
+        todo &= ~pixels;
         // A light is missing when it is not in the part of the list that a
         // walk over all lights in order would match: the entries up to the
         // first that does not ascend or is no light.
-        bool walked = true;
-        uint32_t before = 0;
-        for (uint32_t j = 0; j < cnt; j += kListIlp) {
-            uint32_t li[kListIlp];
-#pragma unroll
-            for (uint32_t e = 0; e < kListIlp; ++e) li[e] = __ldg(&A.indices[off + min(j + e, cnt - 1)]);
-#pragma unroll
-            for (uint32_t e = 0; e < kListIlp; ++e) {
-                if (j + e >= cnt) break;
-                const bool light = li[e] < A.light_count;
-                if (!light) s.flags |= CF_FRAGMENT_BAD_CELL;
-                if (kCheck) {
-                    walked = walked && light && (j + e == 0 || li[e] > before);
-                    before = li[e];
-                }
-                if (!light) continue;
-                float p[3], r2;
+        uint32_t walked = ~0u, before = 0;
+        uint32_t li = lane < n ? __ldg(&A.indices[list + lane]) : 0u;
+        for (uint32_t j = 0; j < n; j += 32) {
+            const bool has = j + lane < n, light = has && li < A.light_count;
+            const uint32_t here = li;
+            float p[3] = {0.0f, 0.0f, 0.0f}, r2 = __uint_as_float(0xff800000u);  // no light: reaches nothing
+            if (light) {
                 if (whole) {
-                    const float4 L = table[li[e]];
+                    const float4 L = table[here];
                     p[0] = L.x;
                     p[1] = L.y;
                     p[2] = L.z;
                     r2 = L.w;
                 } else {
-                    light_view(u.cameraView, &A.lights[li[e]], p, &r2);
+                    light_view(u.cameraView, &A.lights[here], p, &r2);
                 }
-                const uint32_t hit = contains(frag, p, r2) ? 1u : 0u;
-                s.covering += hit;
-                if (kCheck) in_list += walked ? hit : 0u;
             }
+            if (j + 32 + lane < n) li = __ldg(&A.indices[list + j + 32 + lane]);  // for the next round
+            if (__any_sync(cfk::kFull, has && !light) && mine) s.flags |= CF_FRAGMENT_BAD_CELL;
+            if (kCheck) {
+                uint32_t prev = __shfl_up_sync(cfk::kFull, here, 1);
+                if (lane == 0) prev = before;
+                const uint32_t out = __ballot_sync(cfk::kFull, !light || (j + lane != 0 && here <= prev));
+                if (walked) walked = out ? (out & (0u - out)) - 1u : ~0u;  // those before the first such entry
+                before = __shfl_sync(cfk::kFull, here, 31);
+            }
+            // A light that does not reach the box contains none of the fragments.
+            const bool reach = light && (n <= kBoxList || cfk::hit_fast(make_float4(p[0], p[1], p[2], r2), lo, hi));
+            const uint32_t reached = __ballot_sync(cfk::kFull, reach), ns = __popc(reached);
+            if (kFewPixels * n_pixels < ns) {
+                for (uint32_t m = pixels; m; m &= m - 1) {
+                    const uint32_t t = __ffs(m) - 1;
+                    const float f[3] = {__shfl_sync(cfk::kFull, frag[0], t), __shfl_sync(cfk::kFull, frag[1], t),
+                                        __shfl_sync(cfk::kFull, frag[2], t)};
+                    const uint32_t hits = __ballot_sync(cfk::kFull, contains(f, p, r2));
+                    if (lane == t) {
+                        s.covering += __popc(hits);
+                        if (kCheck) in_list += __popc(hits & walked);
+                    }
+                }
+            } else if (ns) {
+                const uint32_t lower = (1u << lane) - 1u;
+                const uint32_t at = reach ? __popc(reached & lower) : ns + __popc(~reached & lower);
+                w.x[at] = p[0];  // the others follow, and reach nothing
+                w.y[at] = p[1];
+                w.z[at] = p[2];
+                w.r2[at] = reach ? r2 : -inf;
+                __syncwarp();
+                if (mine) {
+                    const uint32_t hits = containing(w, ns, frag);
+                    s.covering += __popc(hits);
+                    // the walked ones are the first of those that reach
+                    if (kCheck) in_list += __popc(hits & (uint32_t)((1ull << __popc(reached & walked)) - 1));
+                }
+                __syncwarp();
+            }
+            if (kCheck && walked != ~0u) walked = 0u;
         }
-    } else {
-        s.cluster = 0xFFFFFFFFu;
-        s.flags |= CF_FRAGMENT_OUTSIDE_GRID;
     }
     s.offset = off;
     s.count = (s.flags & CF_FRAGMENT_BAD_CELL) ? 0u : cnt;
     if (kCheck) s.missing -= in_list;
 }
 
-// One CTA per tile.  Bound by issue: some 300 instructions a pixel apart from
-// its list, six of them IEEE divisions.  A sorted warp's listed loop runs about
-// as long as its mean list; lights come from the table where the whole set fits
-// it.  The all-lights check runs the set through the table in pieces, a filter
-// of 32 lights at a time against the box of the warp's fragments.
+// One CTA per tile.  Bound by issue (62% of the slots at 1920x1080): some 300
+// instructions a pixel apart from its list, six of them IEEE divisions.  A
+// warp's lists cost a transform per 32 entries and a test per entry that
+// reaches its fragments' box; when each lane walked its own list the lookup of
+// that image took 59 us, with 3000 lights on surfaces 193 us (now 72).  With
+// the check, lights come from the table where the whole set fits it; the check
+// runs the set through the table in pieces, 32 lights at a time against the box
+// of the warp's fragments.
 template <uint32_t kSide, uint32_t kThreads, bool kCheck>
-__global__ void __launch_bounds__(kThreads) lookup_kernel(const __grid_constant__ LookupArgs A)
+__global__ void __launch_bounds__(kThreads, 5 * 256 / kThreads) lookup_kernel(const __grid_constant__ LookupArgs A)
 {
     constexpr uint32_t kPixels = kSide * kSide, kUnits = kPixels / 32;
-    __shared__ __align__(16) float4 table[kTableLights];
+    __shared__ __align__(16) float4 table[kCheck ? kTableLights : 1];
+    __shared__ __align__(16) ListWarp lists[kThreads / 32];
     __shared__ uint32_t missing[kCheck ? kPixels : 1];  // by place in the order, between pieces
     __shared__ uint16_t order[kPixels];
     __shared__ TileSort sort;
@@ -339,7 +437,7 @@ __global__ void __launch_bounds__(kThreads) lookup_kernel(const __grid_constant_
     const uint32_t lane = threadIdx.x & 31;
     const CfClusterForwardUBO& u = A.u;
     const Tile<kSide> tile(A.im);
-    const bool whole = A.light_count <= kTableLights;  // the set fits the table
+    const bool whole = kCheck && A.light_count <= kTableLights;  // the set fits the table
     if (whole) fill_table(A, table, 0, A.light_count);
     fill_axes(u, A.im, tile, axes);
     sort_tile<kSide, kThreads>(u, A.im, tile, sort, order, [&](uint32_t p) { return __ldg(&A.depth[p]); });
@@ -384,13 +482,8 @@ __global__ void __launch_bounds__(kThreads) lookup_kernel(const __grid_constant_
                 float lo[3], hi[3];
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {  // a NaN coordinate is in no sphere: fminf and fmaxf pass it over
-                    lo[a] = valid ? frag[a] : inf;
-                    hi[a] = valid ? frag[a] : -inf;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        lo[a] = fminf(lo[a], __shfl_xor_sync(cfk::kFull, lo[a], o));
-                        hi[a] = fmaxf(hi[a], __shfl_xor_sync(cfk::kFull, hi[a], o));
-                    }
+                    lo[a] = cfk::warp_min(valid ? frag[a] : inf);
+                    hi[a] = cfk::warp_max(valid ? frag[a] : -inf);
                 }
                 s.missing = count_containing(table, n, frag, lo, hi, lane) + (piece ? missing[unit * 32 + lane] : 0u);
                 if (piece + 1 < pieces) {
@@ -398,13 +491,16 @@ __global__ void __launch_bounds__(kThreads) lookup_kernel(const __grid_constant_
                     continue;
                 }
             }
+            look_up<kCheck>(A, table, whole, lists[threadIdx.x >> 5], lane, valid, xf, yf, z, frag, s);
             if (!valid) continue;
-            look_up<kCheck>(A, table, whole, xf, yf, z, frag, s);
             CfFragmentSample* out = &A.out[y * A.im.width + x];
             if (A.out_aligned) {
-                uint4* o = reinterpret_cast<uint4*>(out);
-                o[0] = make_uint4(s.cluster, s.offset, s.count, s.covering);
-                o[1] = make_uint4(s.missing, s.flags, __float_as_uint(s.view_z), __float_as_uint(s.linear_depth));
+                // a whole sector; the samples of a large image pass through L2,
+                // and should leave it first
+                asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                             ::"l"(out), "r"(s.cluster), "r"(s.offset), "r"(s.count), "r"(s.covering), "r"(s.missing),
+                             "r"(s.flags), "r"(__float_as_uint(s.view_z)), "r"(__float_as_uint(s.linear_depth))
+                             : "memory");
             } else {
                 *out = s;
             }
@@ -690,13 +786,17 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
     }
 }
 
-// Tiles of 32x32 pixels with 256 threads where an image has enough of them to
-// fill the GPU four times over.  Smaller images take them with 1024 threads
-// (lookup: the finer a tile's depths are sorted, the smaller the box that the
-// all-lights check filters by) or take tiles of 16x16 (shading, whose warps
-// need 3.5 KB of shared memory each; and lookups of less than one small tile
-// per SM).
-constexpr uint64_t kLargePixels = 152ull * 4 * 1024, kSmallPixels = 152ull * 256;
+// A tile of 32x32 pixels, whose sorted warps read one or two lists each, and as
+// many threads as the image's tiles need to fill the GPU: 256 where there are
+// four tiles per SM, 512 down to one, 1024 below that.  A lookup of less than a
+// quarter of a tile per SM takes 16x16.  Lookup without the check, one thread
+// per unsorted pixel / 1024 threads / 512 / tiles of 16x16, in us:
+//   960x540, every pixel at its own depth, 3000 lights    75.4 / 41.2 / 32.8 / 45.5
+//   960x540, surfaces                                     65.9 / 32.2 / 29.3 / 24.9
+//   480x270, every pixel at its own depth                 43.5 / 25.5 / 25.1 / 36.5
+//   480x270, the all-lights check                          812 / 53.1 / 57.9 / 76.4
+// Shading's smaller images take 16x16: its warps need 3.5 KB of shared memory each.
+constexpr uint64_t kLargePixels = 152ull * 4 * 1024, kMiddlePixels = 152ull * 1024, kSmallPixels = 152ull * 256;
 
 Image image_of(const CfClusterForwardUBO& u, uint32_t width, uint32_t height, uint32_t side)
 {
@@ -727,10 +827,12 @@ ReachLimits reach_limits(const CfPBRPushConstant& pc)
 }
 
 template <bool kCheck>
-void launch_lookup(const LookupArgs& A, bool large, bool small, cudaStream_t stream)
+void launch_lookup(const LookupArgs& A, cudaStream_t stream)
 {
-    if (large) lookup_kernel<32, 256, kCheck><<<image_blocks(A.im, 32), 256, 0, stream>>>(A);
-    else if (!small) lookup_kernel<32, 1024, kCheck><<<image_blocks(A.im, 32), 1024, 0, stream>>>(A);
+    const uint64_t n = A.im.n_pixels;
+    if (n >= kLargePixels) lookup_kernel<32, 256, kCheck><<<image_blocks(A.im, 32), 256, 0, stream>>>(A);
+    else if (n >= kMiddlePixels) lookup_kernel<32, 512, kCheck><<<image_blocks(A.im, 32), 512, 0, stream>>>(A);
+    else if (n >= kSmallPixels) lookup_kernel<32, 1024, kCheck><<<image_blocks(A.im, 32), 1024, 0, stream>>>(A);
     else lookup_kernel<16, 256, kCheck><<<image_blocks(A.im, 16), 256, 0, stream>>>(A);
 }
 
@@ -797,10 +899,9 @@ extern "C" int cf_lookup_clusters(const CfClusterForwardUBO* ubo, const float* d
     if (n > (1ull << 31)) return fail(CF_ERROR_INVALID_ARGUMENT, "depth buffer of %llu pixels", (unsigned long long)n);
     if (reinterpret_cast<uintptr_t>(d_lights) & 15 || reinterpret_cast<uintptr_t>(d_aabbs) & 15)
         return fail(CF_ERROR_INVALID_ARGUMENT, "lights and AABBs must be 16-byte aligned");
-    const bool large = n >= kLargePixels, small = n < kSmallPixels;
     LookupArgs A;
     A.u = *ubo;
-    A.im = image_of(*ubo, width, height, small ? 16 : 32);
+    A.im = image_of(*ubo, width, height, n < kSmallPixels ? 16 : 32);
     A.depth = d_depth;
     A.cells = d_cells;
     A.indices = d_indices;
@@ -810,9 +911,9 @@ extern "C" int cf_lookup_clusters(const CfClusterForwardUBO* ubo, const float* d
     A.out = d_out;
     A.light_count = light_count;
     A.cap = cap ? cap : 0xFFFFFFFFu;
-    A.out_aligned = (reinterpret_cast<uintptr_t>(d_out) & 15) == 0;
-    if (check_all_lights) launch_lookup<true>(A, large, small, (cudaStream_t)stream);
-    else launch_lookup<false>(A, large, small, (cudaStream_t)stream);
+    A.out_aligned = (reinterpret_cast<uintptr_t>(d_out) & 31) == 0;
+    if (check_all_lights) launch_lookup<true>(A, (cudaStream_t)stream);
+    else launch_lookup<false>(A, (cudaStream_t)stream);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "cluster lookup launch");
 }

@@ -69,19 +69,6 @@ __device__ __forceinline__ float4 max4(float4 a, float4 b)
     return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), 0.f);
 }
 
-__device__ __forceinline__ float warp_min(float x)
-{
-    float r;
-    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float warp_max(float x)
-{
-    float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 // The union of the lanes' boxes, in every lane: six instructions, for sixty of a
 // butterfly of shuffles.
 __device__ __forceinline__ void warp_union(float4& lo, float4& hi)

@@ -54,6 +54,28 @@ def test_lookup_light_tables(gpu, oracle, n_lights):
     assert same(got, oracle.lookup_clusters(v.ubo, depth, cells, idx, v.lights, v.cap, aabbs, True))
 
 
+@pytest.mark.parametrize("depths", ["scattered", "one", "ramp"])
+@pytest.mark.parametrize("res", [(96, 64), (512, 320)])
+def test_lookup_lists_read_by_a_warp(gpu, oracle, res, depths):
+    """Lists of no light to five times a warp's width, with non-finite lights
+    and entries that are no light in them: clusters with a few of a warp's
+    pixels each, with all of them, and with fragments whose box few of the
+    listed lights reach; images on both sides of a tile per SM."""
+    v, rng = view_of(res, 1500, grid=(3, 2, 16), r=(0.2, 9.0))
+    v.lights[[5, 400], 0], v.lights[9, 1], v.lights[20, 8] = np.nan, -np.inf, np.inf
+    aabbs, cells, idx = run_pipeline(gpu, v)
+    assert cells[:, 1].max() > 96 and (cells[:, 1] < 8).any()
+    idx = idx.copy()
+    idx[rng.integers(0, idx.size, 40)] = rng.choice([1500, 0xFFFFFFFF], 40)
+    if depths == "scattered":
+        depth = scenes.depth_log_uniform(rng, *res, 0.1, 300.0)
+    else:
+        lin = np.full(res[::-1], 20.0) if depths == "one" else np.broadcast_to(np.linspace(2.0, 59.0, res[0]), res[::-1])
+        depth = ((0.1 * 300.0 / lin - 300.0) / (0.1 - 300.0)).astype(np.float32)
+    got = device_lookup(v, depth, cells, idx, aabbs, False)
+    assert same(got, oracle.lookup_clusters(v.ubo, depth, cells, idx, v.lights, v.cap, aabbs, False))
+
+
 def test_lookup_lists_that_do_not_ascend(gpu, oracle):
     """A walk over all lights in order matches a list up to its first entry
     that does not ascend or is no light; the lights after that count as
