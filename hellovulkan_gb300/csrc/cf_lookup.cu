@@ -70,7 +70,8 @@ __device__ __forceinline__ bool contains(const float f[3], const float c[3], flo
 // ---------------------------------------------------------------------------
 // Tiles of pixels, sorted by depth.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kDepthBins = 64;
+constexpr uint32_t kDepthBins = 128;  // of each of a tile's cluster columns, up to four
+constexpr uint32_t kBins = 4 * kDepthBins + 1;  // the last one: past the image
 constexpr uint32_t kNoPixel = 0xffffu;
 
 struct Image {
@@ -127,37 +128,50 @@ __device__ __forceinline__ void fill_axes(const CfClusterForwardUBO& u, const Im
     a.clip[axis][i] = clip_coord(p, u.screenSize[axis]);
 }
 
-// A pixel's depth bin: a quarter of an octave of the denominator of
+// A pixel's depth bin: an eighth of an octave of the denominator of
 // LinearDepth, so of the linear depth itself.  It orders the work and nothing
 // else; a depth outside [0, 1] or a NaN gets some bin.
 __device__ __forceinline__ uint32_t depth_bin(const CfClusterForwardUBO& u, float z)
 {
     const float t = u.cameraFar + z * (u.cameraNear - u.cameraFar);
-    const int b = ((int)__float_as_uint(t) - (int)__float_as_uint(u.cameraNear)) >> 21;
-    return (uint32_t)min(max(b, 0), (int)kDepthBins - 2);
+    const int b = ((int)__float_as_uint(t) - (int)__float_as_uint(u.cameraNear)) >> 20;
+    return (uint32_t)min(max(b, 0), (int)kDepthBins - 1);
 }
 
 struct TileSort {
-    uint32_t start[kDepthBins];
+    uint32_t start[(kBins + 31) / 32 * 32];
     uint32_t next;  // unit not yet taken
 };
 
-// order[]: the tile's pixels by depth bin, those past the image (kNoPixel)
-// last.  `depth` gives a pixel's depth.  Every thread of the CTA takes part.
-template <uint32_t kSide, uint32_t kThreads, typename Depth>
+// order[]: the tile's pixels by cluster column, if asked (left or right of the
+// first boundary in the tile, above or below it), and depth bin, those past the
+// image (kNoPixel) last.  `depth` gives a pixel's depth.  Every thread of the CTA
+// takes part.
+template <bool kColumns, uint32_t kSide, uint32_t kThreads, typename Depth>
 __device__ __forceinline__ void sort_tile(const CfClusterForwardUBO& u, const Image& im, const Tile<kSide>& tile,
-                                          TileSort& s, uint16_t* order, Depth depth)
+                                          const TileAxes<kSide>& axes, TileSort& s, uint16_t* order, Depth depth)
 {
     constexpr uint32_t kPer = kSide * kSide / kThreads;
     const uint32_t tid = threadIdx.x, lane = tid & 31;
-    if (tid < kDepthBins) s.start[tid] = 0;
+    constexpr uint32_t kSlots = sizeof(s.start) / sizeof(s.start[0]);
+    for (uint32_t b = tid; b < kSlots; b += kThreads) s.start[b] = 0;
     uint32_t bin[kPer], rank[kPer];
 #pragma unroll
     for (uint32_t q = 0; q < kPer; ++q) {
         uint32_t x, y;
-        bin[q] = tile.at(im, q * kThreads + tid, x, y) ? depth_bin(u, depth(y * im.width + x)) : kDepthBins - 1;
+        const uint32_t i = q * kThreads + tid;
+        bin[q] = tile.at(im, i, x, y) ? depth_bin(u, depth(y * im.width + x)) : kBins - 1;
     }
-    __syncthreads();
+    __syncthreads();  // also the axes'
+    if (kColumns && im.tiles_x) {
+        const float x1 = floorf(axes.tile[0][0]) + 1.0f, y1 = floorf(axes.tile[1][0]) + 1.0f;
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; ++q) {
+            const uint32_t i = q * kThreads + tid;
+            if (bin[q] != kBins - 1)
+                bin[q] += (axes.tile[0][i % kSide] >= x1 ? kDepthBins : 0u) + (axes.tile[1][i / kSide] >= y1 ? 2 * kDepthBins : 0u);
+        }
+    }
 #pragma unroll
     for (uint32_t q = 0; q < kPer; ++q) {  // the order within a bin is of no account
         if (__all_sync(cfk::kFull, bin[q] == __shfl_sync(cfk::kFull, bin[q], 0))) {  // a surface: one count for the warp
@@ -169,16 +183,22 @@ __device__ __forceinline__ void sort_tile(const CfClusterForwardUBO& u, const Im
     }
     __syncthreads();
     if (tid < 32) {
-        const uint32_t a = s.start[2 * tid], b = s.start[2 * tid + 1];
-        const uint32_t incl = cfk::warp_inclusive_scan(a + b, tid);
-        s.start[2 * tid] = incl - a - b;
-        s.start[2 * tid + 1] = incl - b;
+        constexpr uint32_t kEach = kSlots / 32;
+        uint32_t n = 0, c[kEach];
+#pragma unroll
+        for (uint32_t b = 0; b < kEach; ++b) n += c[b] = s.start[kEach * tid + b];
+        n = cfk::warp_inclusive_scan(n, tid) - n;
+#pragma unroll
+        for (uint32_t b = 0; b < kEach; ++b) {
+            s.start[kEach * tid + b] = n;
+            n += c[b];
+        }
         if (tid == 0) s.next = 0;
     }
     __syncthreads();
 #pragma unroll
     for (uint32_t q = 0; q < kPer; ++q)
-        order[s.start[bin[q]] + rank[q]] = (uint16_t)(bin[q] == kDepthBins - 1 ? kNoPixel : q * kThreads + tid);
+        order[s.start[bin[q]] + rank[q]] = (uint16_t)(bin[q] == kBins - 1 ? kNoPixel : q * kThreads + tid);
     __syncthreads();
 }
 
@@ -354,8 +374,8 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
         // first that does not ascend or is no light.
         uint32_t walked = ~0u, before = 0;
         uint32_t li = lane < n ? __ldg(&A.indices[list + lane]) : 0u;
-        for (uint32_t j = 0; j < n; j += 32) {
-            const bool has = j + lane < n, light = has && li < A.light_count;
+        for (uint32_t j = 0;; j += 32) {
+            const bool has = lane < n - j, more = n - j > 32, light = has && li < A.light_count;
             const uint32_t here = li;
             float p[3] = {0.0f, 0.0f, 0.0f}, r2 = __uint_as_float(0xff800000u);  // no light: reaches nothing
             if (light) {
@@ -369,7 +389,7 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
                     light_view(u.cameraView, &A.lights[here], p, &r2);
                 }
             }
-            if (j + 32 + lane < n) li = __ldg(&A.indices[list + j + 32 + lane]);  // for the next round
+            if (more && lane < n - j - 32) li = __ldg(&A.indices[list + j + 32 + lane]);  // for the next round
             if (__any_sync(cfk::kFull, has && !light) && mine) s.flags |= CF_FRAGMENT_BAD_CELL;
             if (kCheck) {
                 uint32_t prev = __shfl_up_sync(cfk::kFull, here, 1);
@@ -409,6 +429,7 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
                 __syncwarp();
             }
             if (kCheck && walked != ~0u) walked = 0u;
+            if (!more) break;
         }
     }
     s.offset = off;
@@ -440,7 +461,7 @@ __global__ void __launch_bounds__(kThreads, 5 * 256 / kThreads) lookup_kernel(co
     const bool whole = kCheck && A.light_count <= kTableLights;  // the set fits the table
     if (whole) fill_table(A, table, 0, A.light_count);
     fill_axes(u, A.im, tile, axes);
-    sort_tile<kSide, kThreads>(u, A.im, tile, sort, order, [&](uint32_t p) { return __ldg(&A.depth[p]); });
+    sort_tile<!kCheck, kSide, kThreads>(u, A.im, tile, axes, sort, order, [&](uint32_t p) { return __ldg(&A.depth[p]); });
     const uint32_t pieces = kCheck ? (A.light_count + kTableLights - 1) / kTableLights : 0u;
     for (uint32_t piece = 0; piece < max(pieces, 1u); ++piece) {
         const uint32_t n = pieces ? min(kTableLights, A.light_count - piece * kTableLights) : 0u;
@@ -537,9 +558,11 @@ enum TexelField { kPx, kPy, kPz, kNx, kNy, kNz, kVx, kVy, kVz, kAx, kAy, kAz, kF
 // Shared memory of one shading warp.
 struct ShadeWarp {
     float f[kTexelFields][32];
-    float lo[3][32];       // the texels' sums so far
+    float term[3][32];     // what the pairs being evaluated add
+    uint32_t pairs[32];    // ... and which of them are a texel's
     uint32_t light[64];    // ring of (light, texel) pairs to evaluate
     uint32_t texel[64];
+    float x[32], y[32], z[32], e[32];  // a list's lights as out_of_reach sees them
 };
 
 // Radiance (Radiance.glsl:2-57) of one light at texel t of w, in the shader's
@@ -616,12 +639,46 @@ __device__ __forceinline__ float4 reach_entry(const CfLightData* __restrict__ li
 // att is at most 2^20 and rad at most 2^60; the light is not opposite the
 // camera, so V + L keeps a length of at least 0.1 and H is a unit vector up to
 // rounding; and the texel is `tame` (see shade_kernel), which bounds diff + spec.
-__device__ __forceinline__ bool out_of_reach(const float4& e, const ReachLimits& lim, V3 P, V3 V, V3 N)
+// With d from the texel to the light: dd = d.d, vd = V.d, nd = N.d; e: the
+// light's reach_entry squared distance.
+__device__ __forceinline__ bool out_of_reach(float e, const ReachLimits& lim, float dd, float vd, float nd)
 {
-    const V3 d = v3_sub(V3{e.x, e.y, e.z}, P);
-    const float dd = v3_dot(d, d), vd = v3_dot(V, d), nd = v3_dot(N, d);
-    const bool far = dd >= e.w, behind = nd < 0.0f && nd * nd > 1e-10f * dd && e.w <= 3e38f;
+    const bool far = dd >= e, behind = nd < 0.0f && nd * nd > 1e-10f * dd && e <= 3e38f;
     return (far || behind) && dd >= lim.dd_min && dd <= lim.dd_max && (vd >= 0.0f || vd * vd <= 0.98f * dd);
+}
+
+// The same for the first n lights of w (n up to 32, rounded up to four) at one
+// texel: a mask of those that may add something.  Two lights per packed
+// operation, and fused ones: the test's margins are wider than any rounding.
+__device__ __forceinline__ uint32_t within_reach(const ShadeWarp& w, uint32_t n, const ReachLimits& lim, V3 P, V3 V, V3 N)
+{
+    using namespace cfk;
+    const f2 px = f2_pack(P.x, P.x), py = f2_pack(P.y, P.y), pz = f2_pack(P.z, P.z), vx = f2_pack(V.x, V.x),
+             vy = f2_pack(V.y, V.y), vz = f2_pack(V.z, V.z), nx = f2_pack(N.x, N.x), ny = f2_pack(N.y, N.y),
+             nz = f2_pack(N.z, N.z);
+    uint32_t word = 0;
+    for (uint32_t j = 0; j < n; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(&w.x[j]);
+        const float4 y = *reinterpret_cast<const float4*>(&w.y[j]);
+        const float4 z = *reinterpret_cast<const float4*>(&w.z[j]);
+        const float4 e = *reinterpret_cast<const float4*>(&w.e[j]);
+        const float far[4] = {e.x, e.y, e.z, e.w};
+        float dd[4], vd[4], nd[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const f2 dx = f2_sub(h ? f2_pack(x.z, x.w) : f2_pack(x.x, x.y), px),
+                     dy = f2_sub(h ? f2_pack(y.z, y.w) : f2_pack(y.x, y.y), py),
+                     dz = f2_sub(h ? f2_pack(z.z, z.w) : f2_pack(z.x, z.y), pz);
+            f2_unpack(f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx))), dd[2 * h], dd[2 * h + 1]);
+            f2_unpack(f2_fma(vz, dz, f2_fma(vy, dy, f2_mul(vx, dx))), vd[2 * h], vd[2 * h + 1]);
+            f2_unpack(f2_fma(nz, dz, f2_fma(ny, dy, f2_mul(nx, dx))), nd[2 * h], nd[2 * h + 1]);
+        }
+        uint32_t m = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) m |= out_of_reach(far[q], lim, dd[q], vd[q], nd[q]) ? 0u : 1u << q;
+        word |= m << j;
+    }
+    return word;
 }
 
 struct ShadeArgs {
@@ -640,50 +697,59 @@ struct ShadeArgs {
 };
 
 // Evaluates the ring's pairs [at, at + n) and adds their terms to the texels'
-// sums, each texel's in the ring's order: pairs of one texel take turns.
-__device__ __forceinline__ void evaluate_pairs(const ShadeArgs& A, ShadeWarp& w, uint32_t at, uint32_t n, uint32_t lane)
+// sums (lane i: texel i's), each texel's in the ring's order.
+__device__ __forceinline__ void evaluate_pairs(const ShadeArgs& A, ShadeWarp& w, uint32_t at, uint32_t n, uint32_t lane,
+                                               float lo[3])
 {
+    w.pairs[lane] = 0;
     __syncwarp();
-    const uint32_t t = lane < n ? w.texel[(at + lane) & 63u] : 32u + lane;
-    const uint32_t earlier = __match_any_sync(cfk::kFull, t) & ((1u << lane) - 1u);
-    float term[3] = {0.0f, 0.0f, 0.0f};
-    if (lane < n) radiance(&A.lights[w.light[(at + lane) & 63u]], w, t, A.pc, term);
-    const uint32_t turn = __popc(earlier), turns = __reduce_max_sync(cfk::kFull, turn);
-    for (uint32_t k = 0; k <= turns; ++k) {
-        if (turn == k && lane < n) {
+    const uint32_t t = lane < n ? w.texel[(at + lane) & 63u] : 32u;
+    const uint32_t same = __match_any_sync(cfk::kFull, t);
+    if (lane < n) {
+        float term[3];
+        radiance(&A.lights[w.light[(at + lane) & 63u]], w, t, A.pc, term);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) w.lo[c][t] = cf_fadd(w.lo[c][t], term[c]);
-        }
-        __syncwarp();
+        for (int c = 0; c < 3; ++c) w.term[c][lane] = term[c];
+        w.pairs[t] = same;
     }
+    __syncwarp();
+    for (uint32_t m = w.pairs[lane]; m; m &= m - 1) {
+        const uint32_t k = __ffs(m) - 1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) lo[c] = cf_fadd(lo[c], w.term[c][k]);
+    }
+    __syncwarp();
 }
 
-// One CTA per tile of texels.  Bound by issue: about 450 instructions a light
-// evaluated, with some twenty IEEE divisions and square roots.  Most listed
-// lights add nothing (of 20 listed on surfaces 3 reach the texel), so each is
-// tested first (out_of_reach, about 35 instructions, from a table in shared
-// memory where the set fits it) and the pairs that may add something are
-// gathered per warp and evaluated 32 at a time, so that no lane idles while
-// others evaluate.  A 1920x1080 G-buffer of surfaces, 20 listed lights a texel:
-// every light evaluated 683 us, with the test 227 us (3600 instructions per 32
-// texels at 3.3 per cycle: 60 % of them in 3.7 evaluations).
+// One CTA per tile of texels.  Bound by issue (80% of the slots on surfaces):
+// some 600 instructions per 32 lights evaluated, with eighteen IEEE divisions
+// and two square roots.  Most listed lights add nothing (of 20 listed on
+// surfaces 3 reach the texel), so each is tested first: the lanes of a warp
+// fetch the entries of each cluster that its texels lie in, 32 at a time, and
+// each of the cluster's texels tests them four at a time (21 instructions an
+// entry), or, where the cluster has few of the texels, the lanes test their
+// entries against one texel after another.  The pairs that may add something
+// are gathered per warp and evaluated 32 at a time, so that no lane idles while
+// others evaluate.  1920x1080, 1024 lights, surfaces with 20 listed lights a
+// texel: every light evaluated 776 us, tested one by one from each texel's own
+// list 228 us, so 161 us (2400 instructions per 32 texels, two thirds of them in
+// 3.7 evaluations); every texel at its own depth 1113 / 139 / 125 us.
+// (Grids whose lists are short and whose texels are scattered over many of
+// them gain less: 27x4x55, 4 lights a list, 202 / 60 / 75 us.)
+constexpr uint32_t kFewTexels = 2;  // entries per texel from which a texel's turn is cheaper than four entries' test
 template <uint32_t kSide, uint32_t kThreads>
 __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__ ShadeArgs A)
 {
     constexpr uint32_t kPixels = kSide * kSide, kUnits = kPixels / 32;
-    __shared__ __align__(16) float4 table[kTableLights];
     __shared__ uint16_t order[kPixels];
     __shared__ TileSort sort;
     __shared__ TileAxes<kSide> axes;
-    __shared__ ShadeWarp warps[kThreads / 32];
+    __shared__ __align__(16) ShadeWarp warps[kThreads / 32];
     const uint32_t lane = threadIdx.x & 31, lt_mask = (1u << lane) - 1u;
     ShadeWarp& w = warps[threadIdx.x >> 5];
     const Tile<kSide> tile(A.im);
-    const bool whole = A.light_count <= kTableLights;
-    if (whole)
-        for (uint32_t i = threadIdx.x; i < A.light_count; i += kThreads) table[i] = reach_entry(&A.lights[i]);
     fill_axes(A.u, A.im, tile, axes);
-    sort_tile<kSide, kThreads>(A.u, A.im, tile, sort, order, [&](uint32_t p) { return __ldg(&A.gbuf[p].position[3]); });
+    sort_tile<true, kSide, kThreads>(A.u, A.im, tile, axes, sort, order, [&](uint32_t p) { return __ldg(&A.gbuf[p].position[3]); });
     for (uint32_t unit; (unit = next_unit(sort, lane)) < kUnits;) {
         const uint32_t i = order[unit * 32 + lane];
         const bool valid = i != kNoPixel;
@@ -712,12 +778,13 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         w.f[kNx][lane] = N.x, w.f[kNy][lane] = N.y, w.f[kNz][lane] = N.z;
         w.f[kVx][lane] = V.x, w.f[kVy][lane] = V.y, w.f[kVz][lane] = V.z;
         bool colours = true;
+        float lo[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const float f0 = cf_fadd(cf_fmul(A.pc.baseReflectivity, mi), cf_fmul(al[c], metallic));
             w.f[kAx + c][lane] = al[c];
             w.f[kFx + c][lane] = f0;
-            w.lo[c][lane] = cf_fmul(al[c], A.pc.albedoMultipler);
+            lo[c] = cf_fmul(al[c], A.pc.albedoMultipler);
             colours = colours && fabsf(al[c]) <= kMostTexel && fabsf(f0) <= kMostTexel;
         }
         w.f[kA2][lane] = a2;
@@ -745,41 +812,72 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
                 cnt = cell.count;
             }
         }
+        __syncwarp();
         bool lit = false;  // a light of the list is one of the set
         uint32_t put = 0, done = 0;
-        const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
-        for (uint32_t j = 0; j < longest; ++j) {
-            bool need = false;
-            uint32_t li = 0;
-            if (j < cnt) {
-                li = __ldg(&A.indices[off + j]);
-                if (li >= A.light_count) {
-                    alpha = 0.0f;
-                } else {
-                    lit = true;
-                    need = !(tame && out_of_reach(whole ? table[li] : reach_entry(&A.lights[li]), A.lim, P, V, N));
+        // The lists of the clusters that the warp's texels lie in, one after
+        // another: each lane fetches an entry, each texel of the cluster tests 32.
+        for (uint32_t todo = __ballot_sync(cfk::kFull, cnt != 0); todo;) {
+            const uint32_t leader = __ffs(todo) - 1;
+            const uint32_t list_c = __shfl_sync(cfk::kFull, c, leader), list = __shfl_sync(cfk::kFull, off, leader),
+                           n = __shfl_sync(cfk::kFull, cnt, leader);
+            const bool mine = cnt != 0 && c == list_c;
+            const uint32_t texels = __ballot_sync(cfk::kFull, mine), n_texels = __popc(texels);
+            todo &= ~texels;
+            uint32_t li = lane < n ? __ldg(&A.indices[list + lane]) : 0u;
+            for (uint32_t j = 0;; j += 32) {
+                const uint32_t here = li;
+                const bool has = lane < n - j, more = n - j > 32, light = has && here < A.light_count;
+                if (more && lane < n - j - 32) li = __ldg(&A.indices[list + j + 32 + lane]);  // for the next round
+                const float4 e = light ? reach_entry(&A.lights[here]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                const uint32_t lights = __ballot_sync(cfk::kFull, light);
+                if (mine) {
+                    lit = lit || lights;
+                    if (lights != (n - j < 32 ? (1u << (n - j)) - 1u : ~0u)) alpha = 0.0f;  // an entry that is no light
                 }
-            }
-            const uint32_t m = __ballot_sync(cfk::kFull, need);
-            if (!m) continue;
-            if (need) {
-                const uint32_t at = (put + __popc(m & lt_mask)) & 63u;
-                w.light[at] = li;
-                w.texel[at] = lane;
-            }
-            put += __popc(m);
-            if (put - done >= 32) {
-                evaluate_pairs(A, w, done, 32, lane);
-                done += 32;
+                uint32_t need = 0;
+                if (kFewTexels * n_texels < min(32u, n - j)) {
+                    for (uint32_t m = texels; m; m &= m - 1) {
+                        const uint32_t t = __ffs(m) - 1;
+                        const V3 d = v3_sub(V3{e.x, e.y, e.z}, V3{w.f[kPx][t], w.f[kPy][t], w.f[kPz][t]});
+                        const float vd = v3_dot(V3{w.f[kVx][t], w.f[kVy][t], w.f[kVz][t]}, d);
+                        const float nd = v3_dot(V3{w.f[kNx][t], w.f[kNy][t], w.f[kNz][t]}, d);
+                        const uint32_t reach = __ballot_sync(cfk::kFull, !out_of_reach(e.w, A.lim, v3_dot(d, d), vd, nd));
+                        if (lane == t) need = (tame ? reach : ~0u) & lights;
+                    }
+                } else {
+                    w.x[lane] = e.x;
+                    w.y[lane] = e.y;
+                    w.z[lane] = e.z;
+                    w.e[lane] = e.w;
+                    __syncwarp();
+                    if (mine) need = (tame ? within_reach(w, min(32u, n - j), A.lim, P, V, N) : ~0u) & lights;
+                }
+                for (uint32_t any = __reduce_or_sync(cfk::kFull, need); any; any &= any - 1) {
+                    const uint32_t q = __ffs(any) - 1, index = __shfl_sync(cfk::kFull, here, q);
+                    const bool pair = (need >> q) & 1u;
+                    const uint32_t m = __ballot_sync(cfk::kFull, pair);
+                    if (pair) {
+                        const uint32_t at = (put + __popc(m & lt_mask)) & 63u;
+                        w.light[at] = index;
+                        w.texel[at] = lane;
+                    }
+                    put += __popc(m);
+                    if (put - done >= 32) {
+                        evaluate_pairs(A, w, done, 32, lane, lo);
+                        done += 32;
+                    }
+                }
+                __syncwarp();  // the next entries take these ones' place
+                if (!more) break;
             }
         }
-        if (put > done) evaluate_pairs(A, w, done, put - done, lane);
+        if (put > done) evaluate_pairs(A, w, done, put - done, lane, lo);
         __syncwarp();
         if (valid) {
             // the lights out of reach added +0, which turns a -0 sum into +0
-            float lo[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) lo[k] = lit ? cf_fadd(w.lo[k][lane], 0.0f) : w.lo[k][lane];
+            for (int k = 0; k < 3; ++k) lo[k] = lit ? cf_fadd(lo[k], 0.0f) : lo[k];
             A.out[pix] = make_float4(lo[0], lo[1], lo[2], alpha);
         }
         __syncwarp();
