@@ -17,9 +17,9 @@
 // lists: with every pixel at its own depth, unsorted warps had 5 to 10 of 32
 // lanes active.  A sorted warp's fragments also lie in a small box, which few
 // lights of the whole set reach.  1920x1080, 1024 lights, every pixel at its own
-// depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 55 us,
-// shading 1108 -> 150 us; 480x270 with 3000 lights and the all-lights check
-// 812 -> 52 us.
+// depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 47 us,
+// shading 1113 -> 121 us; 480x270 with 3000 lights and the all-lights check
+// 812 -> 48 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -321,8 +321,11 @@ __device__ __forceinline__ uint32_t containing(const ListWarp& w, uint32_t n, co
 // 32 of them, or, where the cluster has few of the warp's pixels, the lanes
 // test their entries against one pixel after another.
 constexpr uint32_t kFewPixels = 3;  // entries per pixel from which a pixel's turn is cheaper than four entries' test
+// Where all lists of a warp's pixels are this short, each pixel walks its own (in
+// the launches of many tiles; 1920x1080, scattered: 49.5 -> 46.9 us).
+constexpr uint32_t kShortLookup = 4;
 constexpr uint32_t kBoxList = 8;    // a list up to this long is not worth a box
-template <bool kCheck>
+template <bool kCheck, bool kOwn>
 __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table, bool whole, ListWarp& w, uint32_t lane,
                                         bool valid, float xf, float yf, float z, const float frag[3], CfFragmentSample& s)
 {
@@ -351,7 +354,22 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
         s.cluster = 0xFFFFFFFFu;
         s.flags |= CF_FRAGMENT_OUTSIDE_GRID;
     }
-    for (uint32_t todo = __ballot_sync(cfk::kFull, cnt != 0); todo;) {
+    const bool own = kOwn && __reduce_max_sync(cfk::kFull, cnt) <= kShortLookup;
+    if (own) {
+        uint32_t li[kShortLookup];
+#pragma unroll
+        for (uint32_t e = 0; e < kShortLookup; ++e) li[e] = e < cnt ? __ldg(&A.indices[off + e]) : 0u;
+#pragma unroll
+        for (uint32_t e = 0; e < kShortLookup; ++e) {
+            if (e < cnt && li[e] >= A.light_count) s.flags |= CF_FRAGMENT_BAD_CELL;
+            if (e < cnt && li[e] < A.light_count) {
+                float p[3], r2;
+                light_view(u.cameraView, &A.lights[li[e]], p, &r2);
+                s.covering += contains(frag, p, r2) ? 1u : 0u;
+            }
+        }
+    }
+    for (uint32_t todo = own ? 0u : __ballot_sync(cfk::kFull, cnt != 0); todo;) {
         const uint32_t leader = __ffs(todo) - 1;
         const uint32_t list_c = __shfl_sync(cfk::kFull, c, leader), list = __shfl_sync(cfk::kFull, off, leader),
                        n = __shfl_sync(cfk::kFull, cnt, leader);
@@ -512,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, 5 * 256 / kThreads) lookup_kernel(co
                     continue;
                 }
             }
-            look_up<kCheck>(A, table, whole, lists[threadIdx.x >> 5], lane, valid, xf, yf, z, frag, s);
+            look_up<kCheck, !kCheck && kSide == 32 && kThreads <= 256>(A, table, whole, lists[threadIdx.x >> 5], lane, valid, xf, yf, z, frag, s);
             if (!valid) continue;
             CfFragmentSample* out = &A.out[y * A.im.width + x];
             if (A.out_aligned) {
@@ -732,10 +750,13 @@ __device__ __forceinline__ void evaluate_pairs(const ShadeArgs& A, ShadeWarp& w,
 // are gathered per warp and evaluated 32 at a time, so that no lane idles while
 // others evaluate.  1920x1080, 1024 lights, surfaces with 20 listed lights a
 // texel: every light evaluated 776 us, tested one by one from each texel's own
-// list 228 us, so 161 us (2400 instructions per 32 texels, two thirds of them in
-// 3.7 evaluations); every texel at its own depth 1113 / 139 / 125 us.
-// (Grids whose lists are short and whose texels are scattered over many of
-// them gain less: 27x4x55, 4 lights a list, 202 / 60 / 75 us.)
+// list 228 us, so 164 us (2400 instructions per 32 texels, two thirds of them in
+// 3.7 evaluations); every texel at its own depth 1113 / 139 / 121 us.
+// Lists up to kShortList each texel walks itself, as the lists of many clusters
+// one after another cost more than they save: 27x4x55, four lights a list,
+// scattered depths 62 us against 76; with a limit of 4 / 8 / 16 the surfaces above take
+// 164 / 166 / 172 us.
+constexpr uint32_t kShortList = 6;
 constexpr uint32_t kFewTexels = 2;  // entries per texel from which a texel's turn is cheaper than four entries' test
 template <uint32_t kSide, uint32_t kThreads>
 __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__ ShadeArgs A)
@@ -815,64 +836,104 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         __syncwarp();
         bool lit = false;  // a light of the list is one of the set
         uint32_t put = 0, done = 0;
-        // The lists of the clusters that the warp's texels lie in, one after
-        // another: each lane fetches an entry, each texel of the cluster tests 32.
-        for (uint32_t todo = __ballot_sync(cfk::kFull, cnt != 0); todo;) {
-            const uint32_t leader = __ffs(todo) - 1;
-            const uint32_t list_c = __shfl_sync(cfk::kFull, c, leader), list = __shfl_sync(cfk::kFull, off, leader),
-                           n = __shfl_sync(cfk::kFull, cnt, leader);
-            const bool mine = cnt != 0 && c == list_c;
-            const uint32_t texels = __ballot_sync(cfk::kFull, mine), n_texels = __popc(texels);
-            todo &= ~texels;
-            uint32_t li = lane < n ? __ldg(&A.indices[list + lane]) : 0u;
-            for (uint32_t j = 0;; j += 32) {
-                const uint32_t here = li;
-                const bool has = lane < n - j, more = n - j > 32, light = has && here < A.light_count;
-                if (more && lane < n - j - 32) li = __ldg(&A.indices[list + j + 32 + lane]);  // for the next round
-                const float4 e = light ? reach_entry(&A.lights[here]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                const uint32_t lights = __ballot_sync(cfk::kFull, light);
-                if (mine) {
-                    lit = lit || lights;
-                    if (lights != (n - j < 32 ? (1u << (n - j)) - 1u : ~0u)) alpha = 0.0f;  // an entry that is no light
-                }
-                uint32_t need = 0;
-                if (kFewTexels * n_texels < min(32u, n - j)) {
-                    for (uint32_t m = texels; m; m &= m - 1) {
-                        const uint32_t t = __ffs(m) - 1;
-                        const V3 d = v3_sub(V3{e.x, e.y, e.z}, V3{w.f[kPx][t], w.f[kPy][t], w.f[kPz][t]});
-                        const float vd = v3_dot(V3{w.f[kVx][t], w.f[kVy][t], w.f[kVz][t]}, d);
-                        const float nd = v3_dot(V3{w.f[kNx][t], w.f[kNy][t], w.f[kNz][t]}, d);
-                        const uint32_t reach = __ballot_sync(cfk::kFull, !out_of_reach(e.w, A.lim, v3_dot(d, d), vd, nd));
-                        if (lane == t) need = (tame ? reach : ~0u) & lights;
+        // Rounds of up to 32 entries' tests.  Where all lists of the warp's texels
+        // are short, a round is one entry of each texel's own; else 32 entries of
+        // the list of one cluster after another, an entry fetched by each lane and
+        // tested by each texel of the cluster.  (One loop over all rounds, so that
+        // the evaluation is there once: it is half of the kernel's instructions.)
+        const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
+        const bool own = longest <= kShortList;
+        uint32_t todo = own ? 0u : __ballot_sync(cfk::kFull, cnt != 0), texels = 0, n_texels = 0, list = 0, left = 0, li = 0;
+        uint32_t step = 0;
+        bool mine = false;
+        for (bool more = true; more;) {
+            uint32_t any = 0, need = 0, here = 0;  // need: bit q: entry q may add something to the lane's texel
+            if (own) {
+                more = step < longest;
+                if (more) {
+                    const bool has = step < cnt;
+                    here = has ? __ldg(&A.indices[off + step]) : 0u;
+                    const bool light = has && here < A.light_count;
+                    if (has && !light) alpha = 0.0f;  // an entry that is no light
+                    if (light) {
+                        lit = true;
+                        const float4 e = reach_entry(&A.lights[here]);
+                        const V3 d = v3_sub(V3{e.x, e.y, e.z}, P);
+                        need = tame && out_of_reach(e.w, A.lim, v3_dot(d, d), v3_dot(V, d), v3_dot(N, d)) ? 0u : 1u;
                     }
-                } else {
-                    w.x[lane] = e.x;
-                    w.y[lane] = e.y;
-                    w.z[lane] = e.z;
-                    w.e[lane] = e.w;
-                    __syncwarp();
-                    if (mine) need = (tame ? within_reach(w, min(32u, n - j), A.lim, P, V, N) : ~0u) & lights;
+                    any = __any_sync(cfk::kFull, need) ? 1u : 0u;
+                    ++step;
                 }
-                for (uint32_t any = __reduce_or_sync(cfk::kFull, need); any; any &= any - 1) {
-                    const uint32_t q = __ffs(any) - 1, index = __shfl_sync(cfk::kFull, here, q);
+            } else {
+                if (left == 0) {  // the next list
+                    more = todo != 0;
+                    if (more) {
+                        const uint32_t leader = __ffs(todo) - 1;
+                        const uint32_t list_c = __shfl_sync(cfk::kFull, c, leader);
+                        list = __shfl_sync(cfk::kFull, off, leader);
+                        left = __shfl_sync(cfk::kFull, cnt, leader);
+                        mine = cnt != 0 && c == list_c;
+                        texels = __ballot_sync(cfk::kFull, mine);
+                        n_texels = __popc(texels);
+                        todo &= ~texels;
+                        li = lane < left ? __ldg(&A.indices[list + lane]) : 0u;
+                    }
+                }
+                if (more) {
+                    const uint32_t n = min(32u, left);
+                    here = li;
+                    const bool light = lane < n && here < A.light_count;
+                    left -= n;
+                    list += n;
+                    if (lane < left) li = __ldg(&A.indices[list + lane]);  // for the next round
+                    const float4 e = light ? reach_entry(&A.lights[here]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    const uint32_t lights = __ballot_sync(cfk::kFull, light);
+                    if (mine) {
+                        lit = lit || lights;
+                        if (lights != (n < 32 ? (1u << n) - 1u : ~0u)) alpha = 0.0f;  // an entry that is no light
+                    }
+                    if (kFewTexels * n_texels < n) {
+                        for (uint32_t m = texels; m; m &= m - 1) {
+                            const uint32_t t = __ffs(m) - 1;
+                            const V3 d = v3_sub(V3{e.x, e.y, e.z}, V3{w.f[kPx][t], w.f[kPy][t], w.f[kPz][t]});
+                            const float vd = v3_dot(V3{w.f[kVx][t], w.f[kVy][t], w.f[kVz][t]}, d);
+                            const float nd = v3_dot(V3{w.f[kNx][t], w.f[kNy][t], w.f[kNz][t]}, d);
+                            const uint32_t reach = __ballot_sync(cfk::kFull, !out_of_reach(e.w, A.lim, v3_dot(d, d), vd, nd));
+                            if (lane == t) need = (tame ? reach : ~0u) & lights;
+                        }
+                    } else {
+                        w.x[lane] = e.x;
+                        w.y[lane] = e.y;
+                        w.z[lane] = e.z;
+                        w.e[lane] = e.w;
+                        __syncwarp();
+                        if (mine) need = (tame ? within_reach(w, n, A.lim, P, V, N) : ~0u) & lights;
+                        __syncwarp();  // the next entries take these ones' place
+                    }
+                    any = __reduce_or_sync(cfk::kFull, need);
+                }
+            }
+            for (;;) {
+                if (any) {
+                    const uint32_t q = __ffs(any) - 1, from = __shfl_sync(cfk::kFull, here, q);
+                    any &= any - 1;
                     const bool pair = (need >> q) & 1u;
                     const uint32_t m = __ballot_sync(cfk::kFull, pair);
                     if (pair) {
                         const uint32_t at = (put + __popc(m & lt_mask)) & 63u;
-                        w.light[at] = index;
+                        w.light[at] = own ? here : from;
                         w.texel[at] = lane;
                     }
                     put += __popc(m);
-                    if (put - done >= 32) {
-                        evaluate_pairs(A, w, done, 32, lane, lo);
-                        done += 32;
-                    }
                 }
-                __syncwarp();  // the next entries take these ones' place
-                if (!more) break;
+                if (put - done >= 32 || (!more && put != done)) {
+                    const uint32_t n = min(32u, put - done);
+                    evaluate_pairs(A, w, done, n, lane, lo);
+                    done += n;
+                }
+                if (!any) break;
             }
         }
-        if (put > done) evaluate_pairs(A, w, done, put - done, lane, lo);
         __syncwarp();
         if (valid) {
             // the lights out of reach added +0, which turns a -0 sum into +0

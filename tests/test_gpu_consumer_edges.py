@@ -159,6 +159,27 @@ def test_shading_light_tables(gpu, oracle, n_lights):
 ODD = np.array([0.0, -0.0, 1e-30, -1e-3, 1.0, 1.8, 1.9, 2.0, 1e7, 1e30, np.inf, -np.inf, np.nan], np.float32)
 
 
+@pytest.mark.parametrize("depths", ["scattered", "one"])
+@pytest.mark.parametrize("r", [(0.2, 1.5), (0.2, 9.0)])
+def test_shading_lists_read_by_a_warp(gpu, oracle, r, depths):
+    """Lists that each texel walks itself and lists, of up to five times a
+    warp's width, that a warp reads for all its texels of a cluster; clusters
+    with a few of its texels and with all; entries that are no light."""
+    v, rng = view_of((96, 64), 1500, grid=(3, 2, 16), r=r)
+    _, cells, idx = run_pipeline(gpu, v)
+    if r[1] > 5:
+        assert cells[:, 1].max() > 96
+    cells, idx = cells.copy(), idx.copy()
+    if r[1] < 5:
+        cells[:, 1] = np.minimum(cells[:, 1], rng.integers(0, 8, cells.shape[0]))  # around what counts as short
+    idx[rng.integers(0, idx.size, 40)] = rng.choice([1500, 0xFFFFFFFF], 40)
+    g = scenes.gbuffer(rng, v.ubo)
+    if depths == "one":
+        g[..., 3] = np.float32((0.1 * 300.0 / 20.0 - 300.0) / (0.1 - 300.0))
+    cam = scenes.camera_position(v.ubo)
+    assert same_shading(shade(v, g, cells, idx, PC, cam), oracle.shade_clusters(v.ubo, cam, PC, g, cells, idx, v.lights))
+
+
 @pytest.mark.parametrize("falloff", [0.1, 0.0, 2.0, -1.5, 60.0, 120.0, 121.0, np.inf, np.nan])
 @pytest.mark.parametrize("intensity", [1.75, 0.0, np.inf])
 def test_shading_odd_texels_and_lights(gpu, oracle, falloff, intensity):
