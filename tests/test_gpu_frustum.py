@@ -61,3 +61,30 @@ def test_frustum_culling_matches_the_reference_golden(gpu, golden_consumers):
         frustum_cull(f, d_boxes, d_cmds)
         got = d_cmds.cpu().numpy().view(np.uint32)[:, 1]
         assert np.array_equal(got, golden_consumers["frustum/instance%d" % k].astype(np.uint32)), k
+
+
+@pytest.mark.parametrize("offset", [0, 4])
+@pytest.mark.parametrize("n", [1, 255, 257, 4099])
+def test_frustum_corners_and_alignment(gpu, oracle, n, offset):
+    """Box arrays at a 32- and at a 16-byte boundary; frusta whose corners are
+    finite, hold a NaN or an infinity on an axis, or lie on the boxes' sides."""
+    import torch
+    from hellovulkan_gb300.consumer import frustum_cull
+    rng = np.random.default_rng(n)
+    boxes = scenes.random_boxes(rng, n)
+    boxes[::7, 0] = np.nan
+    boxes[::11, 6] = -np.inf
+    d = torch.zeros(8 * n + 8, device="cuda")
+    d[offset:offset + 8 * n] = torch.from_numpy(boxes).cuda().reshape(-1)
+    d_boxes = d[offset:offset + 8 * n].reshape(n, 8)
+    for axis, value in ((None, 0.0), (0, np.nan), (1, np.inf), (2, -np.inf), (2, float(boxes[n // 2, 6]))):
+        f = frustum_ubo(1.0, 1.5, 0.1, 300.0, scenes.random_camera(rng))
+        if axis is not None:
+            for corner in ((3,), range(8))[value == value and abs(value) < 1e30]:
+                f.corners[corner][axis] = value
+        d_cmds = torch.full((n, 4), 9, dtype=torch.int32, device="cuda")
+        visible = torch.zeros(1, dtype=torch.int32, device="cuda")
+        frustum_cull(f, d_boxes, d_cmds, visible)
+        want = oracle.frustum_cull(f, boxes)
+        assert np.array_equal(d_cmds.cpu().numpy()[:, 1], want.astype(np.int32))
+        assert int(visible.item()) == int(want.sum())
