@@ -1594,6 +1594,8 @@ __global__ void __launch_bounds__(256) readback_kernel(const uint32_t* __restric
                                                        uint32_t* __restrict__ h_cells, uint32_t* __restrict__ h_indices,
                                                        uint32_t* __restrict__ h_total, bool vec_cells, bool vec_indices)
 {
+    grid_dependency_wait();
+    launch_dependents();
     const uint32_t total = *d_total;
     const uint64_t tid = (uint64_t)blockIdx.x * 256 + threadIdx.x, stride = (uint64_t)gridDim.x * 256;
     if (tid == 0) *h_total = total;
@@ -1610,10 +1612,9 @@ cudaError_t launch_readback(const CfLightCell* cells, uint32_t clusters, const u
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const uint64_t words = std::max<uint64_t>(2ull * clusters, h_indices ? capacity : 0ull);
     const uint32_t blocks = (uint32_t)std::min<uint64_t>(std::max<uint64_t>((words + 1023) / 1024, 1ull), 1216ull);
-    readback_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(cells), 2u * clusters, indices,
-                                                d_total, capacity, reinterpret_cast<uint32_t*>(h_cells), h_indices,
-                                                h_total, al16(cells) && al16(h_cells), al16(indices) && al16(h_indices));
-    return cudaGetLastError();
+    return launch_kernel(true, readback_kernel, dim3(blocks), dim3(256), 0, stream, reinterpret_cast<const uint32_t*>(cells),
+                         2u * clusters, indices, d_total, capacity, reinterpret_cast<uint32_t*>(h_cells), h_indices, h_total,
+                         al16(cells) && al16(h_cells), al16(indices) && al16(h_indices));
 }
 
 // ---------------------------------------------------------------------------

@@ -25,6 +25,7 @@
 #include <cmath>
 
 #include "cf_device.cuh"
+#include "cf_launch.cuh"
 #include "cf_pinned_math.h"
 #include "cf_runtime_internal.h"
 #include "cfcull.h"
@@ -477,6 +478,8 @@ __global__ void __launch_bounds__(kThreads, 5 * 256 / kThreads) lookup_kernel(co
     const CfClusterForwardUBO& u = A.u;
     const Tile<kSide> tile(A.im);
     const bool whole = kCheck && A.light_count <= kTableLights;  // the set fits the table
+    cfk::grid_dependency_wait();
+    cfk::launch_dependents();
     if (whole) fill_table(A, table, 0, A.light_count);
     fill_axes(u, A.im, tile, axes);
     sort_tile<!kCheck, kSide, kThreads>(u, A.im, tile, axes, sort, order, [&](uint32_t p) { return __ldg(&A.depth[p]); });
@@ -769,6 +772,8 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
     const uint32_t lane = threadIdx.x & 31, lt_mask = (1u << lane) - 1u;
     ShadeWarp& w = warps[threadIdx.x >> 5];
     const Tile<kSide> tile(A.im);
+    cfk::grid_dependency_wait();
+    cfk::launch_dependents();
     fill_axes(A.u, A.im, tile, axes);
     sort_tile<true, kSide, kThreads>(A.u, A.im, tile, axes, sort, order, [&](uint32_t p) { return __ldg(&A.gbuf[p].position[3]); });
     for (uint32_t unit; (unit = next_unit(sort, lane)) < kUnits;) {
@@ -985,14 +990,21 @@ ReachLimits reach_limits(const CfPBRPushConstant& pc)
     return {std::ldexp(1.0f, -2 * k), std::ldexp(1.0f, 2 * k)};
 }
 
+// A tile per CTA; the launch overlaps with the end of the stream's previous one.
+template <typename Args>
+cudaError_t launch_tiles(void (*kernel)(Args), const Args& A, uint32_t side, uint32_t threads, cudaStream_t stream)
+{
+    return cfk::launch_kernel(true, kernel, dim3(image_blocks(A.im, side)), dim3(threads), 0, stream, A);
+}
+
 template <bool kCheck>
-void launch_lookup(const LookupArgs& A, cudaStream_t stream)
+cudaError_t launch_lookup(const LookupArgs& A, cudaStream_t stream)
 {
     const uint64_t n = A.im.n_pixels;
-    if (n >= kLargePixels) lookup_kernel<32, 256, kCheck><<<image_blocks(A.im, 32), 256, 0, stream>>>(A);
-    else if (n >= kMiddlePixels) lookup_kernel<32, 512, kCheck><<<image_blocks(A.im, 32), 512, 0, stream>>>(A);
-    else if (n >= kSmallPixels) lookup_kernel<32, 1024, kCheck><<<image_blocks(A.im, 32), 1024, 0, stream>>>(A);
-    else lookup_kernel<16, 256, kCheck><<<image_blocks(A.im, 16), 256, 0, stream>>>(A);
+    if (n >= kLargePixels) return launch_tiles(lookup_kernel<32, 256, kCheck>, A, 32, 256, stream);
+    if (n >= kMiddlePixels) return launch_tiles(lookup_kernel<32, 512, kCheck>, A, 32, 512, stream);
+    if (n >= kSmallPixels) return launch_tiles(lookup_kernel<32, 1024, kCheck>, A, 32, 1024, stream);
+    return launch_tiles(lookup_kernel<16, 256, kCheck>, A, 16, 256, stream);
 }
 
 }  // namespace
@@ -1033,9 +1045,8 @@ extern "C" int cf_shade_clusters(const CfClusterForwardUBO* ubo, const float cam
     A.lights = d_lights;
     A.out = reinterpret_cast<float4*>(d_out);
     A.light_count = light_count;
-    if (large) shade_kernel<32, 256><<<image_blocks(A.im, 32), 256, 0, (cudaStream_t)stream>>>(A);
-    else shade_kernel<16, 256><<<image_blocks(A.im, 16), 256, 0, (cudaStream_t)stream>>>(A);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = large ? launch_tiles(shade_kernel<32, 256>, A, 32, 256, (cudaStream_t)stream)
+                                : launch_tiles(shade_kernel<16, 256>, A, 16, 256, (cudaStream_t)stream);
     return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "clustered shading launch");
 }
 
@@ -1071,8 +1082,7 @@ extern "C" int cf_lookup_clusters(const CfClusterForwardUBO* ubo, const float* d
     A.light_count = light_count;
     A.cap = cap ? cap : 0xFFFFFFFFu;
     A.out_aligned = (reinterpret_cast<uintptr_t>(d_out) & 31) == 0;
-    if (check_all_lights) launch_lookup<true>(A, (cudaStream_t)stream);
-    else launch_lookup<false>(A, (cudaStream_t)stream);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = check_all_lights ? launch_lookup<true>(A, (cudaStream_t)stream)
+                                           : launch_lookup<false>(A, (cudaStream_t)stream);
     return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "cluster lookup launch");
 }
