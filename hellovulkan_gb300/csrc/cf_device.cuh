@@ -134,7 +134,8 @@ __device__ __forceinline__ bool hit_exact(const float4& L, const float* mn, cons
 
 // ---- packed float pairs ------------------------------------------------------
 // sub/mul/add.rn.f32x2: two IEEE binary32 round-to-nearest operations per
-// instruction, each the same bits as the scalar one (no contraction).
+// instruction, each the same bits as the scalar one; but a packed product that
+// is only used in a packed sum is contracted with it (see hit_pair_twice_rounded).
 typedef unsigned long long f2;  // two floats in one 64-bit register pair: (lo, hi)
 
 __device__ __forceinline__ f2 f2_pack(float lo, float hi)

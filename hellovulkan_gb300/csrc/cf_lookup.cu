@@ -19,7 +19,7 @@
 // lights of the whole set reach.  1920x1080, 1024 lights, every pixel at its own
 // depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 47 us,
 // shading 1113 -> 121 us; 480x270 with 3000 lights and the all-lights check
-// 812 -> 48 us.
+// 812 -> 40 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -260,15 +260,26 @@ __device__ __forceinline__ void fragment_view(const CfClusterForwardUBO& u, floa
 __device__ __forceinline__ uint32_t count_containing(const float4* table, uint32_t n, const float frag[3], const float lo[3],
                                                      const float hi[3], uint32_t lane)
 {
+    using namespace cfk;
+    const f2 lx = f2_pack(lo[0], lo[0]), ly = f2_pack(lo[1], lo[1]), lz = f2_pack(lo[2], lo[2]), hx = f2_pack(hi[0], hi[0]),
+             hy = f2_pack(hi[1], hi[1]), hz = f2_pack(hi[2], hi[2]);
     uint32_t count = 0;
-    for (uint32_t c = 0; c < n; c += 32) {
-        const bool in = c + lane < n;
-        const float4 L = table[in ? c + lane : c];
-        for (uint32_t m = __ballot_sync(cfk::kFull, in && cfk::hit_fast(L, lo, hi)); m; m &= m - 1) {
-            const float4 q = table[c + __ffs(m) - 1];
-            const float p[3] = {q.x, q.y, q.z};
-            count += contains(frag, p, q.w) ? 1u : 0u;
-        }
+    // two lights per lane, in packed operations: a filter of one took a third
+    // more instructions (480x270, 3000 lights: 45.7 -> 40.1 us)
+    for (uint32_t c = 0; c < n; c += 64) {
+        const bool in0 = c + lane < n, in1 = c + 32 + lane < n;
+        const float4 a = table[in0 ? c + lane : c], b = table[in1 ? c + 32 + lane : c];
+        bool reach0, reach1;
+        hit_pair_twice_rounded(f2_pack(a.x, b.x), f2_pack(a.y, b.y), f2_pack(a.z, b.z), a.w, b.w, lx, ly, lz, hx, hy, hz,
+                               reach0, reach1);
+        const uint32_t m0 = __ballot_sync(kFull, in0 && reach0), m1 = __ballot_sync(kFull, in1 && reach1);
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h)
+            for (uint32_t m = h ? m1 : m0; m; m &= m - 1) {
+                const float4 q = table[c + 32 * h + __ffs(m) - 1];
+                const float p[3] = {q.x, q.y, q.z};
+                count += contains(frag, p, q.w) ? 1u : 0u;
+            }
     }
     return count;
 }

@@ -43,7 +43,7 @@ def test_lookup_images(gpu, oracle, res):
         assert same(got, want)
 
 
-@pytest.mark.parametrize("n_lights", [0, 1, 31, 1023, 1024, 1025, 2048, 2500])
+@pytest.mark.parametrize("n_lights", [0, 1, 31, 33, 63, 65, 1023, 1024, 1025, 1088, 2048, 2500])
 def test_lookup_light_tables(gpu, oracle, n_lights):
     v, rng = view_of((160, 96), n_lights)
     if n_lights > 31:
