@@ -804,6 +804,24 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         const V3 P = {pos.x, pos.y, pos.z}, N = {nrm.x, nrm.y, nrm.z};
         const float al[3] = {alb.x, alb.y, alb.z};
         const float metallic = nrm.w, roughness = alb.w;
+        uint32_t c = 0, off = 0, cnt = 0;
+        float lin = 0.0f, alpha = 0.0f;
+        if (valid && fragment_cluster(A.u, xf, yf, pos.w, &c, &lin)) {
+            const CfLightCell cell = A.cells[c];
+            if ((uint64_t)cell.offset + cell.count <= A.index_count) {
+                alpha = 1.0f;
+                off = cell.offset;
+                cnt = cell.count;
+            }
+        }
+        float lo[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) lo[k] = cf_fmul(al[k], A.pc.albedoMultipler);
+        const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
+        if (longest == 0) {  // the sorted texels of unlit clusters: nothing else is asked of them
+            if (valid) A.out[pix] = make_float4(lo[0], lo[1], lo[2], alpha);
+            continue;
+        }
         // Scene.frag:82-115: V, NoV, F0 = mix(baseReflectivity, albedo, metallic), Lo = albedo * albedoMultipler
         const V3 V = v3_normalize(v3_sub(V3{A.cam[0], A.cam[1], A.cam[2]}, P));
         const float NoV = cf_glsl_max(v3_dot(N, V), 0.0f);
@@ -815,13 +833,11 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         w.f[kNx][lane] = N.x, w.f[kNy][lane] = N.y, w.f[kNz][lane] = N.z;
         w.f[kVx][lane] = V.x, w.f[kVy][lane] = V.y, w.f[kVz][lane] = V.z;
         bool colours = true;
-        float lo[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const float f0 = cf_fadd(cf_fmul(A.pc.baseReflectivity, mi), cf_fmul(al[c], metallic));
             w.f[kAx + c][lane] = al[c];
             w.f[kFx + c][lane] = f0;
-            lo[c] = cf_fmul(al[c], A.pc.albedoMultipler);
             colours = colours && fabsf(al[c]) <= kMostTexel && fabsf(f0) <= kMostTexel;
         }
         w.f[kA2][lane] = a2;
@@ -839,16 +855,6 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         const float vv = v3_dot(V, V), nn = v3_dot(N, N);
         const bool tame = colours && vv >= 0.999f && vv <= 1.001f && nn <= 1.0001f && roughness >= 0.0f &&
                           roughness <= 1.8f && fabsf(metallic) <= kMostTexel && a2 * nn + (1.0f - nn * 1.000002f) > 4e-6f;
-        uint32_t c = 0, off = 0, cnt = 0;
-        float lin = 0.0f, alpha = 0.0f;
-        if (valid && fragment_cluster(A.u, xf, yf, pos.w, &c, &lin)) {
-            const CfLightCell cell = A.cells[c];
-            if ((uint64_t)cell.offset + cell.count <= A.index_count) {
-                alpha = 1.0f;
-                off = cell.offset;
-                cnt = cell.count;
-            }
-        }
         __syncwarp();
         bool lit = false;  // a light of the list is one of the set
         uint32_t put = 0, done = 0;
@@ -857,7 +863,6 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         // the list of one cluster after another, an entry fetched by each lane and
         // tested by each texel of the cluster.  (One loop over all rounds, so that
         // the evaluation is there once: it is half of the kernel's instructions.)
-        const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
         const bool own = longest <= kShortList;
         uint32_t todo = own ? 0u : __ballot_sync(cfk::kFull, cnt != 0), texels = 0, n_texels = 0, list = 0, left = 0, li = 0;
         uint32_t step = 0;
@@ -970,7 +975,11 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
 //   960x540, surfaces                                     65.9 / 32.2 / 29.3 / 24.9
 //   480x270, every pixel at its own depth                 43.5 / 25.5 / 25.1 / 36.5
 //   480x270, the all-lights check                          812 / 53.1 / 57.9 / 76.4
-// Shading's smaller images take 16x16: its warps need 3.5 KB of shared memory each.
+// Shading's smaller images take 16x16: its warps need 3.5 KB of shared memory
+// each.  Between four and eight tiles per SM, 512 threads a tile leave the last
+// wave shorter: 940x1000, surfaces 44.0 -> 39.8 and 62.8 -> 53.4 us (scattered
+// depths 83.5 -> 91.7, which gains from warps of few lists); above, 1920x1080
+// takes 163 us with 256, 168 with 512.
 constexpr uint64_t kLargePixels = 152ull * 4 * 1024, kMiddlePixels = 152ull * 1024, kSmallPixels = 152ull * 256;
 
 Image image_of(const CfClusterForwardUBO& u, uint32_t width, uint32_t height, uint32_t side)
@@ -1056,8 +1065,10 @@ extern "C" int cf_shade_clusters(const CfClusterForwardUBO* ubo, const float cam
     A.lights = d_lights;
     A.out = reinterpret_cast<float4*>(d_out);
     A.light_count = light_count;
-    const cudaError_t e = large ? launch_tiles(shade_kernel<32, 256>, A, 32, 256, (cudaStream_t)stream)
-                                : launch_tiles(shade_kernel<16, 256>, A, 16, 256, (cudaStream_t)stream);
+    const cudaStream_t on = (cudaStream_t)stream;
+    const cudaError_t e = n >= 2 * kLargePixels ? launch_tiles(shade_kernel<32, 256>, A, 32, 256, on)
+                          : large               ? launch_tiles(shade_kernel<32, 512>, A, 32, 512, on)
+                                                : launch_tiles(shade_kernel<16, 256>, A, 16, 256, on);
     return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "clustered shading launch");
 }
 

@@ -24,7 +24,7 @@ def view_of(res, n_lights, grid=(5, 4, 12), seed=0, r=(0.5, 6.0)):
                               lights=scenes.uniform_box_lights(rng, n_lights, [-20, -10, -60], [20, 10, -1], *r)), rng
 
 
-RESOLUTIONS = [(1, 1), (7, 300), (300, 7), (15, 16), (16, 16), (33, 31), (97, 64), (1001, 701)]
+RESOLUTIONS = [(1, 1), (7, 300), (300, 7), (15, 16), (16, 16), (33, 31), (97, 64), (1001, 701), (1201, 1051)]
 
 
 @pytest.mark.parametrize("res", RESOLUTIONS)
