@@ -963,8 +963,11 @@ def run_ours(args):
 
     value = ws * tests_per_view * args.steps / (total_ms * 1e-3)
     X, Y, Z = view.grid
+    hit_masks = tuple(cull_cfg_used) == (4, 8, 32, 1, 1)
     if cull_cfg_used[4] == 2:  # the one-launch kernel
         kernels_per_step = 1
+    elif hit_masks:
+        kernels_per_step = 5  # boxes, lists, scan, sums, writing
     else:
         gw = cull_cfg_used[0] * cull_cfg_used[1]
         groups = Z * -(-(X * Y) // gw) if cull_cfg_used[4] else -(-view.clusters // gw)
@@ -983,7 +986,7 @@ def run_ours(args):
     prof = REPO / "profiles" / "dram_bytes_per_launch.json"
     if prof.exists():
         try:
-            traffic = json.loads(prof.read_text()).get(args.workload, {})
+            traffic = {} if hit_masks else json.loads(prof.read_text()).get(args.workload, {})  # of the staged kernels
         except ValueError:
             traffic = {}
     st_x, st_c, st_f = (float(np.mean(stage[:, i])) for i in range(3))
@@ -993,6 +996,8 @@ def run_ours(args):
     auto_cfg = cull_cfg_used
     if auto_cfg[4] == 2:
         cull_kernel_name = "one_launch_kernel (%d clusters per CTA, %d warps)" % tuple(auto_cfg[:2])
+    elif hit_masks:
+        cull_kernel_name = "box_kernel + list_kernel + scan_kernel (hit masks)"
     else:
         cull_kernel_name = ("bin_slices_kernel + cull_pipe_kernel<%d,%d,%d,%d> (binned)" if auto_cfg[4] else
                             "cull_kernel<%d,%d,%d,%d> (brute force)") % tuple(auto_cfg[:4])
@@ -1006,7 +1011,8 @@ def run_ours(args):
     else:
         ach = fin_bytes / (st_f * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": ach, "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
-                "traffic": traffic.get("finalize"), "kernel": "finalize_kernel", "bytes_per_launch": fin_bytes,
+                "traffic": traffic.get("finalize"), "kernel": "sum_kernel + emit_kernel" if hit_masks else "finalize_kernel",
+                "bytes_per_launch": fin_bytes,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)"}
     # the whole step against HBM: the algorithmic bytes of one view (lights
     # read, AABBs read, LightCells and indices written, the UBO) per step
