@@ -1426,23 +1426,24 @@ bool cull_config_supported(const CullConfig& c)
 }
 
 // Where the lines lie (GB300, back-to-back passes, brute force against the
-// hit-mask path, which takes 16 to 20 us whatever the size of a small view:
+// hit-mask path, which takes 17 to 19 us whatever the size of a small view:
 // its five dependent launches are what it costs):
-//   lights   3456 clusters, 2604 lights (9 M tests)   23.9 against 19.5 us
-//            1024 clusters, 2929 lights (3 M)         21.7          19.4
-//            3105 clusters, 2254 lights (7 M)         20.9          20.0
+//   lights   4800 clusters, 2400 lights (12 M tests)  24.3 against 18.8 us
+//            3456 clusters, 2400 lights (8 M)         22.4          18.4
+//            1024 clusters, 2400 lights (2 M)         19.3          18.6
+//            1024 clusters, 2112 lights (2 M)         18.0          18.6
 //            the brute-force kernel's time grows with the lights each warp
 //            streams, so above kMaskMinLights the hit-mask path always wins
-//   tests    27648 clusters, 434 lights (12 M)        19.0          18.1
-//            10752 clusters, 1116 lights (12 M)       20.0          18.4
-//            10752 clusters,  837 lights (9 M)        16.9          18.8
+//   tests    27648 clusters, 600 lights (17 M)        23.6          18.4
+//            10752 clusters, 1000 lights (11 M)       18.6          18.5
+//            27648 clusters, 300 lights (8 M)         16.4          17.5
 // Below both lines, a view whose lights fit one launch's registers (at most
 // kOneLaunchMaxLights) and whose clusters spread over the resident CTAs at
 // most kOneLaunchMaxClustersPerCta each is culled in one launch; the rest
 // brute force.  Grids beyond the hit-mask path's limits (mask_fits) take the
 // staged binned path once it pays: 453 M tests cull five times faster with it
 // than brute force, 16 M about the same.
-constexpr uint32_t kMaskMinLights = 2560;
+constexpr uint32_t kMaskMinLights = 2304;
 constexpr uint64_t kMaskMinTests = 10ull << 20;
 constexpr uint64_t kStagedMinTests = 16ull << 20;
 

@@ -148,3 +148,26 @@ def test_boxes_of_other_shapes(gpu, oracle, grid):
         oc, oi, _ = oracle.cull(v.ubo, given[q], v.lights, v.cap)
         assert np.array_equal(cells, oc) and np.array_equal(idx, oi), q
     b.close()
+
+
+@pytest.mark.parametrize("grid", [(8, 8, 16), (16, 9, 24), (8, 10, 30)])
+@pytest.mark.parametrize("n_lights", [2303, 2304])
+def test_the_line_between_brute_force_and_hit_masks(gpu, oracle, grid, n_lights):
+    """More lights than one launch takes, on both sides of the line: the chosen
+    kernels, and their output."""
+    from hellovulkan_gb300.pipelines import PipelineLightCulling, ResourcesClusterForward, ResourcesLight
+    rng = np.random.default_rng(n_lights)
+    v = scenes.custom_view(grid, 1920, 1080, 0.1, 300.0,
+                           lights=scenes.uniform_box_lights(rng, n_lights, [-30, -15, -60], [30, 15, -5], 1.0, 6.0))
+    rl, rc = ResourcesLight(gpu), ResourcesClusterForward(gpu)
+    rl.add_lights(v.lights)
+    rc.create_buffers(*v.grid, v.cap)
+    cull = PipelineLightCulling(gpu, rl, rc)
+    cull.set_cluster_forward_ubo(v.ubo)
+    if n_lights == 2304:
+        assert cull.tuning() == MASK
+    else:
+        assert cull.tuning()[4] == 0
+    for o in (cull, rc, rl):
+        o.close()
+    assert_matches_oracle(oracle, v, *run_pipeline(gpu, v))
