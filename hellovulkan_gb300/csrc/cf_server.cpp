@@ -1182,7 +1182,10 @@ int cf_server_set_tuning(CfServer* s, uint32_t slice_clusters, int clusters_per_
         return CF_SUCCESS;
     }
     const cfk::CullConfig c{clusters_per_warp, warps, tile, stages, 1};
-    if (!cfk::cull_config_supported(c)) return fail(CF_ERROR_INVALID_ARGUMENT, "unsupported configuration");
+    // a batch of requests runs the staged kernels: there is none for the hit masks
+    if (!cfk::cull_config_supported(c) || cfk::is_mask_config(c))
+        return fail(CF_ERROR_INVALID_ARGUMENT, "no served culling kernel for K=%d warps=%d tile=%d stages=%d",
+                    clusters_per_warp, warps, tile, stages);
     s->tuned[slice_clusters] = c;
     return CF_SUCCESS;
 }

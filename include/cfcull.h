@@ -360,6 +360,9 @@ CFCULL_API int cf_server_release(CfServer* server, uint64_t request_id);
  * no outputs are skipped; the call then returns CF_ERROR_INVALID_ARGUMENT
  * after releasing every other one. */
 CFCULL_API int cf_server_release_many(CfServer* server, const uint64_t* request_ids, uint32_t n);
+/* Culling configuration of a grid's served requests, as cf_batch_set_tuning;
+ * (4, 8, 32, 1), the hit masks, is a batch's and a single view's only and is
+ * refused with CF_ERROR_INVALID_ARGUMENT. */
 CFCULL_API int cf_server_set_tuning(CfServer* server, uint32_t slice_clusters, int clusters_per_warp, int warps,
                                     int tile, int stages);
 CFCULL_API int cf_server_get_stats(CfServer* server, CfServerStats* stats);
