@@ -233,6 +233,8 @@ _SIGS = {
     "cf_testing_inject_stall": [_U32],
     "cf_testing_fail_allocation_after": [C.c_int32],
     "cf_testing_fail_version_writes": [C.c_int32],
+    "cf_testing_fail_server_batches": [C.c_int32],
+    "cf_testing_early_batch_releases": [],
     "cf_batch_create": [_P, C.POINTER(_P)],
     "cf_batch_destroy": [_P],
     "cf_batch_set_views": [_P, C.POINTER(CfBatchView), _U32],

@@ -104,15 +104,21 @@ DeviceGuard::~DeviceGuard()
 namespace {
 std::atomic<int32_t> g_fail_allocation_after{-1};  // allocations to let through before one fails; < 0: none
 std::atomic<int32_t> g_fail_version_writes{0};     // server version-write launches still to fail
-}  // namespace
+std::atomic<int32_t> g_fail_server_batches{0};     // server batches still to fail
+std::atomic<uint32_t> g_early_batch_releases{0};
 
-bool take_injected_version_write_failure()
+bool take_one(std::atomic<int32_t>& left)
 {
-    int32_t n = g_fail_version_writes.load();
+    int32_t n = left.load();
     while (n > 0)
-        if (g_fail_version_writes.compare_exchange_weak(n, n - 1)) return true;
+        if (left.compare_exchange_weak(n, n - 1)) return true;
     return false;
 }
+}  // namespace
+
+bool take_injected_version_write_failure() { return take_one(g_fail_version_writes); }
+bool take_injected_server_batch_failure() { return take_one(g_fail_server_batches); }
+void note_early_batch_release() { g_early_batch_releases.fetch_add(1); }
 
 cudaError_t device_malloc(void** ptr, size_t bytes)
 {
@@ -953,5 +959,13 @@ int cf_testing_fail_version_writes(int32_t n)
     g_fail_version_writes.store(n > 0 ? n : 0);
     return CF_SUCCESS;
 }
+
+int cf_testing_fail_server_batches(int32_t n)
+{
+    g_fail_server_batches.store(n > 0 ? n : 0);
+    return CF_SUCCESS;
+}
+
+uint32_t cf_testing_early_batch_releases(void) { return g_early_batch_releases.load(); }
 
 }  // extern "C"

@@ -53,6 +53,12 @@ cudaError_t device_malloc(void** ptr, size_t bytes);
 // queued light-set uploads and jitters to fail (cf_testing_fail_version_writes).
 bool take_injected_version_write_failure();
 
+// The same for the server's next batch, after its first kernels
+// (cf_testing_fail_server_batches); and counts a batch that failed and whose
+// memory was given back before its stream was idle.
+bool take_injected_server_batch_failure();
+void note_early_batch_release();
+
 // Ensures *ptr holds at least `bytes` of zero-filled device memory.
 int grow(void** ptr, size_t* capacity, size_t bytes, const char* what);
 

@@ -557,6 +557,7 @@ int enqueue_batch(CfServer* s, int slot_i, const LaunchPlan& plan, const std::ve
         e = cfk::launch_batch_xform(d_jobs, d_prefix, n, plan.xform_blocks, sl.d_queues,
                                     (uint32_t)plan.buckets.size(), st);
     if (e == cudaSuccess) e = cfk::launch_batch_bin(d_jobs, d_prefix + n, nullptr, n, plan.bin_blocks, st);
+    if (e == cudaSuccess && take_injected_server_batch_failure()) return fail(CF_ERROR_CUDA, "server batch launch (injected)");
     for (size_t q = 0; q < plan.buckets.size() && e == cudaSuccess; ++q) {
         const LaunchPlan::Bucket& bk = plan.buckets[q];
         int ctas = 0;
@@ -704,6 +705,13 @@ void worker_main(CfServer* s)
             fill_tables(s, (int)q, batch, plan);
             const int jst = launch_jobs(s, jobs);
             const int st = jst == CF_SUCCESS ? enqueue_batch(s, (int)q, plan, batch) : jst;
+            if (st != CF_SUCCESS) {
+                // What was launched before the failure still uses the requests'
+                // workspaces and the slot's tables: both may go to another
+                // stream's batch, or be rewritten, only once it has finished.
+                cudaStreamSynchronize(s->slots[q].s);
+                if (cudaStreamQuery(s->slots[q].s) == cudaErrorNotReady) note_early_batch_release();
+            }
             lk = take_lock(s->mu);
             if (jst != CF_SUCCESS) mark_failed(jobs);
             release_jobs(s, jobs);

@@ -42,6 +42,14 @@ CFCULL_API int cf_testing_fail_allocation_after(int32_t n);
  * n <= 0 turns this off.  The versions they would have written are marked
  * failed, and every request bound to one completes with CF_ERROR_CUDA. */
 CFCULL_API int cf_testing_fail_version_writes(int32_t n);
+/* Makes the servers' next n batches fail as a failed launch in their middle
+ * would: the light transform and the slice lists are launched, the culling is
+ * not, and every request of the batch completes with CF_ERROR_CUDA; n <= 0
+ * turns this off. */
+CFCULL_API int cf_testing_fail_server_batches(int32_t n);
+/* How many failed batches of this process gave their workspaces and tables
+ * back while kernels of theirs were still in flight (0: none may). */
+CFCULL_API uint32_t cf_testing_early_batch_releases(void);
 
 #ifdef __cplusplus
 }
