@@ -166,37 +166,9 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
-{
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 
-// hit_fast (cf_device.cuh) for two lights against one box at once: light A
-// in the low halves, light B in the high halves; the box bounds duplicated
-// in both halves.  Each half is exactly hit_fast's arithmetic.
-__device__ __forceinline__ void hit_pair(f2 lx, f2 ly, f2 lz, float ar2, float br2, f2 mnx, f2 mny, f2 mnz, f2 mxx,
-                                         f2 mxy, f2 mxz, bool& ha, bool& hb)
-{
-    float a0, a1, b0, b1;
-    f2_unpack(f2_sub(mnx, lx), a0, a1);
-    f2_unpack(f2_sub(lx, mxx), b0, b1);
-    const f2 dx = f2_pack(max3f(a0, b0, 0.0f), max3f(a1, b1, 0.0f));
-    f2_unpack(f2_sub(mny, ly), a0, a1);
-    f2_unpack(f2_sub(ly, mxy), b0, b1);
-    const f2 dy = f2_pack(max3f(a0, b0, 0.0f), max3f(a1, b1, 0.0f));
-    f2_unpack(f2_sub(mnz, lz), a0, a1);
-    f2_unpack(f2_sub(lz, mxz), b0, b1);
-    const f2 dz = f2_pack(max3f(a0, b0, 0.0f), max3f(a1, b1, 0.0f));
-    const f2 sq = f2_add(f2_add(f2_mul(dx, dx), f2_mul(dy, dy)), f2_mul(dz, dz));
-    float sa, sb;
-    f2_unpack(sq, sa, sb);
-    ha = sa < ar2;
-    hb = sb < br2;
-}
-
-// hit_fast for two lights against one box: the differences and squares packed,
+// hit_fast for two lights against one box, light A in the low halves and light
+// B in the high halves, the box bounds in both: the differences and squares packed,
 // the sums scalar.  The compiler merges a packed product and a packed sum into
 // one packed FMA, rounding once where the shader rounds twice (a light one ulp
 // from a box's reach then changes sides), also under -fmad=false and however

@@ -9,12 +9,13 @@
 //      a packed instruction wants.
 //   2. The CTA's W*S warps form S sets of W: warp w of a set owns light chunks
 //      [w*J, (w+1)*J) of 32 lights each; every lane transforms its J lights
-//      itself, two per packed operation (posView = cameraView * position in
+//      itself, two per packed product (posView = cameraView * position in
 //      the pinned order, r^2), and keeps them in registers.
 //   3. Set s tests its chunks against boxes s, s+S, ... of the CTA, two
-//      chunks per packed instruction (sub/mul/add.rn.f32x2: two IEEE
-//      round-to-nearest operations each, the same bits as the scalar ones),
-//      and stores each test's 32 results as one __ballot_sync mask:
+//      chunks per packed difference and square (sub/mul.rn.f32x2: two IEEE
+//      round-to-nearest operations each, the same bits as the scalar ones;
+//      the sums are scalar, as a packed one would be merged with the products
+//      and round once), and stores each test's 32 results as one __ballot_sync mask:
 //      mask[m][chunk].  A chunk holding a non-finite light coordinate takes
 //      the shader's branchy test.
 //   4. Cluster m's list is its masks' set bits in chunk order: a warp scan of
@@ -113,10 +114,13 @@ __global__ void __launch_bounds__(W * S * 32) one_launch_kernel(const FusedCull 
 #pragma unroll
         for (int row = 0; row < 3; ++row) {  // ((m[row]*x + m[4+row]*y) + m[8+row]*z) + m[12+row]*w
             const float* m = f.view;
-            f2 acc = f2_add(f2_mul(f2_pack(m[row], m[row]), px), f2_mul(f2_pack(m[4 + row], m[4 + row]), py));
-            acc = f2_add(acc, f2_mul(f2_pack(m[8 + row], m[8 + row]), pz));
-            acc = f2_add(acc, f2_mul(f2_pack(m[12 + row], m[12 + row]), pw));
-            f2_unpack(acc, v[row][0], v[row][1]);
+            float x[2], y[2], z[2], w[2];  // products packed, sums scalar (see hit_pair_twice_rounded)
+            f2_unpack(f2_mul(f2_pack(m[row], m[row]), px), x[0], x[1]);
+            f2_unpack(f2_mul(f2_pack(m[4 + row], m[4 + row]), py), y[0], y[1]);
+            f2_unpack(f2_mul(f2_pack(m[8 + row], m[8 + row]), pz), z[0], z[1]);
+            f2_unpack(f2_mul(f2_pack(m[12 + row], m[12 + row]), pw), w[0], w[1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) v[row][h] = __fadd_rn(__fadd_rn(__fadd_rn(x[h], y[h]), z[h]), w[h]);
         }
         float r2a, r2b;
         f2_unpack(f2_mul(f2_pack(ra, rb), f2_pack(ra, rb)), r2a, r2b);
@@ -163,7 +167,7 @@ __global__ void __launch_bounds__(W * S * 32) one_launch_kernel(const FusedCull 
             for (int q = 0; q < J / 2; ++q) {
                 bool ha, hb;
                 if (!(bad & (3u << (2 * q)))) {
-                    hit_pair(px[q], py[q], pz[q], lr2[2 * q], lr2[2 * q + 1], mnx, mny, mnz, mxx, mxy, mxz, ha, hb);
+                    hit_pair_twice_rounded(px[q], py[q], pz[q], lr2[2 * q], lr2[2 * q + 1], mnx, mny, mnz, mxx, mxy, mxz, ha, hb);
                 } else {
                     float t0, t1;
                     float mn[3], mx[3];
