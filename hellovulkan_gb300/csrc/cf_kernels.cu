@@ -1448,21 +1448,24 @@ bool cull_config_supported(const CullConfig& c)
 // Below both lines, a view whose lights fit one launch's registers (at most
 // kOneLaunchMaxLights) and whose clusters spread over the resident CTAs at
 // most kOneLaunchMaxClustersPerCta each is culled in one launch; the rest
-// brute force.  Grids beyond the hit-mask path's limits (mask_fits) take the
-// staged binned path once it pays: 453 M tests cull five times faster with it
-// than brute force, 16 M about the same.
+// brute force.  Without the hit masks (grids beyond mask_fits, or scratch that
+// does not hold theirs), the staged binned path once it pays: 453 M tests cull
+// five times faster with it than brute force, 16 M about the same.
 constexpr uint32_t kMaskMinLights = 2304;
 constexpr uint64_t kMaskMinTests = 10ull << 20;
 constexpr uint64_t kStagedMinTests = 16ull << 20;
 
 CullConfig default_cull_config(uint32_t clusters, uint32_t lights, uint32_t slices)
 {
-    const uint64_t tests = (uint64_t)clusters * lights;
-    if (slices >= 2 && mask_fits(clusters, clusters / slices, slices)) {
-        if (lights >= kMaskMinLights || tests >= kMaskMinTests) return kMaskConfig;
-    } else if (slices >= 2 && tests >= kStagedMinTests) {
-        return kStagedConfig;
-    }
+    if (slices >= 2 && mask_fits(clusters, clusters / slices, slices) &&
+        (lights >= kMaskMinLights || (uint64_t)clusters * lights >= kMaskMinTests))
+        return kMaskConfig;
+    return unmasked_cull_config(clusters, lights, slices);
+}
+
+CullConfig unmasked_cull_config(uint32_t clusters, uint32_t lights, uint32_t slices)
+{
+    if (slices >= 2 && (uint64_t)clusters * lights >= kStagedMinTests) return kStagedConfig;
     CullConfig one{};
     if (one_launch_config(clusters, lights, &one)) return one;
     if (clusters <= 8192) return CullConfig{1, 8, 512, 4, 0};

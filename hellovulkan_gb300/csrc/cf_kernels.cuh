@@ -243,6 +243,7 @@ cudaError_t launch_one_launch(const FusedCull& f, int warps, int max_lights, uin
 
 bool cull_config_supported(const CullConfig& c);
 CullConfig default_cull_config(uint32_t clusters, uint32_t lights, uint32_t slices);
+CullConfig unmasked_cull_config(uint32_t clusters, uint32_t lights, uint32_t slices);  // ... without the hit masks
 
 // Test knobs of the culling kernels on the current device (cf_device.cuh):
 // the bounded-wait limit and the injected stall bits, per translation unit.

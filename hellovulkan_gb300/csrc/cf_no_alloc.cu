@@ -126,13 +126,14 @@ extern "C" int cf_cull_lights_static_scratch(const CfClusterForwardUBO* ubo, con
     if (index_capacity < (uint64_t)C * cap)
         return fail(CF_ERROR_CAPACITY, "index capacity %llu < clusters x cap = %llu", (unsigned long long)index_capacity,
                     (unsigned long long)C * cap);
-    // the automatic kernel choice when its scratch fits, else the brute-force
-    // kernels, which need less (both give the same result)
-    cfk::CullConfig cfg = choose_config(*ubo, light_count, nullptr);
-    uint64_t bytes = scratch_bytes(*ubo, light_count, cap, cfg);
+    // the automatic kernel choice when its scratch fits, without the hit masks
+    // when theirs does not, else the brute-force kernels, which need least (all
+    // give the same result)
+    uint64_t bytes = 0;
+    cfk::CullConfig cfg = choose_within(*ubo, light_count, cap, kStaticScratchBytes, &bytes);
     if (bytes > kStaticScratchBytes && cfg.binned) {
-        cfg = cfk::default_cull_config(C, light_count, 1);
-        bytes = scratch_bytes(*ubo, light_count, cap, cfg);
+        cfg = cfk::unmasked_cull_config(C, light_count, 1);
+        bytes = cull_bytes(*ubo, light_count, cap, cfg);
     }
     if (bytes > kStaticScratchBytes)
         return fail(CF_ERROR_CAPACITY,

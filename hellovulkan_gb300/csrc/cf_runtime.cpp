@@ -172,11 +172,15 @@ cfk::WorkspaceLayout layout_for(const CfClusterForwardUBO& ubo, uint32_t light_c
     return cfk::workspace_layout(C, light_count, cap, ubo.sliceCountZ, cfg.binned, groups);
 }
 
-uint64_t scratch_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, const cfk::CullConfig& cfg)
+cfk::CullConfig choose_within(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, uint64_t available,
+                              uint64_t* needed)
 {
-    const uint64_t needed = cull_bytes(ubo, light_count, cap, cfg);
-    if (!cfk::is_mask_config(cfg)) return needed;
-    return std::max<uint64_t>(needed, layout_for(ubo, light_count, cap, cfk::kStagedConfig).bytes);
+    cfk::CullConfig cfg = choose_config(ubo, light_count, nullptr);
+    *needed = cull_bytes(ubo, light_count, cap, cfg);
+    if (!cfk::is_mask_config(cfg) || *needed <= available) return cfg;
+    cfg = cfk::unmasked_cull_config(ubo.sliceCountX * ubo.sliceCountY * ubo.sliceCountZ, light_count, ubo.sliceCountZ);
+    *needed = cull_bytes(ubo, light_count, cap, cfg);
+    return cfg;
 }
 
 uint64_t cull_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, const cfk::CullConfig& cfg)
@@ -865,7 +869,11 @@ int cf_cull_workspace_size(const CfClusterForwardUBO* ubo, uint32_t light_count,
     uint32_t C = 0;
     int s = validate_grid(ubo->sliceCountX, ubo->sliceCountY, ubo->sliceCountZ, cap, &C);
     if (s) return s;
-    *bytes = scratch_bytes(*ubo, light_count, cap, choose_config(*ubo, light_count, nullptr));
+    // enough for the automatic choice, and never less than what cf_cull_lights takes
+    uint64_t best = 0, least = 0;
+    choose_within(*ubo, light_count, cap, UINT64_MAX, &best);
+    choose_within(*ubo, light_count, cap, 0, &least);
+    *bytes = std::max(best, least);
     return CF_SUCCESS;
 }
 
@@ -906,8 +914,8 @@ int cf_cull_lights(const CfClusterForwardUBO* ubo, const CfAABB* d_aabbs, const 
     if (index_capacity < (uint64_t)C * cap)
         return fail(CF_ERROR_CAPACITY, "index capacity %llu < clusters x cap = %llu", (unsigned long long)index_capacity,
                     (unsigned long long)C * cap);
-    const cfk::CullConfig cfg = choose_config(*ubo, light_count, nullptr);
-    const uint64_t needed = scratch_bytes(*ubo, light_count, cap, cfg);
+    uint64_t needed = 0;
+    const cfk::CullConfig cfg = choose_within(*ubo, light_count, cap, workspace_bytes, &needed);
     if (workspace_bytes < needed)
         return fail(CF_ERROR_CAPACITY, "workspace %llu bytes < %llu needed", (unsigned long long)workspace_bytes,
                     (unsigned long long)needed);

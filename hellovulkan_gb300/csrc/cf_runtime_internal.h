@@ -67,11 +67,15 @@ cfk::CullConfig choose_config(const CfClusterForwardUBO& ubo, uint32_t light_cou
                               const cfk::CullConfig* override_cfg);
 cfk::WorkspaceLayout layout_for(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap,
                                 const cfk::CullConfig& cfg);
-// Scratch that enqueue_cull needs, and the size that callers who bring their
-// own are asked for: never less than the staged binned path's, so that views
-// accepted or refused by size before the hit-mask path still are.
+// Scratch that enqueue_cull needs.
 uint64_t cull_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, const cfk::CullConfig& cfg);
-uint64_t scratch_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, const cfk::CullConfig& cfg);
+// The automatic choice for a caller who brings `available` bytes of scratch: the
+// hit masks need more than what a view took before they came (by a factor of
+// up to three on large grids, of hundreds on views of a few clusters), so where
+// they are chosen and do not fit, the choice without them; *needed is the
+// scratch of the configuration returned.
+cfk::CullConfig choose_within(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, uint64_t available,
+                              uint64_t* needed);
 
 // Light transform (+ slice binning) + culling + offset scan of one view on `stream`.
 int enqueue_cull(const CfClusterForwardUBO& ubo, const CfAABB* d_aabbs, const CfLightData* d_lights,

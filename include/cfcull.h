@@ -410,8 +410,10 @@ CFCULL_API int cf_serve_run_load(CfServer* server, const CfServeLoad* load, CfSe
 /* Stateless entry points on caller-owned device memory.                     */
 /* ------------------------------------------------------------------------ */
 
-/* Bytes of device workspace cf_cull_lights needs for a view of this grid
- * (ubo: host pointer) and light count. */
+/* Bytes of device workspace with which cf_cull_lights takes its own choice of
+ * kernels for a view of this grid (ubo: host pointer) and light count.  (A
+ * view that would be culled by hit masks is taken with less, by the other
+ * kernels, with the same output.) */
 CFCULL_API int cf_cull_workspace_size(const CfClusterForwardUBO* ubo, uint32_t light_count,
                                       uint32_t max_lights_per_cluster, uint64_t* bytes);
 /* AABBGenerator.comp over the grid of `ubo` (host pointer) into
@@ -475,7 +477,7 @@ CFCULL_API int cf_frustum_cull(const CfFrustum* frustum, const CfAABB* d_boxes, 
                                CfDrawIndirectCommand* d_commands, uint32_t* d_visible, void* stream);
 /* LightCulling.comp: d_cells[C] and d_indices (capacity >= C * cap) from
  * d_aabbs[C] and d_lights[light_count]; d_total (optional, device) receives
- * the number of indices.  d_workspace: >= cf_cull_workspace_size bytes,
+ * the number of indices.  d_workspace: cf_cull_workspace_size bytes,
  * 256-byte aligned, zero-filled once after allocation (its first word is the
  * device error word that bounded in-kernel waits set on timeout). */
 CFCULL_API int cf_cull_lights(const CfClusterForwardUBO* ubo, const CfAABB* d_aabbs, const CfLightData* d_lights,
