@@ -142,12 +142,16 @@ void drop_graph(CfBatch* b)
 }
 
 // The configuration of a view of this grid: the bucket's tuning (a hit-mask
-// tuning only where the grid fits it), else the hit-mask path where it fits.
-cfk::CullConfig config_for(const CfBatch* b, uint32_t key, uint32_t slices)
+// tuning only where the grid fits it), else the hit-mask path where it pays.
+cfk::CullConfig config_for(const CfBatch* b, uint32_t key, uint32_t slices, uint32_t lights)
 {
     auto it = b->tuned.find(key);
-    const cfk::CullConfig c = it == b->tuned.end() ? cfk::kMaskConfig : it->second;
-    return cfk::is_mask_config(c) && !cfk::mask_fits(key * slices, key, slices) ? cfk::kStagedConfig : c;
+    const bool tuned = it != b->tuned.end();
+    const cfk::CullConfig c = tuned ? it->second : cfk::kMaskConfig;
+    if (!cfk::is_mask_config(c)) return c;
+    return (tuned ? cfk::mask_fits(key * slices, key, slices) : cfk::mask_pays(key * slices, key, slices, lights))
+               ? c
+               : cfk::kStagedConfig;
 }
 
 // The staged configuration of a grid's views that are not on the hit-mask path.
@@ -177,7 +181,9 @@ int validate_view(const CfBatchView& v, uint32_t i, uint32_t* clusters)
 }
 
 // Recomputes every derived table from b->views and b->tuned and uploads it.
-int rebuild(CfBatch* b)
+// Where the device has no room for the workspaces with hit masks, which need up
+// to a few times the staged path's, once more without them (`masks` false).
+int rebuild(CfBatch* b, bool masks = true)
 {
     const int w = wait_idle(b);  // passes still queued read the tables rewritten below
     if (w) return w;
@@ -198,7 +204,8 @@ int rebuild(CfBatch* b)
         uint32_t C = 0;
         const int s = validate_view(bv, i, &C);
         if (s) return s;
-        cfgs[i] = config_for(b, bv.ubo.sliceCountX * bv.ubo.sliceCountY, bv.ubo.sliceCountZ);
+        cfgs[i] = config_for(b, bv.ubo.sliceCountX * bv.ubo.sliceCountY, bv.ubo.sliceCountZ, bv.light_count);
+        if (!masks && cfk::is_mask_config(cfgs[i])) cfgs[i] = cfk::kStagedConfig;
         if (cfk::is_mask_config(cfgs[i])) {
             mask_views.push_back(i);
             most_lights = std::max(most_lights, bv.light_count);
@@ -268,6 +275,10 @@ int rebuild(CfBatch* b)
     b->ws_bytes = ws;
     DeviceGuard g(b->device);
     int s = grow(reinterpret_cast<void**>(&b->d_ws), &b->ws_cap, std::max<size_t>(ws, 256), "batch workspace");
+    if (s == CF_ERROR_OUT_OF_MEMORY && nm) {
+        cudaGetLastError();
+        return rebuild(b, false);
+    }
     if (s) return s;
     for (uint32_t i = 0; i < n; ++i) {
         cfk::ViewJob& j = b->jobs[b->pos[i]];
@@ -316,7 +327,7 @@ int rebuild(CfBatch* b)
     b->launches.clear();
     for (auto it = by_key.rbegin(); it != by_key.rend(); ++it) {
         std::vector<uint32_t>& vs = it->second;
-        // a bucket has one configuration, but for slices too many for the hit-mask path
+        // a bucket has one configuration, but for views with slices or lights too many for the hit-mask path
         uint32_t mask_ctas = 0, mask_groups = 0;
         auto on_mask = [&](uint32_t q) { return q >= ns; };
         for (uint32_t q : vs)

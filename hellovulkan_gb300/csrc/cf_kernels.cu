@@ -1448,7 +1448,7 @@ bool cull_config_supported(const CullConfig& c)
 // Below both lines, a view whose lights fit one launch's registers (at most
 // kOneLaunchMaxLights) and whose clusters spread over the resident CTAs at
 // most kOneLaunchMaxClustersPerCta each is culled in one launch; the rest
-// brute force.  Without the hit masks (grids beyond mask_fits, or scratch that
+// brute force.  Without the hit masks (views beyond mask_pays, or scratch that
 // does not hold theirs), the staged binned path once it pays: 453 M tests cull
 // five times faster with it than brute force, 16 M about the same.
 constexpr uint32_t kMaskMinLights = 2304;
@@ -1457,7 +1457,7 @@ constexpr uint64_t kStagedMinTests = 16ull << 20;
 
 CullConfig default_cull_config(uint32_t clusters, uint32_t lights, uint32_t slices)
 {
-    if (slices >= 2 && mask_fits(clusters, clusters / slices, slices) &&
+    if (slices >= 2 && mask_pays(clusters, clusters / slices, slices, lights) &&
         (lights >= kMaskMinLights || (uint64_t)clusters * lights >= kMaskMinTests))
         return kMaskConfig;
     return unmasked_cull_config(clusters, lights, slices);

@@ -201,6 +201,27 @@ inline bool mask_fits(uint32_t clusters, uint32_t slice_clusters, uint32_t slice
 {
     return slices <= kMaskMaxSlices && group_count(clusters, slice_clusters, slices, kMaskGroup, kModeBinned) <= kMaskMaxGroups;
 }
+// Whether the automatic choices may give the hit-mask path a view of that many
+// lights.  A unit (128 lights of every group) has 100 bytes of its workspace:
+// they may be half a gigabyte, or twice the slice lists, which the staged path
+// has too (128x128x64 with 65536 lights would take 1.8 GB where that takes
+// 0.3).  And a scanning warp steps over the windows of 32 segments (32768
+// lights) before its candidates; units times windows, hit masks against staged:
+//   16x9x24,  4 M lights   457 M   1175 against  2088 us
+//   40x24x56, 1 M lights   400 M    666 against   880 us
+//   8x8x16,  16 M lights  1950 M   6009 against 10674 us (few groups: staged is slow)
+//   32x18x48, 4 M lights  3300 M   3419 against  2074 us
+//   16x9x24, 16 M lights  7300 M  10575 against  8166 us
+constexpr uint64_t kMaskUnitBytes = 100, kMaskMaxUnitBytes = 512ull << 20, kMaskMaxWindowSteps = 2000ull << 20;
+inline bool mask_pays(uint32_t clusters, uint32_t slice_clusters, uint32_t slices, uint32_t lights)
+{
+    if (!mask_fits(clusters, slice_clusters, slices)) return false;
+    const uint64_t lpad = pad_lights(lights), groups = group_count(clusters, slice_clusters, slices, kMaskGroup, kModeBinned);
+    const uint64_t units = groups * ((lpad + kMaskMaxRun - 1) / kMaskMaxRun), lists = 20ull * slices * lpad;
+    const uint64_t windows = (lpad + 32 * kMaxSegLights - 1) / (32 * kMaxSegLights);
+    const uint64_t most = 2 * lists > kMaskMaxUnitBytes ? 2 * lists : kMaskMaxUnitBytes;
+    return kMaskUnitBytes * units <= most && units * windows <= kMaskMaxWindowSteps;
+}
 
 // One-launch culling of a small view (cf_fused.cu): light transform,
 // LightCulling.comp's test for every (cluster, light) pair, the capped

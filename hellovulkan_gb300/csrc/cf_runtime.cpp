@@ -156,13 +156,6 @@ int grow(void** ptr, size_t* capacity, size_t bytes, const char* what)
     return CF_SUCCESS;
 }
 
-cfk::CullConfig choose_config(const CfClusterForwardUBO& ubo, uint32_t light_count, const cfk::CullConfig* override_cfg)
-{
-    if (override_cfg) return *override_cfg;
-    const uint32_t C = ubo.sliceCountX * ubo.sliceCountY * ubo.sliceCountZ;
-    return cfk::default_cull_config(C, light_count, ubo.sliceCountZ);
-}
-
 cfk::WorkspaceLayout layout_for(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap,
                                 const cfk::CullConfig& cfg)
 {
@@ -175,10 +168,11 @@ cfk::WorkspaceLayout layout_for(const CfClusterForwardUBO& ubo, uint32_t light_c
 cfk::CullConfig choose_within(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap, uint64_t available,
                               uint64_t* needed)
 {
-    cfk::CullConfig cfg = choose_config(ubo, light_count, nullptr);
+    const uint32_t C = ubo.sliceCountX * ubo.sliceCountY * ubo.sliceCountZ;
+    cfk::CullConfig cfg = cfk::default_cull_config(C, light_count, ubo.sliceCountZ);
     *needed = cull_bytes(ubo, light_count, cap, cfg);
     if (!cfk::is_mask_config(cfg) || *needed <= available) return cfg;
-    cfg = cfk::unmasked_cull_config(ubo.sliceCountX * ubo.sliceCountY * ubo.sliceCountZ, light_count, ubo.sliceCountZ);
+    cfg = cfk::unmasked_cull_config(C, light_count, ubo.sliceCountZ);
     *needed = cull_bytes(ubo, light_count, cap, cfg);
     return cfg;
 }
@@ -331,6 +325,7 @@ struct CfResourcesClusterForward {
     uint32_t* d_total = nullptr;
     unsigned char* d_ws = nullptr;
     size_t ws_capacity = 0;
+    uint64_t ws_refused = UINT64_MAX;  // least workspace that the device had no room for since CreateBuffers
     uint32_t* h_total = nullptr;  // pinned word the one-launch read-back writes the total into
     bool aabb_dirty = true;
     bool aabb_built = false;
@@ -363,6 +358,14 @@ uint32_t* context_error_word(const CfContext* ctx) { return ctx->dev_error; }
 
 namespace {
 
+// The tuning, or the automatic choice within what the device had room for; its scratch in *bytes.
+cfk::CullConfig pipeline_config(const CfPipelineLightCulling* p, uint64_t* bytes)
+{
+    if (!p->has_cfg) return choose_within(p->ubo, p->lights->count, p->res->cap, p->res->ws_refused - 1, bytes);
+    *bytes = cull_bytes(p->ubo, p->lights->count, p->res->cap, p->cfg);
+    return p->cfg;
+}
+
 void free_cluster_buffers(CfResourcesClusterForward* r)
 {
     cudaFree(r->d_aabbs);
@@ -376,6 +379,7 @@ void free_cluster_buffers(CfResourcesClusterForward* r)
     r->d_total = nullptr;
     r->d_ws = nullptr;
     r->ws_capacity = 0;
+    r->ws_refused = UINT64_MAX;
 }
 
 }  // namespace
@@ -809,9 +813,16 @@ int cf_pipeline_light_culling_fill_command_buffer(CfPipelineLightCulling* p, voi
     if (p->lights->count && !p->lights->d_lights) return fail(CF_ERROR_NOT_READY, "no lights uploaded");
     DeviceGuard g(p->ctx->device);
     if (g.err()) return cuda_fail(g.err(), "cudaSetDevice");
-    const cfk::CullConfig cfg = choose_config(p->ubo, p->lights->count, p->has_cfg ? &p->cfg : nullptr);
-    int s = grow(reinterpret_cast<void**>(&r->d_ws), &r->ws_capacity, cull_bytes(p->ubo, p->lights->count, r->cap, cfg),
-                 "culling workspace");
+    uint64_t bytes = 0;
+    cfk::CullConfig cfg = pipeline_config(p, &bytes);
+    int s = grow(reinterpret_cast<void**>(&r->d_ws), &r->ws_capacity, bytes, "culling workspace");
+    if (s == CF_ERROR_OUT_OF_MEMORY && !p->has_cfg && cfk::is_mask_config(cfg)) {
+        // no room for the hit masks: the kernels that need less, from now on too
+        cudaGetLastError();
+        r->ws_refused = bytes;
+        cfg = pipeline_config(p, &bytes);
+        s = grow(reinterpret_cast<void**>(&r->d_ws), &r->ws_capacity, bytes, "culling workspace");
+    }
     if (s) return s;
     return enqueue_cull(p->ubo, r->d_aabbs, p->lights->d_lights, p->lights->count, r->cap, r->d_cells, r->d_indices,
                         r->d_total, r->d_ws, p->ctx->dev_error, cfg, (cudaStream_t)stream,
@@ -841,7 +852,8 @@ int cf_pipeline_light_culling_get_tuning(const CfPipelineLightCulling* p, int co
 {
     if (!p || !config) return fail(CF_ERROR_INVALID_ARGUMENT, "null argument");
     if (!p->has_ubo || !p->lights) return fail(CF_ERROR_NOT_READY, "no cluster-forward UBO set yet");
-    const cfk::CullConfig c = choose_config(p->ubo, p->lights->count, p->has_cfg ? &p->cfg : nullptr);
+    uint64_t bytes = 0;
+    const cfk::CullConfig c = pipeline_config(p, &bytes);
     config[0] = c.clusters_per_warp;
     config[1] = c.warps;
     config[2] = c.tile;

@@ -62,9 +62,6 @@ void note_early_batch_release();
 // Ensures *ptr holds at least `bytes` of zero-filled device memory.
 int grow(void** ptr, size_t* capacity, size_t bytes, const char* what);
 
-// The culling configuration for a view: the override, else the automatic choice.
-cfk::CullConfig choose_config(const CfClusterForwardUBO& ubo, uint32_t light_count,
-                              const cfk::CullConfig* override_cfg);
 cfk::WorkspaceLayout layout_for(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32_t cap,
                                 const cfk::CullConfig& cfg);
 // Scratch that enqueue_cull needs.

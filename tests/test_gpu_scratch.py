@@ -65,3 +65,97 @@ def test_static_scratch_takes_the_staged_kernels_before_brute_force(cflib, hooks
         cflib.cf_testing_set_wait_limit_ns(0)
     o_cells, o_idx = _oracle(oracle, v, aabbs)
     assert np.array_equal(cells, o_cells) and np.array_equal(idx, o_idx)
+
+
+def pipeline(gpu, v):
+    from hellovulkan_gb300.pipelines import (PipelineAABBGenerator, PipelineLightCulling, ResourcesClusterForward,
+                                             ResourcesLight)
+    rl, rc = ResourcesLight(gpu), ResourcesClusterForward(gpu)
+    rl.add_lights(v.lights)
+    rc.create_buffers(*v.grid, v.cap)
+    gen, cull = PipelineAABBGenerator(gpu, rc), PipelineLightCulling(gpu, rl, rc)
+    gen.set_cluster_forward_ubo(v.ubo)
+    gen.fill_command_buffer()
+    cull.set_cluster_forward_ubo(v.ubo)
+    return cull, rc, (cull, gen, rc, rl)
+
+
+STAGED, MASK = (2, 8, 1024, 2, 1), (4, 8, 32, 1, 1)
+
+
+# units of 128 lights and a group: 100 bytes each, half a gigabyte or twice the lists' bytes at most
+@pytest.mark.parametrize("grid, n_lights, want", [((128, 128, 24), 32768, MASK), ((128, 128, 24), 65536, STAGED),
+                                                  ((64, 36, 4), 3500000, STAGED), ((64, 18, 4), 1000000, MASK)])
+def test_views_whose_masks_would_take_too_much_memory(gpu, oracle, grid, n_lights, want):
+    """The choice on both sides of the line, for a pipeline and for a batch,
+    and the same lists from both sides."""
+    import torch
+
+    from hellovulkan_gb300.batch import Batch, BatchBuffers
+    v = view(grid, n_lights, cap=4)
+    cull, rc, objects = pipeline(gpu, v)
+    assert cull.tuning() == want
+    cull.fill_command_buffer()
+    cells, idx = rc.read_outputs()
+    cells, idx = cells.copy(), idx.copy()
+    cull.set_tuning(*(STAGED if want == MASK else MASK))
+    cull.fill_command_buffer()
+    other = rc.read_outputs()
+    assert np.array_equal(cells, other[0]) and np.array_equal(idx, other[1])
+    for o in objects:
+        o.close()
+    bufs = BatchBuffers([v])
+    b = Batch(gpu)
+    b.set_views(bufs.batch_views())
+    assert b.info()["bucket_configs"][0]["config"] == list(want[:4])
+    b.generate_aabbs()
+    b.cull()
+    torch.cuda.synchronize()
+    _, c, i = bufs.read(0)
+    assert np.array_equal(cells, c) and np.array_equal(idx, i)
+    b.close()
+
+
+def test_without_room_for_the_masks_the_other_kernels_run(gpu, hooks, oracle):  # noqa: F811
+    from hellovulkan_gb300.batch import Batch, BatchBuffers
+    v = view((16, 9, 24), 6000, cap=150)
+    a = oracle.generate_aabbs(v.ubo)
+    oc, oi, _ = oracle.cull(v.ubo, a, v.lights, v.cap)
+    cull, rc, objects = pipeline(gpu, v)
+    assert cull.tuning() == MASK
+    hooks.cf_testing_fail_allocation_after(0)  # the workspace with hit masks
+    for _ in range(2):
+        cull.fill_command_buffer()
+        cells, idx = rc.read_outputs()
+        assert np.array_equal(cells, oc) and np.array_equal(idx, oi)
+        assert cull.tuning() == STAGED
+    hooks.cf_testing_fail_allocation_after(-1)
+    rc.create_buffers(*v.grid, v.cap)
+    assert cull.tuning() == MASK
+    for o in objects:
+        o.close()
+    bufs = BatchBuffers([v])
+    b = Batch(gpu)
+    hooks.cf_testing_fail_allocation_after(0)
+    b.set_views(bufs.batch_views())
+    hooks.cf_testing_fail_allocation_after(-1)
+    assert b.info()["bucket_configs"][0]["config"] == list(STAGED[:4])
+    b.generate_aabbs()
+    b.cull()
+    _, c, i = bufs.read(0)
+    assert np.array_equal(oc, c) and np.array_equal(oi, i)
+    b.close()
+
+
+def test_without_room_for_any_the_failure_is_reported(gpu, hooks):  # noqa: F811
+    from hellovulkan_gb300._lib import CfError
+    v = view((16, 9, 24), 6000)
+    cull, rc, objects = pipeline(gpu, v)
+    cull.set_tuning(*MASK)  # asked for by name: nothing takes its place
+    hooks.cf_testing_fail_allocation_after(0)
+    with pytest.raises(CfError) as e:
+        cull.fill_command_buffer()
+    assert e.value.status == 2  # CF_ERROR_OUT_OF_MEMORY
+    hooks.cf_testing_fail_allocation_after(-1)
+    for o in objects:
+        o.close()
