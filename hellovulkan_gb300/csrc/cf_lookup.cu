@@ -331,13 +331,26 @@ __device__ __forceinline__ uint32_t containing(const ListWarp& w, uint32_t n, co
 // The warp reads the list of each cluster that its pixels lie in together: a
 // lane fetches and transforms an entry; then each pixel of the cluster tests
 // 32 of them, or, where the cluster has few of the warp's pixels, the lanes
-// test their entries against one pixel after another.
+// test their entries against one pixel after another.  Without the check, a warp
+// of many clusters or short lists has each pixel walk its own list, kOwnStep
+// entries at a time with the next ones' indices on their way.
 constexpr uint32_t kFewPixels = 3;  // entries per pixel from which a pixel's turn is cheaper than four entries' test
-// Where all lists of a warp's pixels are this short, each pixel walks its own (in
-// the launches of many tiles; 1920x1080, scattered: 49.5 -> 46.9 us).
+// Where all lists of a warp's pixels are this short, each pixel walks its own
+// (1920x1080, scattered: 49.5 -> 46.9 us), and where they lie in so many clusters
+// that the longest list has at most kOwnPerList entries for each: a cluster after
+// another is then a chain of round trips for a pixel or two each.  One thread
+// per unsorted pixel / only short lists walked / this rule, in us:
+//   96x64,    32x18x48, 16384 lights, scattered    45.3 / 59.5 / 14.5
+//   480x270,  64x64x64, 2000 lights, scattered     18.6 / 30.0 / 14.6
+//   480x270, 128x72x24, 4000 lights, surfaces      22.7 / 24.3 / 20.7
+//   20x20000, 16x9x24,  1024 lights, scattered     22.6 / 38.5 / 15.7
+//   1920x1080, 64x64x64, 2000 lights, scattered   107   / 114  / 64
+// A launch of many tiles is bound by issue and takes 4 entries per cluster
+// (6 / 8 / 12: the reference view's surfaces 46.4 -> 48.5 / 50.0 / 52.3), two at
+// a time; one of a tile per SM or less by latency: 12, four at a time.
 constexpr uint32_t kShortLookup = 4;
 constexpr uint32_t kBoxList = 8;    // a list up to this long is not worth a box
-template <bool kCheck, bool kOwn>
+template <bool kCheck, uint32_t kOwnStep, uint32_t kOwnPerList>
 __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table, bool whole, ListWarp& w, uint32_t lane,
                                         bool valid, float xf, float yf, float z, const float frag[3], CfFragmentSample& s)
 {
@@ -366,18 +379,38 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
         s.cluster = 0xFFFFFFFFu;
         s.flags |= CF_FRAGMENT_OUTSIDE_GRID;
     }
-    const bool own = kOwn && __reduce_max_sync(cfk::kFull, cnt) <= kShortLookup;
-    if (own) {
-        uint32_t li[kShortLookup];
+    bool own = false;
+    if (!kCheck) {
+        const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
+        own = longest <= kShortLookup;
+        if (!own) {
+            const uint32_t same = __match_any_sync(cfk::kFull, cnt ? c : ~0u);
+            own = longest <= kOwnPerList * __popc(__ballot_sync(cfk::kFull, cnt && (same & ((1u << lane) - 1u)) == 0));
+        }
+        if (own) {
+            uint32_t next[kOwnStep];
 #pragma unroll
-        for (uint32_t e = 0; e < kShortLookup; ++e) li[e] = e < cnt ? __ldg(&A.indices[off + e]) : 0u;
+            for (uint32_t e = 0; e < kOwnStep; ++e) next[e] = e < cnt ? __ldg(&A.indices[off + e]) : 0u;
+            for (uint32_t j = 0; j < longest; j += kOwnStep) {
+                float4 q[kOwnStep];
+                float r[kOwnStep];
 #pragma unroll
-        for (uint32_t e = 0; e < kShortLookup; ++e) {
-            if (e < cnt && li[e] >= A.light_count) s.flags |= CF_FRAGMENT_BAD_CELL;
-            if (e < cnt && li[e] < A.light_count) {
-                float p[3], r2;
-                light_view(u.cameraView, &A.lights[li[e]], p, &r2);
-                s.covering += contains(frag, p, r2) ? 1u : 0u;
+                for (uint32_t e = 0; e < kOwnStep; ++e) {
+                    const bool has = j + e < cnt, light = has && next[e] < A.light_count;
+                    if (has && !light) s.flags |= CF_FRAGMENT_BAD_CELL;
+                    const CfLightData* l = &A.lights[next[e]];
+                    q[e] = light ? __ldg(reinterpret_cast<const float4*>(&l->position[0])) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    r[e] = light ? __ldg(&l->radius) : __uint_as_float(0x7fffffffu);  // NaN: contains nothing
+                    next[e] = j + kOwnStep + e < cnt ? __ldg(&A.indices[off + j + kOwnStep + e]) : 0u;
+                }
+#pragma unroll
+                for (uint32_t e = 0; e < kOwnStep; ++e) {
+                    const float* V = u.cameraView;
+                    const float p[3] = {cf_mat4_row(V, 0, q[e].x, q[e].y, q[e].z, q[e].w),
+                                        cf_mat4_row(V, 1, q[e].x, q[e].y, q[e].z, q[e].w),
+                                        cf_mat4_row(V, 2, q[e].x, q[e].y, q[e].z, q[e].w)};
+                    s.covering += contains(frag, p, cf_fmul(r[e], r[e])) ? 1u : 0u;
+                }
             }
         }
     }
@@ -476,7 +509,7 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
 // runs the set through the table in pieces, 32 lights at a time against the box
 // of the warp's fragments.
 template <uint32_t kSide, uint32_t kThreads, bool kCheck>
-__global__ void __launch_bounds__(kThreads, 5 * 256 / kThreads) lookup_kernel(const __grid_constant__ LookupArgs A)
+__global__ void __launch_bounds__(kThreads, kSide == 16 ? 2 : 5 * 256 / kThreads) lookup_kernel(const __grid_constant__ LookupArgs A)
 {
     constexpr uint32_t kPixels = kSide * kSide, kUnits = kPixels / 32;
     __shared__ __align__(16) float4 table[kCheck ? kTableLights : 1];
@@ -544,7 +577,8 @@ __global__ void __launch_bounds__(kThreads, 5 * 256 / kThreads) lookup_kernel(co
                     continue;
                 }
             }
-            look_up<kCheck, !kCheck && kSide == 32 && kThreads <= 256>(A, table, whole, lists[threadIdx.x >> 5], lane, valid, xf, yf, z, frag, s);
+            constexpr bool kMany = kSide == 32 && kThreads <= 512;  // tiles
+            look_up<kCheck, kMany ? 2 : 4, kMany ? 4 : 12>(A, table, whole, lists[threadIdx.x >> 5], lane, valid, xf, yf, z, frag, s);
             if (!valid) continue;
             CfFragmentSample* out = &A.out[y * A.im.width + x];
             if (A.out_aligned) {

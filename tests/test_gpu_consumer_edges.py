@@ -218,3 +218,21 @@ def test_shading_odd_texels_and_lights(gpu, oracle, falloff, intensity):
     idx = np.arange(300, dtype=np.uint32)
     pc = CfPBRPushConstant(intensity, 0.01, 0.0, falloff, -0.0)
     assert same_shading(shade(v, g, cells, idx, pc, cam), oracle.shade_clusters(v.ubo, cam, pc, g, cells, idx, v.lights))
+
+
+@pytest.mark.parametrize("res, grid, n_lights", [((96, 64), (40, 24, 30), 4000), ((20, 3000), (16, 9, 24), 3500),
+                                                 ((330, 200), (64, 60, 20), 2500), ((900, 500), (90, 70, 12), 2500)])
+def test_lookup_of_many_clusters_per_warp(gpu, oracle, res, grid, n_lights):
+    """Clusters of a few pixels or less: each pixel of a warp walks its own
+    list, of none to over a hundred entries, some of them no light."""
+    v, rng = view_of(res, n_lights, grid=grid, r=(0.2, 5.0))
+    v.lights[[5, 400], 0], v.lights[9, 1], v.lights[20, 8] = np.nan, -np.inf, np.inf
+    aabbs, cells, idx = run_pipeline(gpu, v)
+    assert cells[:, 1].max() > 64
+    idx = idx.copy()
+    idx[rng.integers(0, idx.size, idx.size // 200)] = rng.choice([n_lights, 0xFFFFFFFF], idx.size // 200)
+    cells = cells.copy()
+    cells[rng.integers(0, cells.shape[0], 5)] = [idx.size - 2, 3]  # no cell of this list
+    depth = scenes.depth_log_uniform(rng, *res, 0.1, 300.0, far_plane_fraction=0.02)
+    got = device_lookup(v, depth, cells, idx, aabbs, False)
+    assert same(got, oracle.lookup_clusters(v.ubo, depth, cells, idx, v.lights, v.cap, aabbs, False))
