@@ -804,7 +804,11 @@ __device__ __forceinline__ void evaluate_pairs(const ShadeArgs& A, ShadeWarp& w,
 // one after another cost more than they save: 27x4x55, four lights a list,
 // scattered depths 62 us against 76; with a limit of 4 / 8 / 16 the surfaces above take
 // 164 / 166 / 172 us.
-constexpr uint32_t kShortList = 6;
+// In the smaller images, bound by the latency of a cluster's round trips, also
+// lists of up to kOwnEntries entries for each of the warp's clusters: 96x64,
+// 40x24x56, 8000 lights, scattered depths: one thread per texel 132 us, without
+// this rule 150, with 1 / 2 / 4 entries 149 / 149 / 68.
+constexpr uint32_t kShortList = 6, kOwnEntries = 4;
 constexpr uint32_t kFewTexels = 2;  // entries per texel from which a texel's turn is cheaper than four entries' test
 template <uint32_t kSide, uint32_t kThreads>
 __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__ ShadeArgs A)
@@ -897,8 +901,13 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         // the list of one cluster after another, an entry fetched by each lane and
         // tested by each texel of the cluster.  (One loop over all rounds, so that
         // the evaluation is there once: it is half of the kernel's instructions.)
-        const bool own = longest <= kShortList;
+        bool own = longest <= kShortList;
+        if (kSide == 16 && !own) {
+            const uint32_t same = __match_any_sync(cfk::kFull, cnt ? c : ~0u);
+            own = longest <= kOwnEntries * __popc(__ballot_sync(cfk::kFull, cnt && (same & lt_mask) == 0));
+        }
         uint32_t todo = own ? 0u : __ballot_sync(cfk::kFull, cnt != 0), texels = 0, n_texels = 0, list = 0, left = 0, li = 0;
+        if (own && cnt) li = __ldg(&A.indices[off]);
         uint32_t step = 0;
         bool mine = false;
         for (bool more = true; more;) {
@@ -907,7 +916,8 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
                 more = step < longest;
                 if (more) {
                     const bool has = step < cnt;
-                    here = has ? __ldg(&A.indices[off + step]) : 0u;
+                    here = li;
+                    if (step + 1 < cnt) li = __ldg(&A.indices[off + step + 1]);  // for the next round
                     const bool light = has && here < A.light_count;
                     if (has && !light) alpha = 0.0f;  // an entry that is no light
                     if (light) {

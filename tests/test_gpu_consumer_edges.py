@@ -236,3 +236,18 @@ def test_lookup_of_many_clusters_per_warp(gpu, oracle, res, grid, n_lights):
     depth = scenes.depth_log_uniform(rng, *res, 0.1, 300.0, far_plane_fraction=0.02)
     got = device_lookup(v, depth, cells, idx, aabbs, False)
     assert same(got, oracle.lookup_clusters(v.ubo, depth, cells, idx, v.lights, v.cap, aabbs, False))
+
+
+@pytest.mark.parametrize("res, grid, n_lights", [((96, 64), (40, 24, 30), 4000), ((20, 3000), (16, 9, 24), 3500),
+                                                 ((330, 200), (64, 60, 20), 2500)])
+def test_shading_of_many_clusters_per_warp(gpu, oracle, res, grid, n_lights):
+    """As the lookup's: each texel walks its own list, some of whose entries
+    are no light, and warps on both sides of the rule."""
+    v, rng = view_of(res, n_lights, grid=grid, r=(0.2, 5.0))
+    _, cells, idx = run_pipeline(gpu, v)
+    assert cells[:, 1].max() > 64
+    idx = idx.copy()
+    idx[rng.integers(0, idx.size, idx.size // 200)] = rng.choice([n_lights, 0xFFFFFFFF], idx.size // 200)
+    g = scenes.gbuffer(rng, v.ubo, far_plane_fraction=0.02)
+    cam = scenes.camera_position(v.ubo)
+    assert same_shading(shade(v, g, cells, idx, PC, cam), oracle.shade_clusters(v.ubo, cam, PC, g, cells, idx, v.lights))
