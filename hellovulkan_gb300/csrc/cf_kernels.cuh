@@ -79,7 +79,9 @@ struct ViewCull {
     // part per segment of seg_lights lights, from entry segment * seg_lights
     float4* slice_boxes;             // per slice: the union of its boxes (lo, hi)
     uint32_t* seg_count;             // [slice * segs + segment]: lights listed
-    uint32_t* slice_total;           // per slice: lights listed
+    uint2* slice_total;              // per slice: lights listed, lights that cover it (see list_covering)
+    uint32_t* slice_stop;            // per slice: where its list may end
+    uint32_t* slice_kept;            // per slice: lights listed up to there
     uint32_t* slice_first;           // the scan's plan (see Plan)
     uint32_t* group_total;           // per group: hits
     uint16_t* group_count;           // per group and cluster: hits
@@ -174,8 +176,8 @@ inline uint32_t mask_segments(uint32_t lpad, uint32_t seg_lights) { return (lpad
 
 // Scratch of one view on the hit-mask path.
 struct MaskLayout {
-    size_t slice_first, group_total, group_count, block_total, group_boxes, slice_boxes, seg_count, pool_head, slice_total, unit_run,
-        unit_count, unit_before, pool, slice_lights, slice_idx, bytes;
+    size_t slice_first, group_total, group_count, block_total, group_boxes, slice_boxes, seg_count, pool_head, slice_total, slice_stop, slice_kept,
+        unit_run, unit_count, unit_before, pool, slice_lights, slice_idx, bytes;
     uint32_t pool_batches;
 };
 MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slices, uint32_t lights, uint32_t cap,

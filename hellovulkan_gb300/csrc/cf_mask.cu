@@ -9,7 +9,9 @@
 //                  transforms its lights (posView = cameraView * position,
 //                  r^2) and writes, per slice, those whose sphere reaches the
 //                  slice's box, in light order, into the segment's own part of
-//                  the slice's list.  No segment needs another's count.
+//                  the slice's list.  No segment needs another's count.  A list
+//                  ends where lights that reach the whole slice have filled its
+//                  clusters' lists (see list_covering).
 //   scan_kernel    warps take units, each a run of a slice's candidates against
 //                  one group: the warp keeps the lights that reach the group's
 //                  union box and tests each of them against 32 clusters, one
@@ -90,7 +92,8 @@ __device__ __forceinline__ void box_body(const ViewCull& v, uint32_t k)
     const uint32_t blocks = (v.groups + kGroup - 1) / kGroup;
     for (uint32_t u = k + v.slices * threadIdx.x; u < blocks; u += v.slices * kThreads) v.block_total[u] = 0u;
     if (threadIdx.x == 0) {
-        v.slice_total[k] = 0u;
+        v.slice_total[k] = make_uint2(0u, 0u);
+        v.slice_stop[k] = ~0u;
         if (k == 0) *v.pool_head = 0ull;
     }
     float4 lo = make_float4(inf, inf, inf, 0.f), hi = make_float4(-inf, -inf, -inf, 0.f);
@@ -110,10 +113,9 @@ __device__ __forceinline__ void box_body(const ViewCull& v, uint32_t k)
         for (uint32_t e = 0; e < kBoxIlp; ++e) {
             const uint32_t g = g0 + e * kWarps;
             if (g >= gps) break;
-            const bool nan = (a[e].x != a[e].x) | (a[e].y != a[e].y) | (a[e].z != a[e].z) | (b[e].x != b[e].x) |
-                             (b[e].y != b[e].y) | (b[e].z != b[e].z);
+            const bool odd = g * kGroup + lane < xy && !(a[e].x <= b[e].x && a[e].y <= b[e].y && a[e].z <= b[e].z);
             warp_union(a[e], b[e]);
-            if (__any_sync(kFull, nan)) {
+            if (__any_sync(kFull, odd)) {  // a NaN, or bounds the wrong way round (see covers)
                 a[e] = make_float4(-inf, -inf, -inf, 0.f);
                 b[e] = make_float4(inf, inf, inf, 0.f);
             }
@@ -166,6 +168,64 @@ __device__ __forceinline__ bool reaches(const float4& L, const float4& lo, const
 {
     const float mn[3] = {lo.x, lo.y, lo.z}, mx[3] = {hi.x, hi.y, hi.z};
     return hit_fast(L, mn, mx);
+}
+
+// Whether a light reaches every cluster of a slice whose boxes lie in [lo, hi],
+// by a test that may say no when it does: per axis a box is no further from it
+// than the further side of the union, rounded operation by rounded operation
+// (see box_body for boxes of which that does not hold).
+__device__ __forceinline__ bool covers(const float4& L, const float4& lo, const float4& hi)
+{
+    const float dx = max3f(cf_fsub(hi.x, L.x), cf_fsub(L.x, lo.x), 0.0f), dy = max3f(cf_fsub(hi.y, L.y), cf_fsub(L.y, lo.y), 0.0f),
+                dz = max3f(cf_fsub(hi.z, L.z), cf_fsub(L.z, lo.z), 0.0f);
+    return cf_fadd(cf_fadd(cf_fmul(dx, dx), cf_fmul(dy, dy)), cf_fmul(dz, dz)) < L.w;
+}
+
+// A slice's list ends where its clusters' lists are full for certain: with the
+// segment in which the covering lights reach the cap.  The higher half of a
+// seg_count word is how many of the segment's lights cover the slice, that of
+// slice_total their number in all segments; where one segment has as many as the
+// cap, slice_stop is the first such segment and the lights it lists up to the
+// last one that is needed.  Without an end, the many lights of full lists were
+// all scanned, where the staged kernels stop at a cluster's cap; staged / without
+// / with it, in us:
+//   46x51x9,  39359 lights that reach all, cap 150    54 /  622 / 115
+//   32x18x48, 24181 of radius 20 to 60, cap 255       75 /  247 /  97
+//   22 views of 36x10x53, 18698 that reach all       814 / 6500 / 1021
+//   24x14x32, 10658 that reach all, cap 150           33 /  128 /  36
+constexpr uint32_t kCountMask = 0xffffu;
+constexpr uint32_t kStopShift = 11;
+static_assert(kMaxSegLights < 1u << kStopShift);
+// Lights of a warp that reach a slice from which they are tested for covering
+// it: the second view above 143 us with 16, 97 with 8 or 4, and views whose lists
+// are not full take as long.
+constexpr uint32_t kCoverMin = 8;
+
+// Counts the covering lights of a list CTA's segment (slices z0 to z0 + nz, boxes
+// and masks as list_body has them; `most`: the slices to test the warp's lights
+// for).  Every thread of the CTA takes part.  Out of line: its registers would
+// be every CTA's, and few segments have such lights.
+__device__ __noinline__ void list_covering(const ViewCull& v, float4 L, uint32_t most, const float4* s_box,
+                                           const uint32_t (*s_mask)[32], uint32_t seg, uint32_t z0, uint32_t nz)
+{
+    __shared__ uint32_t s_covers[kListSlices][32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (uint32_t q = 0; q < nz; ++q) {
+        uint32_t n = 0;
+        if ((most >> q) & 1u) n = __popc(__ballot_sync(kFull, covers(L, s_box[2 * q], s_box[2 * q + 1])));
+        if (lane == 0) s_covers[q][warp] = n;
+    }
+    __syncthreads();
+    for (uint32_t q = warp; q < nz; q += nw) {
+        const uint32_t covering = warp_inclusive_scan(lane < nw ? s_covers[q][lane] : 0u, lane);
+        const uint32_t listed = warp_inclusive_scan(lane < nw ? __popc(s_mask[q][lane]) : 0u, lane);
+        if (lane == 31 && covering) {
+            v.seg_count[(size_t)(z0 + q) * v.segs + seg] = listed | covering << 16;
+            atomicAdd(&v.slice_total[z0 + q].y, covering);
+        }
+        const uint32_t enough = __ballot_sync(kFull, covering >= v.cap);
+        if (enough && lane == __ffs(enough) - 1) atomicMin(&v.slice_stop[z0 + q], seg << kStopShift | listed);
+    }
 }
 
 __device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
@@ -226,12 +286,14 @@ __device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
         s_off[q][lane] = incl - c;
         if (lane == 31) {
             v.seg_count[(size_t)(z0 + q) * v.segs + seg] = incl;
-            if (incl) atomicAdd(&v.slice_total[z0 + q], incl);
+            if (incl) atomicAdd(&v.slice_total[z0 + q].x, incl);
         }
     }
     __syncthreads();
+    uint32_t most = 0;  // bit q: slice q lists kCoverMin of the warp's lights or more
     for (; reached; reached &= reached - 1) {
         const uint32_t q = __ffs(reached) - 1, m = s_mask[q][warp];
+        if (__popc(m) >= kCoverMin) most |= 1u << q;
         if ((m >> lane) & 1u) {
             const size_t at = (size_t)(z0 + q) * v.lpad + seg * v.seg_lights + s_off[q][warp] +
                               __popc(m & ((1u << lane) - 1u));
@@ -239,6 +301,12 @@ __device__ __forceinline__ void list_body(const ViewJob& j, uint32_t blk)
             v.slice_idx[at] = i;
         }
     }
+    bool any = false;
+    for (uint32_t b = most; b; b &= b - 1) {
+        const uint32_t q = __ffs(b) - 1;
+        any = any || covers(L, s_box[2 * q], s_box[2 * q + 1]);
+    }
+    if (__syncthreads_or(any)) list_covering(v, L, most, s_box, s_mask, seg, z0, nz);
     if (v.work && tid == 0) atomicAdd(&v.work[0], (unsigned long long)nz * blockDim.x);
 }
 
@@ -390,7 +458,7 @@ __device__ __forceinline__ void fetch_candidates(const ViewCull& v, ScanWarp& s,
     const uint32_t* __restrict__ lists_i = v.slice_idx + (size_t)k * v.lpad;
     uint32_t base = 0;  // candidates before the window
     for (uint32_t w0 = 0; w0 < v.segs && base < t0 + n; w0 += 32) {
-        const uint32_t c = w0 + lane < v.segs ? __ldg(&counts[w0 + lane]) : 0u;
+        const uint32_t c = w0 + lane < v.segs ? __ldg(&counts[w0 + lane]) & kCountMask : 0u;
         const uint32_t incl = warp_inclusive_scan(c, lane);
         const uint32_t first = base + incl - c, end = base + __shfl_sync(kFull, incl, 31);
         if (end > t0) {
@@ -526,16 +594,32 @@ __device__ __forceinline__ void scan_unit(const ViewCull& v, uint32_t u, uint32_
     __syncwarp();  // the next unit overwrites the masks
 }
 
-// The runs of a view: slice k's total[k] candidates in runs of kMaskMaxRun,
-// numbered from first[k]; first[slices] is their number.  A run and a group of
+// The runs of a view: slice k's total[k] candidates (up to its list's end, see
+// list_covering) in runs of kMaskMaxRun, numbered from first[k]; first[slices]
+// is their number.  A run and a group of
 // its slice are a unit: first[k] * groups per slice + group * runs of the
 // slice + run.  Every block of the scan makes the same plan; the first one
-// leaves it in the workspace (slice_first) for the later launches.
+// leaves it in the workspace (slice_first, slice_kept) for the later launches.
 struct Plan {
     uint32_t first[kMaskMaxSlices + 1];
     uint32_t total[kMaskMaxSlices];
     uint32_t warp_runs[kScanWarps];
 };
+
+// The lights that slice k, of at least the cap's covering lights, lists up to its
+// end (see list_covering).
+__device__ __forceinline__ uint32_t list_end(const ViewCull& v, uint32_t k)
+{
+    const uint32_t stop = __ldg(&v.slice_stop[k]);
+    uint32_t total = 0, covering = 0;
+    for (uint32_t q = 0; q < v.segs && covering < v.cap; ++q) {
+        if (q == stop >> kStopShift) return total + (stop & ((1u << kStopShift) - 1));
+        const uint32_t c = __ldg(&v.seg_count[(size_t)k * v.segs + q]);
+        total += c & kCountMask;
+        covering += c >> 16;
+    }
+    return total;
+}
 
 __device__ __forceinline__ void make_plan(const ViewCull& v, Plan& p, bool keep)
 {
@@ -543,7 +627,9 @@ __device__ __forceinline__ void make_plan(const ViewCull& v, Plan& p, bool keep)
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t base = 0;
     for (uint32_t k0 = 0; k0 < v.slices; k0 += kThreads) {
-        const uint32_t k = k0 + tid, total = k < v.slices ? __ldg(&v.slice_total[k]) : 0u;
+        const uint32_t k = k0 + tid;
+        const uint2 listed = k < v.slices ? __ldg(&v.slice_total[k]) : make_uint2(0u, 0u);
+        const uint32_t total = listed.y < v.cap ? listed.x : list_end(v, k);
         const uint32_t n = (total + kMaskMaxRun - 1) / kMaskMaxRun, incl = warp_inclusive_scan(n, lane);
         if (lane == 31) p.warp_runs[warp] = incl;
         __syncthreads();
@@ -562,7 +648,10 @@ __device__ __forceinline__ void make_plan(const ViewCull& v, Plan& p, bool keep)
     if (tid == 0) p.first[v.slices] = base;
     __syncthreads();
     if (keep)
-        for (uint32_t k = tid; k <= v.slices; k += kThreads) v.slice_first[k] = p.first[k];
+        for (uint32_t k = tid; k <= v.slices; k += kThreads) {
+            v.slice_first[k] = p.first[k];
+            if (k < v.slices) v.slice_kept[k] = p.total[k];
+        }
 }
 
 // The slice of run r (of all).
@@ -856,7 +945,7 @@ __device__ __forceinline__ void emit_body(const ViewCull& v, uint32_t blk, uint3
     if (v.segs) {  // without lights there was no scan
         for (uint32_t k = threadIdx.x; k <= v.slices; k += kEmitWarps * 32) {
             p.first[k] = __ldg(&v.slice_first[k]);
-            if (k < v.slices) p.total[k] = __ldg(&v.slice_total[k]);
+            if (k < v.slices) p.total[k] = __ldg(&v.slice_kept[k]);
         }
         __syncthreads();
         units = p.first[v.slices] * gps;
@@ -931,7 +1020,9 @@ MaskLayout mask_layout(uint32_t clusters, uint32_t slice_clusters, uint32_t slic
     m.seg_count = take((size_t)slices * mask_segments(lpad, seg_lights) * sizeof(uint32_t));
     const size_t units = (size_t)groups * ((lpad + kMaskMaxRun - 1) / kMaskMaxRun);
     m.pool_head = take(sizeof(unsigned long long));
-    m.slice_total = take((size_t)slices * sizeof(uint32_t));
+    m.slice_total = take((size_t)slices * sizeof(uint2));
+    m.slice_stop = take((size_t)slices * sizeof(uint32_t));
+    m.slice_kept = take((size_t)slices * sizeof(uint32_t));
     m.slice_first = take((size_t)(slices + 1) * sizeof(uint32_t));
     m.unit_run = take(units * sizeof(uint32_t));
     m.unit_count = take(units * kMaskGroup * sizeof(uint8_t));
@@ -975,7 +1066,9 @@ void mask_bind(ViewCull& v, const MaskLayout& m, unsigned char* ws, uint32_t seg
     v.slice_boxes = reinterpret_cast<float4*>(ws + m.slice_boxes);
     v.seg_count = reinterpret_cast<uint32_t*>(ws + m.seg_count);
     v.pool_head = reinterpret_cast<unsigned long long*>(ws + m.pool_head);
-    v.slice_total = reinterpret_cast<uint32_t*>(ws + m.slice_total);
+    v.slice_total = reinterpret_cast<uint2*>(ws + m.slice_total);
+    v.slice_stop = reinterpret_cast<uint32_t*>(ws + m.slice_stop);
+    v.slice_kept = reinterpret_cast<uint32_t*>(ws + m.slice_kept);
     v.slice_first = reinterpret_cast<uint32_t*>(ws + m.slice_first);
     v.unit_run = reinterpret_cast<uint32_t*>(ws + m.unit_run);
     v.unit_count = ws + m.unit_count;
