@@ -800,6 +800,11 @@ __device__ __forceinline__ void evaluate_pairs(const ShadeArgs& A, ShadeWarp& w,
 // texel: every light evaluated 776 us, tested one by one from each texel's own
 // list 228 us, so 164 us (2400 instructions per 32 texels, two thirds of them in
 // 3.7 evaluations); every texel at its own depth 1113 / 139 / 121 us.
+// A cluster's pairs are gathered entry by entry or, where it has few of the
+// texels, texel by texel: entry by entry, lists that all reach took a step for
+// each pair (5804x17, 35x14x33, 2903 lights that reach everything: one thread
+// per texel 1264 us, entry by entry 4103, texel by texel 2098; 354x27, 79x47x8,
+// 104 lights: 114 / 235 / 165).
 // Lists up to kShortList each texel walks itself, as the lists of many clusters
 // one after another cost more than they save: 27x4x55, four lights a list,
 // scattered depths 62 us against 76; with a limit of 4 / 8 / 16 the surfaces above take
@@ -911,6 +916,7 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
         uint32_t step = 0;
         bool mine = false;
         for (bool more = true; more;) {
+            bool few = false;  // the cluster has few of the texels
             uint32_t any = 0, need = 0, here = 0;  // need: bit q: entry q may add something to the lane's texel
             if (own) {
                 more = step < longest;
@@ -957,7 +963,8 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
                         lit = lit || lights;
                         if (lights != (n < 32 ? (1u << n) - 1u : ~0u)) alpha = 0.0f;  // an entry that is no light
                     }
-                    if (kFewTexels * n_texels < n) {
+                    few = kFewTexels * n_texels < n;
+                    if (few) {
                         for (uint32_t m = texels; m; m &= m - 1) {
                             const uint32_t t = __ffs(m) - 1;
                             const V3 d = v3_sub(V3{e.x, e.y, e.z}, V3{w.f[kPx][t], w.f[kPy][t], w.f[kPz][t]});
@@ -978,16 +985,32 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
                     any = __reduce_or_sync(cfk::kFull, need);
                 }
             }
+            // The pairs: of one entry after another and each texel, or of one texel
+            // after another and each entry.
+            uint32_t turns = 0;
+            if (few && any) {
+                turns = __ballot_sync(cfk::kFull, need != 0);
+                any = 0;
+            }
             for (;;) {
-                if (any) {
-                    const uint32_t q = __ffs(any) - 1, from = __shfl_sync(cfk::kFull, here, q);
-                    any &= any - 1;
-                    const bool pair = (need >> q) & 1u;
+                if (any | turns) {
+                    bool pair;
+                    uint32_t light = here, texel = lane;
+                    if (turns) {
+                        texel = __ffs(turns) - 1;
+                        turns &= turns - 1;
+                        pair = (__shfl_sync(cfk::kFull, need, texel) >> lane) & 1u;
+                    } else {
+                        const uint32_t q = __ffs(any) - 1, from = __shfl_sync(cfk::kFull, here, q);
+                        any &= any - 1;
+                        pair = (need >> q) & 1u;
+                        if (!own) light = from;
+                    }
                     const uint32_t m = __ballot_sync(cfk::kFull, pair);
                     if (pair) {
                         const uint32_t at = (put + __popc(m & lt_mask)) & 63u;
-                        w.light[at] = own ? here : from;
-                        w.texel[at] = lane;
+                        w.light[at] = light;
+                        w.texel[at] = texel;
                     }
                     put += __popc(m);
                 }
@@ -996,7 +1019,7 @@ __global__ void __launch_bounds__(kThreads) shade_kernel(const __grid_constant__
                     evaluate_pairs(A, w, done, n, lane, lo);
                     done += n;
                 }
-                if (!any) break;
+                if (!(any | turns)) break;
             }
         }
         __syncwarp();

@@ -251,3 +251,19 @@ def test_shading_of_many_clusters_per_warp(gpu, oracle, res, grid, n_lights):
     g = scenes.gbuffer(rng, v.ubo, far_plane_fraction=0.02)
     cam = scenes.camera_position(v.ubo)
     assert same_shading(shade(v, g, cells, idx, PC, cam), oracle.shade_clusters(v.ubo, cam, PC, g, cells, idx, v.lights))
+
+
+@pytest.mark.parametrize("res, grid, n_lights", [((19, 886), (20, 8, 55), 150), ((97, 64), (22, 20, 24), 70),
+                                                 ((1001, 701), (90, 70, 12), 40), ((1201, 1051), (120, 105, 6), 33)])
+def test_shading_of_lists_that_all_reach(gpu, oracle, res, grid, n_lights):
+    """Every light reaches every texel, with a few texels to a cluster: a
+    texel's pairs are gathered 32 at a time, and the sums keep the list's
+    order; an entry that is no light in the middle of some lists."""
+    v, rng = view_of(res, n_lights, grid=grid, r=(500.0, 2000.0))
+    _, cells, idx = run_pipeline(gpu, v)
+    assert cells[:, 1].min() == n_lights
+    idx = idx.copy()
+    idx[rng.integers(0, idx.size, idx.size // 500)] = n_lights
+    g = scenes.gbuffer(rng, v.ubo, far_plane_fraction=0.02)
+    cam = scenes.camera_position(v.ubo)
+    assert same_shading(shade(v, g, cells, idx, PC, cam), oracle.shade_clusters(v.ubo, cam, PC, g, cells, idx, v.lights))
