@@ -267,3 +267,24 @@ def test_shading_of_lists_that_all_reach(gpu, oracle, res, grid, n_lights):
     g = scenes.gbuffer(rng, v.ubo, far_plane_fraction=0.02)
     cam = scenes.camera_position(v.ubo)
     assert same_shading(shade(v, g, cells, idx, PC, cam), oracle.shade_clusters(v.ubo, cam, PC, g, cells, idx, v.lights))
+
+
+@pytest.mark.parametrize("res", [(31, 400), (97, 64), (1001, 701)])
+def test_shading_of_unlit_tiles(gpu, oracle, res):
+    """An image whose tiles are unlit but for those around a few small lights:
+    unlit clusters, texels outside of the grid and cells that are none, in
+    tiles of their own and beside lit ones; a black albedo's sign."""
+    v, rng = view_of(res, 12, grid=(16, 12, 24), r=(0.05, 0.8))
+    v.lights[:, 0:3] *= np.float32(0.2)
+    _, cells, idx = run_pipeline(gpu, v)
+    lit = cells[:, 1] > 0
+    assert 0 < lit.sum() < 0.1 * lit.size
+    cells = cells.copy()
+    cells[rng.integers(0, cells.shape[0], 40)] = [idx.size, 1]  # no cell of this list
+    g = scenes.gbuffer(rng, v.ubo, far_plane_fraction=0.02)
+    w, h = res
+    g[: h // 3, :, 3] = 1.0
+    g[h // 2:, : w // 2, 3] = rng.choice([1.0, -0.5, 1.5, np.nan], (h - h // 2, w // 2))
+    g[:, :, 8:11] = np.where(rng.uniform(size=(h, w, 1)) < 0.1, np.float32(-0.0), g[:, :, 8:11])
+    cam = scenes.camera_position(v.ubo)
+    assert same_shading(shade(v, g, cells, idx, PC, cam), oracle.shade_clusters(v.ubo, cam, PC, g, cells, idx, v.lights))
