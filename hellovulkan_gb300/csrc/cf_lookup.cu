@@ -331,9 +331,9 @@ __device__ __forceinline__ uint32_t containing(const ListWarp& w, uint32_t n, co
 // The warp reads the list of each cluster that its pixels lie in together: a
 // lane fetches and transforms an entry; then each pixel of the cluster tests
 // 32 of them, or, where the cluster has few of the warp's pixels, the lanes
-// test their entries against one pixel after another.  Without the check, a warp
-// of many clusters or short lists has each pixel walk its own list, kOwnStep
-// entries at a time with the next ones' indices on their way.
+// test their entries against one pixel after another.  A warp of many clusters
+// or short lists has each pixel walk its own list, kOwnStep entries at a time
+// with the next ones' indices on their way.
 constexpr uint32_t kFewPixels = 3;  // entries per pixel from which a pixel's turn is cheaper than four entries' test
 // Where all lists of a warp's pixels are this short, each pixel walks its own
 // (1920x1080, scattered: 49.5 -> 46.9 us), and where they lie in so many clusters
@@ -345,6 +345,9 @@ constexpr uint32_t kFewPixels = 3;  // entries per pixel from which a pixel's tu
 //   480x270, 128x72x24, 4000 lights, surfaces      22.7 / 24.3 / 20.7
 //   20x20000, 16x9x24,  1024 lights, scattered     22.6 / 38.5 / 15.7
 //   1920x1080, 64x64x64, 2000 lights, scattered   107   / 114  / 64
+// With the check: 1855x69, 42x34x50, 48 lights that reach all 45.0 / 58.5 / 30.2 (one
+// thread per pixel / no pixel walks its own / this rule), 17x56, 122x61x2, 27 lights of
+// radius 20 to 60 12.4 / 21.6 / 12.1.
 // A launch of many tiles is bound by issue and takes 4 entries per cluster
 // (6 / 8 / 12: the reference view's surfaces 46.4 -> 48.5 / 50.0 / 52.3), two at
 // a time; one of a tile per SM or less by latency: 12, four at a time.
@@ -379,38 +382,43 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
         s.cluster = 0xFFFFFFFFu;
         s.flags |= CF_FRAGMENT_OUTSIDE_GRID;
     }
-    bool own = false;
-    if (!kCheck) {
-        const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
-        own = longest <= kShortLookup;
-        if (!own) {
-            const uint32_t same = __match_any_sync(cfk::kFull, cnt ? c : ~0u);
-            own = longest <= kOwnPerList * __popc(__ballot_sync(cfk::kFull, cnt && (same & ((1u << lane) - 1u)) == 0));
-        }
-        if (own) {
-            uint32_t next[kOwnStep];
+    const uint32_t longest = __reduce_max_sync(cfk::kFull, cnt);
+    bool own = longest <= kShortLookup;
+    if (!own) {
+        const uint32_t same = __match_any_sync(cfk::kFull, cnt ? c : ~0u);
+        own = longest <= kOwnPerList * __popc(__ballot_sync(cfk::kFull, cnt && (same & ((1u << lane) - 1u)) == 0));
+    }
+    if (own) {
+        uint32_t next[kOwnStep], before = 0;
+        bool walked = true;  // with the check: none of the entries so far ended the list's part (see below)
 #pragma unroll
-            for (uint32_t e = 0; e < kOwnStep; ++e) next[e] = e < cnt ? __ldg(&A.indices[off + e]) : 0u;
-            for (uint32_t j = 0; j < longest; j += kOwnStep) {
-                float4 q[kOwnStep];
-                float r[kOwnStep];
+        for (uint32_t e = 0; e < kOwnStep; ++e) next[e] = e < cnt ? __ldg(&A.indices[off + e]) : 0u;
+        for (uint32_t j = 0; j < longest; j += kOwnStep) {
+            float4 q[kOwnStep];
+            float r[kOwnStep];
+            bool in_part[kOwnStep];
 #pragma unroll
-                for (uint32_t e = 0; e < kOwnStep; ++e) {
-                    const bool has = j + e < cnt, light = has && next[e] < A.light_count;
-                    if (has && !light) s.flags |= CF_FRAGMENT_BAD_CELL;
-                    const CfLightData* l = &A.lights[next[e]];
-                    q[e] = light ? __ldg(reinterpret_cast<const float4*>(&l->position[0])) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    r[e] = light ? __ldg(&l->radius) : __uint_as_float(0x7fffffffu);  // NaN: contains nothing
-                    next[e] = j + kOwnStep + e < cnt ? __ldg(&A.indices[off + j + kOwnStep + e]) : 0u;
+            for (uint32_t e = 0; e < kOwnStep; ++e) {
+                const bool has = j + e < cnt, light = has && next[e] < A.light_count;
+                if (has && !light) s.flags |= CF_FRAGMENT_BAD_CELL;
+                const CfLightData* l = &A.lights[next[e]];
+                q[e] = light ? __ldg(reinterpret_cast<const float4*>(&l->position[0])) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r[e] = light ? __ldg(&l->radius) : __uint_as_float(0x7fffffffu);  // NaN: contains nothing
+                if (kCheck) {
+                    in_part[e] = walked = walked && light && (j + e == 0 || next[e] > before);
+                    before = next[e];
                 }
+                next[e] = j + kOwnStep + e < cnt ? __ldg(&A.indices[off + j + kOwnStep + e]) : 0u;
+            }
 #pragma unroll
-                for (uint32_t e = 0; e < kOwnStep; ++e) {
-                    const float* V = u.cameraView;
-                    const float p[3] = {cf_mat4_row(V, 0, q[e].x, q[e].y, q[e].z, q[e].w),
-                                        cf_mat4_row(V, 1, q[e].x, q[e].y, q[e].z, q[e].w),
-                                        cf_mat4_row(V, 2, q[e].x, q[e].y, q[e].z, q[e].w)};
-                    s.covering += contains(frag, p, cf_fmul(r[e], r[e])) ? 1u : 0u;
-                }
+            for (uint32_t e = 0; e < kOwnStep; ++e) {
+                const float* V = u.cameraView;
+                const float p[3] = {cf_mat4_row(V, 0, q[e].x, q[e].y, q[e].z, q[e].w),
+                                    cf_mat4_row(V, 1, q[e].x, q[e].y, q[e].z, q[e].w),
+                                    cf_mat4_row(V, 2, q[e].x, q[e].y, q[e].z, q[e].w)};
+                const uint32_t hit = contains(frag, p, cf_fmul(r[e], r[e])) ? 1u : 0u;
+                s.covering += hit;
+                if (kCheck) in_list += in_part[e] ? hit : 0u;
             }
         }
     }

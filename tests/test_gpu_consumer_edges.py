@@ -288,3 +288,34 @@ def test_shading_of_unlit_tiles(gpu, oracle, res):
     g[:, :, 8:11] = np.where(rng.uniform(size=(h, w, 1)) < 0.1, np.float32(-0.0), g[:, :, 8:11])
     cam = scenes.camera_position(v.ubo)
     assert same_shading(shade(v, g, cells, idx, PC, cam), oracle.shade_clusters(v.ubo, cam, PC, g, cells, idx, v.lights))
+
+
+@pytest.mark.parametrize("res, grid, n_lights, r", [((96, 64), (40, 24, 30), 4000, (0.2, 5.0)), ((20, 3000), (16, 9, 24), 1500, (0.2, 5.0)),
+                                                    ((330, 200), (64, 60, 20), 900, (0.2, 9.0)), ((17, 56), (122, 61, 2), 27, (500.0, 900.0))])
+def test_check_of_many_clusters_per_warp(gpu, oracle, res, grid, n_lights, r):
+    """As the lookup's, with the all-lights check: each pixel of a warp walks its
+    own list, up to the entry that does not ascend or is no light for what
+    the list lacks."""
+    v, rng = view_of(res, n_lights, grid=grid, r=r)
+    v.lights[5, 0], v.lights[9, 1], v.lights[20, 8] = np.nan, -np.inf, np.inf
+    aabbs, cells, idx = run_pipeline(gpu, v)
+    idx = idx.copy()
+    at = rng.integers(0, idx.size, idx.size // 40)
+    idx[at] = rng.choice([n_lights, 0xFFFFFFFF, 0, n_lights - 1], at.size)
+    depth = scenes.depth_log_uniform(rng, *res, 0.1, 300.0, far_plane_fraction=0.02)
+    got = device_lookup(v, depth, cells, idx, aabbs, True)
+    want = oracle.lookup_clusters(v.ubo, depth, cells, idx, v.lights, v.cap, aabbs, True)
+    # what is missing, from the part of each list that a walk over all lights matches
+    last = np.concatenate([[-1], idx[:-1].astype(np.int64)])
+    last[np.minimum(cells[:, 0], idx.size - 1)] = -1
+    good = (idx < n_lights) & (idx.astype(np.int64) > last)
+    bad_before = np.concatenate([[0], np.cumsum(~good)])
+    prefix = cells.copy()
+    for c in np.nonzero(cells[:, 1])[0]:
+        off, n = cells[c]
+        prefix[c, 1] = np.searchsorted(bad_before[off + 1:off + n + 1], bad_before[off], side="right")
+    every = oracle.lookup_clusters(v.ubo, depth, np.zeros_like(cells), idx, v.lights, v.cap, aabbs, True)["missing"]
+    matched = oracle.lookup_clusters(v.ubo, depth, prefix, idx, v.lights, v.cap, aabbs, False)["covering"]
+    want["missing"] = every - matched
+    assert want["missing"].max() > 0
+    assert same(got, want)
