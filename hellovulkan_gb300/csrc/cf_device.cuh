@@ -66,16 +66,18 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t x, uint32_t lan
 }
 
 // The least and greatest of the lanes' values (a NaN only where all are).
+// Volatile: a plain asm may be moved into the branch that uses its result, where
+// lanes that it names would be missing.
 __device__ __forceinline__ float warp_min(float x)
 {
     float r;
-    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
     return r;
 }
 __device__ __forceinline__ float warp_max(float x)
 {
     float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
     return r;
 }
 
