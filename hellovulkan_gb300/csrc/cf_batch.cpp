@@ -108,6 +108,9 @@ struct CfBatch {
     // changed until it has completed.
     cudaEvent_t last_use = nullptr;
     bool used = false;
+    // False after a rebuild that failed: the tables may be of other views, or
+    // point into memory that was given back.
+    bool ready = true;
 };
 
 namespace {
@@ -185,6 +188,7 @@ int validate_view(const CfBatchView& v, uint32_t i, uint32_t* clusters)
 // to a few times the staged path's, once more without them (`masks` false).
 int rebuild(CfBatch* b, bool masks = true)
 {
+    b->ready = false;
     const int w = wait_idle(b);  // passes still queued read the tables rewritten below
     if (w) return w;
     drop_graph(b);
@@ -378,7 +382,14 @@ int rebuild(CfBatch* b, bool masks = true)
         e = cudaMemcpy(b->d_items, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && n) e = cudaMemcpy(b->d_aabb_jobs, aabb_jobs.data(), n * sizeof(cfk::AabbJob), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && n) e = cudaMemcpy(b->d_aabb_prefix, aabb_prefix.data(), n * 4, cudaMemcpyHostToDevice);
-    return e == cudaSuccess ? CF_SUCCESS : cuda_fail(e, "batch tables upload");
+    if (e != cudaSuccess) return cuda_fail(e, "batch tables upload");
+    b->ready = true;
+    return CF_SUCCESS;
+}
+
+int check_ready(const CfBatch* b)
+{
+    return b->ready ? CF_SUCCESS : fail(CF_ERROR_NOT_READY, "the batch's views could not be set");
 }
 
 int enqueue_batch(CfBatch* b, cudaStream_t st)
@@ -408,6 +419,8 @@ namespace cfrt {
 
 int batch_cull(CfBatch* b, cudaStream_t st)
 {
+    const int r = check_ready(b);
+    if (r) return r;
     DeviceGuard g(b->device);
     if (!b->use_graph || st == nullptr) {
         const int s = enqueue_batch(b, st);
@@ -488,6 +501,11 @@ int cf_batch_destroy(CfBatch* b)
 int cf_batch_set_views(CfBatch* b, const CfBatchView* views, uint32_t n)
 {
     if (!b || (n && !views)) return fail(CF_ERROR_INVALID_ARGUMENT, "cf_batch_set_views: null argument");
+    for (uint32_t i = 0; i < n; ++i) {  // before anything of the batch changes
+        uint32_t clusters = 0;
+        const int s = validate_view(views[i], i, &clusters);
+        if (s) return s;
+    }
     b->views.assign(views, views + n);
     return rebuild(b);
 }
@@ -496,6 +514,8 @@ int cf_batch_update_view_matrices(CfBatch* b, const CfClusterForwardUBO* ubos, u
 {
     if (!b || (n && !ubos)) return fail(CF_ERROR_INVALID_ARGUMENT, "null argument");
     if (n != b->views.size()) return fail(CF_ERROR_INVALID_ARGUMENT, "%u UBOs for %zu views", n, b->views.size());
+    const int r = check_ready(b);
+    if (r) return r;
     DeviceGuard g(b->device);
     const int w = wait_idle(b);  // a pass queued on another stream may still read the table
     if (w) return w;
@@ -513,6 +533,8 @@ int cf_batch_update_view_matrices(CfBatch* b, const CfClusterForwardUBO* ubos, u
 int cf_batch_generate_aabbs(CfBatch* b, void* stream)
 {
     if (!b) return fail(CF_ERROR_INVALID_ARGUMENT, "null batch");
+    const int r = check_ready(b);
+    if (r) return r;
     DeviceGuard g(b->device);
     const cudaError_t e = cfk::launch_batch_aabb(b->d_aabb_jobs, b->d_aabb_prefix, (uint32_t)b->views.size(),
                                                  b->aabb_blocks, (cudaStream_t)stream);

@@ -245,7 +245,9 @@ CFCULL_API int cf_batch_destroy(CfBatch* batch);
  * work-item tables.  Synchronous: it first waits for every pass and AABB
  * generation the batch enqueued (outside a stream capture) to finish, since
  * those read the tables it rewrites.  cf_batch_set_tuning,
- * cf_batch_update_view_matrices and cf_batch_set_graph wait the same way. */
+ * cf_batch_update_view_matrices and cf_batch_set_graph wait the same way.
+ * An invalid view leaves the batch as it was; after any other failure its
+ * passes return CF_ERROR_NOT_READY until views are set. */
 CFCULL_API int cf_batch_set_views(CfBatch* batch, const CfBatchView* views, uint32_t count);
 /* Updates the view matrices (cameraView of each UBO; the projection part must
  * not change) for the next cf_batch_cull.  Synchronises `stream`. */

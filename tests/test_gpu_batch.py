@@ -146,3 +146,41 @@ def test_batch_rejects_bad_views(gpu):
     with pytest.raises(CfError) as e:
         b.set_views(bvs)
     assert e.value.status == 1
+
+
+def test_after_views_that_could_not_be_set_nothing_runs(gpu, cflib, oracle):
+    """A set_views that fails for want of memory leaves tables that point into
+    memory given back: culling, AABBs and new matrices are refused until
+    views are set.  One that is refused for an invalid view changes nothing."""
+    from hellovulkan_gb300._lib import CfError
+    from hellovulkan_gb300.batch import Batch, BatchBuffers
+    few, many = BatchBuffers([scenes.plain_small(5)]), BatchBuffers([scenes.plain_small(6 + i) for i in range(20)])
+    b = Batch(gpu)
+    b.set_views(few.batch_views())
+    b.generate_aabbs()
+    b.cull()
+    cflib.cf_testing_fail_allocation_after(1)  # the workspace grows, the tables do not
+    try:
+        with pytest.raises(CfError) as e:
+            b.set_views(many.batch_views())
+    finally:
+        cflib.cf_testing_fail_allocation_after(-1)
+    assert e.value.status == 2  # CF_ERROR_OUT_OF_MEMORY
+    for call in (b.cull, b.generate_aabbs, lambda: b.update_view_matrices([v.ubo for v in many.views])):
+        with pytest.raises(CfError) as e:
+            call()
+        assert e.value.status == 5  # CF_ERROR_NOT_READY
+    for bufs in (many, few):
+        b.set_views(bufs.batch_views())
+        b.generate_aabbs()
+        b.cull()
+        check_all(oracle, bufs)
+    bad = few.batch_views()
+    bad[0].max_lights_per_cluster = 0
+    with pytest.raises(CfError) as e:
+        b.set_views(bad)
+    assert e.value.status == 1  # CF_ERROR_INVALID_ARGUMENT
+    few.cells[0].fill_(-1)
+    b.cull()
+    check_all(oracle, few)
+    b.close()
