@@ -17,7 +17,7 @@
 // lists: with every pixel at its own depth, unsorted warps had 5 to 10 of 32
 // lanes active.  A sorted warp's fragments also lie in a small box, which few
 // lights of the whole set reach.  1920x1080, 1024 lights, every pixel at its own
-// depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 47 us,
+// depth, one thread per unsorted pixel against sorted tiles: lookup 120 -> 43 us,
 // shading 1113 -> 121 us; 480x270 with 3000 lights and the all-lights check
 // 812 -> 40 us.
 #include <cuda_runtime.h>
@@ -508,8 +508,8 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
     if (kCheck) s.missing -= in_list;
 }
 
-// One CTA per tile.  Bound by issue (62% of the slots at 1920x1080): some 300
-// instructions a pixel apart from its list, six of them IEEE divisions.  A
+// One CTA per tile.  Bound by issue (72% of the slots at 1920x1080): some 300
+// instructions a pixel apart from its list, five of them IEEE divisions.  A
 // warp's lists cost a transform per 32 entries and a test per entry that
 // reaches its fragments' box; when each lane walked its own list the lookup of
 // that image took 59 us, with 3000 lights on surfaces 193 us (now 72).  With
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, kSide == 16 ? 2 : 5 * 256 / kThreads
                 const float inf = __uint_as_float(0x7f800000u);
                 float lo[3], hi[3];
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {  // a NaN coordinate is in no sphere: fminf and fmaxf pass it over
+                for (int a = 0; a < 3; ++a) {  // a NaN coordinate is in no sphere: the reductions pass it over
                     lo[a] = cfk::warp_min(valid ? frag[a] : inf);
                     hi[a] = cfk::warp_max(valid ? frag[a] : -inf);
                 }
