@@ -186,6 +186,9 @@ uint64_t cull_bytes(const CfClusterForwardUBO& ubo, uint32_t light_count, uint32
 
 namespace {
 
+// The hit-mask path's counts: of a cluster in 16 bits, of a unit in 8.
+static_assert(kMaxCap <= 0xffff && cfk::kMaskMaxRun <= 0xff);
+
 // The hit-mask path of one view: slabs, candidate lists, culling straight
 // into the packed list.
 int enqueue_mask(cfk::ViewJob& j, const CfClusterForwardUBO& ubo, const CfLightData* d_lights, uint32_t light_count,
