@@ -1457,7 +1457,7 @@ constexpr uint64_t kStagedMinTests = 16ull << 20;
 
 CullConfig default_cull_config(uint32_t clusters, uint32_t lights, uint32_t slices)
 {
-    if (slices >= 2 && mask_pays(clusters, clusters / slices, slices, lights) &&
+    if (slices && mask_pays(clusters, clusters / slices, slices, lights) &&
         (lights >= kMaskMinLights || (uint64_t)clusters * lights >= kMaskMinTests))
         return kMaskConfig;
     return unmasked_cull_config(clusters, lights, slices);

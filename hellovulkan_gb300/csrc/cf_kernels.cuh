@@ -214,10 +214,15 @@ inline bool mask_fits(uint32_t clusters, uint32_t slice_clusters, uint32_t slice
 //   8x8x16,  16 M lights  1950 M   6009 against 10674 us (few groups: staged is slow)
 //   32x18x48, 4 M lights  3300 M   3419 against  2074 us
 //   16x9x24, 16 M lights  7300 M  10575 against  8166 us
+// Of less than four slices a list hardly prunes, and its end (see list_covering)
+// seldom comes: 61x51x3 with 51841 lights of radius 20 to 60 166 us with hit masks,
+// 47 staged; 40x40x2 with 2304 of them 35, 12.5 by brute force; with 4096 lights of
+// radius 1 to 5 30 and 35.
+constexpr uint32_t kMaskMinSlices = 4;
 constexpr uint64_t kMaskUnitBytes = 100, kMaskMaxUnitBytes = 512ull << 20, kMaskMaxWindowSteps = 2000ull << 20;
 inline bool mask_pays(uint32_t clusters, uint32_t slice_clusters, uint32_t slices, uint32_t lights)
 {
-    if (!mask_fits(clusters, slice_clusters, slices)) return false;
+    if (slices < kMaskMinSlices || !mask_fits(clusters, slice_clusters, slices)) return false;
     const uint64_t lpad = pad_lights(lights), groups = group_count(clusters, slice_clusters, slices, kMaskGroup, kModeBinned);
     const uint64_t units = groups * ((lpad + kMaskMaxRun - 1) / kMaskMaxRun), lists = 20ull * slices * lpad;
     const uint64_t windows = (lpad + 32 * kMaxSegLights - 1) / (32 * kMaxSegLights);

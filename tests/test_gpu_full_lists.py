@@ -61,6 +61,30 @@ def test_lights_that_reach_the_near_slices(gpu, oracle, grid, n, cap):
     assert_matches_oracle(oracle, v, *run_pipeline(gpu, v, MASK))
 
 
+@pytest.mark.parametrize("slices", [1, 3, 4])
+def test_few_slices_are_left_to_the_other_kernels(gpu, oracle, slices):
+    from hellovulkan_gb300.batch import Batch, BatchBuffers
+    from hellovulkan_gb300.pipelines import PipelineLightCulling, ResourcesClusterForward, ResourcesLight
+    v = view((30, 20, slices), 9000, (1.0, 60.0), 20)
+    rl, rc = ResourcesLight(gpu), ResourcesClusterForward(gpu)
+    rl.add_lights(v.lights)
+    rc.create_buffers(*v.grid, v.cap)
+    cull = PipelineLightCulling(gpu, rl, rc)
+    cull.set_cluster_forward_ubo(v.ubo)
+    assert (cull.tuning() == MASK) == (slices == 4)
+    for o in (cull, rc, rl):
+        o.close()
+    assert_matches_oracle(oracle, v, *run_pipeline(gpu, v))
+    bufs = BatchBuffers([v])
+    b = Batch(gpu)
+    b.set_views(bufs.batch_views())
+    assert (b.info()["bucket_configs"][0]["config"] == list(MASK[:4])) == (slices == 4)
+    b.generate_aabbs()
+    b.cull()
+    assert_matches_oracle(oracle, v, *bufs.read(0))
+    b.close()
+
+
 @pytest.mark.parametrize("n", [2000, 9000])
 def test_boxes_the_wrong_way_round(gpu, oracle, n):
     """A box whose lower bounds lie above its upper ones is further from a
