@@ -351,7 +351,10 @@ constexpr uint32_t kFewPixels = 3;  // entries per pixel from which a pixel's tu
 // A launch of many tiles is bound by issue and takes 4 entries per cluster
 // (6 / 8 / 12: the reference view's surfaces 46.4 -> 48.5 / 50.0 / 52.3), two at
 // a time; one of a tile per SM or less by latency: 12, four at a time.
-constexpr uint32_t kShortLookup = 4;
+// From kOwnClusters on a step of the lists side by side has more pixels at work
+// than a round of one list, however long: 31x7444, 57x51x3, 2124 lights in one place
+// 84 / - / 145 without this, 86 with it (with the check 701 / - / 215 and 126).
+constexpr uint32_t kShortLookup = 4, kOwnClusters = 24;
 constexpr uint32_t kBoxList = 8;    // a list up to this long is not worth a box
 template <bool kCheck, uint32_t kOwnStep, uint32_t kOwnPerList>
 __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table, bool whole, ListWarp& w, uint32_t lane,
@@ -386,7 +389,8 @@ __device__ __forceinline__ void look_up(const LookupArgs& A, const float4* table
     bool own = longest <= kShortLookup;
     if (!own) {
         const uint32_t same = __match_any_sync(cfk::kFull, cnt ? c : ~0u);
-        own = longest <= kOwnPerList * __popc(__ballot_sync(cfk::kFull, cnt && (same & ((1u << lane) - 1u)) == 0));
+        const uint32_t clusters = __popc(__ballot_sync(cfk::kFull, cnt && (same & ((1u << lane) - 1u)) == 0));
+        own = longest <= kOwnPerList * clusters || clusters >= kOwnClusters;
     }
     if (own) {
         uint32_t next[kOwnStep], before = 0;

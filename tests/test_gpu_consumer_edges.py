@@ -319,3 +319,20 @@ def test_check_of_many_clusters_per_warp(gpu, oracle, res, grid, n_lights, r):
     want["missing"] = every - matched
     assert want["missing"].max() > 0
     assert same(got, want)
+
+
+@pytest.mark.parametrize("res, grid, n_lights, cap", [((31, 200), (62, 40, 3), 450, 500), ((31, 6000), (62, 50, 3), 150, 150),
+                                                      ((28, 300), (24, 40, 3), 400, 500)])
+@pytest.mark.parametrize("check_all", [False, True])
+def test_lookup_of_long_lists_of_many_clusters(gpu, oracle, res, grid, n_lights, cap, check_all):
+    """A cluster or more for each pixel of a warp, with lists longer than the
+    rule by length takes: each pixel walks its own all the same; and 24
+    clusters or a few less."""
+    v, rng = view_of(res, n_lights, grid=grid, r=(500.0, 900.0))
+    v.cap = cap
+    aabbs, cells, idx = run_pipeline(gpu, v)
+    assert cells[:, 1].min() == n_lights
+    depth = scenes.depth_log_uniform(rng, *res, 0.1, 300.0, far_plane_fraction=0.02)
+    depth[:, :] = depth[:, :1]  # a row at one depth: its pixels lie in the columns' clusters
+    got = device_lookup(v, depth, cells, idx, aabbs, check_all)
+    assert same(got, oracle.lookup_clusters(v.ubo, depth, cells, idx, v.lights, v.cap, aabbs, check_all))
